@@ -48,7 +48,7 @@ public:
         c2_ = DevBuf<float>(cells_);
         out_ = DevBuf<float4>(cells_);
         out_host_ = HostBuf<float>(cells_ * 4);
-        fields_ = DevBuf<IWaveField>(4);
+        fields_ = DevBuf<IWaveField>(2);
         sources_dev_ = DevBuf<IWaveSource>(static_cast<size_t>(d.max_sources) * d.max_substeps);
         sources_host_ = HostBuf<IWaveSource>(static_cast<size_t>(d.max_sources) * d.max_substeps);
         queue_.reset(d.max_sources);
@@ -102,7 +102,8 @@ public:
             const int count = static_cast<int>(first[s + 1] - first[s]);
             if (count > 0) {
                 check(launch_source_mean(sources_dev_.p + first[s], count, stream_), "source mean");
-                check(launch_source_apply(field(), sources_dev_.p + first[s], count, stream_), "sources");
+                check(launch_source_apply(fields_.p + which_, nullptr, make_int2(0, count), sources_dev_.p + first[s], 1,
+                                          static_cast<int>(n_), stream_), "sources");
             }
             substep();
         }
@@ -301,10 +302,7 @@ private:
 
     void finalize()
     {
-        const IWaveField f = field();
-        check(cudaMemcpyAsync(fields_.p + 2, &f, sizeof(f), cudaMemcpyHostToDevice, stream_), "fields");
-        check(launch_iwave_finalize(fields_.p + 2, 1, static_cast<int>(n_), stream_), "finalize");
-        check(cudaStreamSynchronize(stream_), "finalize");
+        check(launch_iwave_finalize(fields_.p + which_, 1, static_cast<int>(n_), stream_), "finalize");
     }
 
     void refresh_host()

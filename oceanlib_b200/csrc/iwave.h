@@ -40,17 +40,16 @@ struct IWaveSource {
     float mean;
     int32_t x0, x1, z0, z1;  // clipped box (inclusive)
 };
+static_assert(sizeof(IWaveSource) == 48 && offsetof(IWaveSource, x0) == 32, "a source's box is one 16-byte load");
 
 cudaError_t launch_iwave_step(int p, const IWaveField* fields, int count, int max_n,
                               const IWaveTaps& taps, cudaStream_t st);
 cudaError_t launch_iwave_finalize(const IWaveField* fields, int count, int max_n, cudaStream_t st);
 cudaError_t launch_source_mean(IWaveSource* sources, int count, cudaStream_t st);
-cudaError_t launch_source_apply(const IWaveField& f, const IWaveSource* sources, int count,
-                                cudaStream_t st);
-// `count` fields at once; field k adds sources [ranges[k].x, +ranges[k].y)
-// (ranges on the device, means already filled).
-cudaError_t launch_source_apply_batch(const IWaveField* fields, const int2* ranges,
-                                      const IWaveSource* sources, int count, int max_n, cudaStream_t st);
+// `count` fields at once; field k adds sources [r.x, r.x + r.y), r = ranges[k]
+// (on the device), or `one` with null ranges; means already filled.
+cudaError_t launch_source_apply(const IWaveField* fields, const int2* ranges, int2 one, const IWaveSource* sources,
+                                int count, int max_n, cudaStream_t st);
 cudaError_t launch_obstruction(const IWaveField& f, const uint32_t* solid, const uint32_t* nearest,
                                uint32_t count, bool dirichlet, cudaStream_t st);
 cudaError_t launch_shift(const float* src, float* dst, int n, int stride, int dx, int dz,

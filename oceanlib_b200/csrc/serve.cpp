@@ -990,8 +990,8 @@ private:
             for (const StepPart& sp : fp.steps) {
                 const IWaveField* fl = reinterpret_cast<const IWaveField*>(d + sp.fields);
                 if (sp.any_sources) {
-                    check(launch_source_apply_batch(fl, reinterpret_cast<const int2*>(d + sp.ranges), dev_src,
-                                                    static_cast<int>(sp.count), static_cast<int>(g.n), stream_),
+                    check(launch_source_apply(fl, reinterpret_cast<const int2*>(d + sp.ranges), int2{}, dev_src,
+                                              static_cast<int>(sp.count), static_cast<int>(g.n), stream_),
                           "sources");
                     ++kernels;
                 }
