@@ -429,8 +429,7 @@ float FoamField::foam_at(float world_x, float world_z) const noexcept
         check(cudaMemcpyAsync(m.q_in.p, m.host_q_in.p, sizeof(float2), cudaMemcpyHostToDevice, m.stream), "query");
         check(ocean_b200::launch_foam_at(static_cast<int>(m.n),
                                          static_cast<float>(m.n) / m.ocean->desc().patch_length, m.cell,
-                                         reinterpret_cast<const float4*>(d.displacement),
-                                         reinterpret_cast<const float4*>(d.normal), m.buf[m.cur].p, m.q_in.p, 1,
+                                         reinterpret_cast<const float4*>(d.displacement), m.buf[m.cur].p, m.q_in.p, 1,
                                          m.q_out.p, m.stream),
               "foam_at");
         check(cudaMemcpyAsync(m.host_q_out.p, m.q_out.p, sizeof(float), cudaMemcpyDeviceToHost, m.stream), "query");

@@ -1,11 +1,11 @@
 // oceanlib-b200: queries on the persistent foam field.
 //
 //   foam_at_kernel        FoamField::foam_at (src/foam.cpp:291-305): the
-//                         ocean's fixed-point inversion (sample_one, the same
-//                         as Ocean::sample_at) gives the parameter position of
+//                         ocean's fixed-point inversion (invert, the same
+//                         as Ocean::sample_at's) gives the parameter position of
 //                         the water at a world point; the foam grid is then
 //                         sampled there with the periodic bilinear fetch of
-//                         src/foam.cpp:22-41. One thread per point.
+//                         src/foam.cpp:22-41. A pair of lanes per point.
 //   foam_coverage_kernel  FoamField::coverage (src/foam.cpp:307-313): the mean
 //                         of the field in double. One CTA; every thread sums a
 //                         fixed strided subset and a fixed tree combines them,
@@ -19,16 +19,19 @@ namespace ocean_b200 {
 namespace {
 
 __global__ void foam_at_kernel(int n, float inv_cell, float cell, const float4* __restrict__ disp,
-                               const float4* __restrict__ normal, const float* __restrict__ foam,
+                               const float* __restrict__ foam,
                                const float2* __restrict__ xz, uint64_t count, float* __restrict__ out)
 {
-    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    const uint64_t at = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / qdev::kQueryLanes;
+    const uint64_t i = at < count ? at : count - 1;  // lanes past the end work along: the shuffles need whole warps
+    const uint32_t odd = threadIdx.x & 1u;
     const float2 p = xz[i];
-    // Only the offsets are used: no velocity taps.
-    const SurfaceEx s = qdev::sample_one(n, inv_cell, disp, normal, nullptr, p, 4, 0.0f);
-    const float u = (p.x - s.offset_x) / cell;
-    const float v = (p.y - s.offset_z) / cell;
+    const qdev::Inverted r = qdev::invert(static_cast<uint32_t>(n), inv_cell, disp, p, 4, 0.0f, odd);
+    const float off_x = qdev::pair_sum(r.d0.x * r.t.w0, r.d1.x * r.t.w1, odd);
+    const float off_z = qdev::pair_sum(r.d0.z * r.t.w0, r.d1.z * r.t.w1, odd);
+    if (odd || at >= count) return;
+    const float u = (p.x - off_x) / cell;
+    const float v = (p.y - off_z) / cell;
     auto get = [&](int z, int x) { return __ldg(&foam[static_cast<size_t>(z) * n + x]); };
     out[i] = foam_blend(foam_fetch(u, v, n, get));
 }
@@ -52,13 +55,12 @@ foam_coverage_kernel(const float* __restrict__ foam, uint64_t cells, double* __r
 
 }  // namespace
 
-cudaError_t launch_foam_at(int n, float inv_cell, float cell, const float4* disp, const float4* normal,
-                           const float* foam, const float2* xz, uint64_t count, float* out,
-                           cudaStream_t stream)
+cudaError_t launch_foam_at(int n, float inv_cell, float cell, const float4* disp, const float* foam,
+                           const float2* xz, uint64_t count, float* out, cudaStream_t stream)
 {
     if (count == 0) return cudaSuccess;
-    const unsigned blocks = static_cast<unsigned>((count + 255) / 256);
-    foam_at_kernel<<<blocks, 256, 0, stream>>>(n, inv_cell, cell, disp, normal, foam, xz, count, out);
+    const unsigned blocks = static_cast<unsigned>((qdev::kQueryLanes * count + 255) / 256);
+    foam_at_kernel<<<blocks, 256, 0, stream>>>(n, inv_cell, cell, disp, foam, xz, count, out);
     return cudaGetLastError();
 }
 

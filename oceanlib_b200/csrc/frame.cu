@@ -22,7 +22,6 @@
 // the other row already in shared memory, so h0 is read from HBM once.
 #include "frame_cells.cuh"
 #include "ocean_device.cuh"
-#include "query_device.cuh"
 #include "spectrum.h"
 #include "tc_dft.cuh"
 #include "tc_dft_small.cuh"
@@ -1190,72 +1189,6 @@ __global__ void foam_step_kernel(int n, int count, const float4* __restrict__ di
 }
 
 // ---------------------------------------------------------------------------
-// World queries (src/ocean.cpp:322-452; sample_one in query_device.cuh)
-// ---------------------------------------------------------------------------
-using qdev::sample_one;
-
-__global__ void sample_kernel(int n, float inv_cell, const float4* __restrict__ disp,
-                              const float4* __restrict__ normal, const float4* __restrict__ vel,
-                              const float2* __restrict__ xz, uint64_t count,
-                              SurfaceEx* __restrict__ out)
-{
-    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    out[i] = sample_one(n, inv_cell, disp, normal, vel, xz[i], 4, 0.0f);
-}
-
-// Summed surface of several cascade levels (src/cascade.cpp:82-153): height,
-// offsets and velocity add exactly; normals add then renormalise; foam
-// combines as 1 - prod(1 - foam_i). Levels are visited in order, so the float
-// sums round as the reference's loop does.
-__global__ void cascade_sample_kernel(CascadeLevels lv, const float2* __restrict__ xz,
-                                      uint64_t count, SurfaceEx* __restrict__ out, int iters,
-                                      float tol)
-{
-    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const float2 p = xz[i];
-    float height = 0.0f, offset_x = 0.0f, offset_z = 0.0f;
-    float normal_x = 0.0f, normal_y = 0.0f, normal_z = 0.0f;
-    float transparency = 1.0f;
-    float vx = 0.0f, vy = 0.0f, vz = 0.0f;
-    for (int l = 0; l < lv.count; ++l) {
-        const LevelView& L = lv.level[l];
-        const SurfaceEx s = sample_one(L.n, L.inv_cell, L.disp, L.normal, L.velocity, p, iters, tol);
-        height += s.height;
-        offset_x += s.offset_x;
-        offset_z += s.offset_z;
-        normal_x += s.normal_x;
-        normal_y += s.normal_y;
-        normal_z += s.normal_z;
-        vx += s.velocity_x;
-        vy += s.velocity_y;
-        vz += s.velocity_z;
-        transparency *= (1.0f - s.foam);
-    }
-    SurfaceEx o;
-    o.height = height;
-    o.offset_x = offset_x;
-    o.offset_z = offset_z;
-    o.foam = 1.0f - transparency;
-    o.velocity_x = vx;
-    o.velocity_y = vy;
-    o.velocity_z = vz;
-    const float len2 = normal_x * normal_x + normal_y * normal_y + normal_z * normal_z;
-    if (len2 > 0.0f) {
-        const float inv = 1.0f / sqrtf(len2);
-        o.normal_x = normal_x * inv;
-        o.normal_y = normal_y * inv;
-        o.normal_z = normal_z * inv;
-    } else {
-        o.normal_x = 0.0f;
-        o.normal_y = 1.0f;
-        o.normal_z = 0.0f;
-    }
-    out[i] = o;
-}
-
-// ---------------------------------------------------------------------------
 // Launch helpers: compile-time dispatch over (log N, fields, form, foam).
 // ---------------------------------------------------------------------------
 template <int LOG_N, int NF>
@@ -1555,25 +1488,6 @@ cudaError_t launch_foam_step(int n, int count, const float4* disp, const float4*
     const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
     foam_step_kernel<<<blocks, 256, 0, stream>>>(n, count, disp, velocity, cur, next, dt, decay,
                                                  gain, scale, drift_x, drift_z, inv_cell);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_cascade_sample(const CascadeLevels& levels, const float2* xz, uint64_t count,
-                                  SurfaceEx* out, int iters, float tol, cudaStream_t stream)
-{
-    if (count == 0) return cudaSuccess;
-    const unsigned blocks = static_cast<unsigned>((count + 255) / 256);
-    cascade_sample_kernel<<<blocks, 256, 0, stream>>>(levels, xz, count, out, iters, tol);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_sample(int n, float inv_cell, const float4* disp, const float4* normal,
-                          const float4* velocity, const float2* xz, uint64_t count,
-                          SurfaceEx* out, cudaStream_t stream)
-{
-    if (count == 0) return cudaSuccess;
-    const unsigned blocks = static_cast<unsigned>((count + 255) / 256);
-    sample_kernel<<<blocks, 256, 0, stream>>>(n, inv_cell, disp, normal, velocity, xz, count, out);
     return cudaGetLastError();
 }
 

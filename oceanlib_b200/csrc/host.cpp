@@ -359,7 +359,7 @@ public:
         const float cell = descs_[i].patch_length / static_cast<float>(n_);
         const float inv_cell = static_cast<float>(n_) / descs_[i].patch_length;
         check(cudaMemcpyAsync(q_in_.p, xz, count * sizeof(float2), cudaMemcpyHostToDevice, stream_), "query");
-        check(launch_foam_at(static_cast<int>(n_), inv_cell, cell, disp(i), normal(i), foam_ptr(i), q_in_.p,
+        check(launch_foam_at(static_cast<int>(n_), inv_cell, cell, disp(i), foam_ptr(i), q_in_.p,
                              count, q_out_.p, stream_), "foam_at kernel");
         check(cudaMemcpyAsync(out, q_out_.p, count * sizeof(float), cudaMemcpyDeviceToHost, stream_), "query");
         check(cudaStreamSynchronize(stream_), "query");

@@ -889,7 +889,6 @@ private:
             QueryJob j;
             std::memset(&j, 0, sizeof(j));
             j.disp = s.slot.disp;
-            j.normal = s.slot.normal;
             j.xz = reinterpret_cast<const float2*>(d + pts_off) + r->out_offset;
             j.out = dev_heights + r->out_offset;
             j.n = static_cast<int32_t>(s.od.size);

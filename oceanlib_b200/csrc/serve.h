@@ -10,7 +10,6 @@ namespace ocean_b200 {
 // (WaterSurface::height_at, src/interaction.cpp:903-908) at `count` points.
 struct QueryJob {
     const float4* disp;      // ocean displacement [n*n]
-    const float4* normal;    // ocean normal [n*n]
     const float2* xz;        // [count] world points
     float* out;              // [count] heights
     const float4* field;     // interaction output [fn*fn], or null (ocean alone)
