@@ -1171,21 +1171,20 @@ __global__ void wait_probe_kernel(const unsigned* counter, unsigned target, unsi
     }
 }
 
-__global__ void foam_step_kernel(int n, int count, const float4* __restrict__ disp,
-                                 const float4* __restrict__ vel, const float* __restrict__ cur,
-                                 float* __restrict__ next, float dt, float decay, float gain,
-                                 float scale, float drift_x, float drift_z, float inv_cell)
+// One thread per cell, blockIdx.y = ocean: n is a power of two, so a cell's
+// row and column are a shift and a mask of its index.
+__global__ void __launch_bounds__(256)
+foam_step_kernel(int log_n, const float4* __restrict__ disp, const float4* __restrict__ vel,
+                 const float* __restrict__ cur, float* __restrict__ next, float dt, float decay, float gain,
+                 float scale, float drift_x, float drift_z, float inv_cell)
 {
-    const uint64_t cells = static_cast<uint64_t>(n) * n;
-    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= cells * count) return;
-    const uint64_t o = i / cells;
-    const uint64_t c = i % cells;
-    const int z = static_cast<int>(c / n), x = static_cast<int>(c % n);
-    const float4 v = vel[i];
-    const float src = disp[i].w;
-    next[i] = foam_cell(cur + o * cells, n, x, z, v.x, v.z, src, dt, decay, gain, scale, drift_x,
-                        drift_z, inv_cell);
+    const int n = 1 << log_n;
+    const unsigned c = blockIdx.x * 256u + threadIdx.x;
+    const size_t base = static_cast<size_t>(blockIdx.y) << (2 * log_n);
+    const int z = static_cast<int>(c >> log_n), x = static_cast<int>(c & (n - 1));
+    const float4 v = vel[base + c];
+    const float src = disp[base + c].w;
+    next[base + c] = foam_cell(cur + base, n, x, z, v.x, v.z, src, dt, decay, gain, scale, drift_x, drift_z, inv_cell);
 }
 
 // ---------------------------------------------------------------------------
@@ -1484,10 +1483,18 @@ cudaError_t launch_foam_step(int n, int count, const float4* disp, const float4*
                              float scale, float drift_x, float drift_z, float inv_cell,
                              cudaStream_t stream)
 {
-    const uint64_t total = static_cast<uint64_t>(n) * n * count;
-    const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-    foam_step_kernel<<<blocks, 256, 0, stream>>>(n, count, disp, velocity, cur, next, dt, decay,
-                                                 gain, scale, drift_x, drift_z, inv_cell);
+    if (count == 0) return cudaSuccess;
+    if (n < 16 || (n & (n - 1)) != 0) return cudaErrorInvalidValue;
+    int log_n = 0;
+    while ((1 << log_n) < n) ++log_n;
+    // 65535 oceans a launch (the grid's y limit).
+    const size_t cells = static_cast<size_t>(n) * n;
+    for (int o = 0; o < count; o += 65535) {
+        const size_t at = o * cells;
+        const dim3 grid(static_cast<unsigned>(cells / 256), static_cast<unsigned>(count - o < 65535 ? count - o : 65535));
+        foam_step_kernel<<<grid, 256, 0, stream>>>(log_n, disp + at, velocity + at, cur + at, next + at, dt, decay, gain,
+                                                   scale, drift_x, drift_z, inv_cell);
+    }
     return cudaGetLastError();
 }
 

@@ -8,51 +8,72 @@
 
 namespace ocean_b200 {
 
-// The evolved spectra of one cell (src/core/evolve.cpp:28-121, and :123-184
+// The evolved amplitude of one cell (src/core/evolve.cpp:28-121, and :123-184
 // for the velocity fields): h0(k) = av, h0(-k) = bm (conjugated here), the
-// cell's (omega, 1/|k|) = wk and wavenumbers kx, kz, at t / 2pi = top. The
-// eight real spectra are packed two per complex field (A + iB) into p[0..3],
-// the velocity spectra into p[4..5] when NF = 6.
-template <int NF>
-__device__ __forceinline__ void evolve_cell(float2 av, float2 bm, float2 wk, float kx, float kz, double top,
-                                            float2 (&p)[NF])
+// cell's omega, at t / 2pi = top. (hr, hi) is h(k, t) and (dr, di) the
+// difference of its two waves.
+struct Amplitude {
+    float hr, hi, dr, di;
+};
+
+__device__ __forceinline__ Amplitude evolve_amplitude(float2 av, float2 bm, float omega, double top)
 {
     const float b_re = bm.x, b_im = -bm.y;
     float s, c;
-    sincos_poly(fold_phase(wk.x, top), s, c);
+    sincos_poly(fold_phase(omega, top), s, c);
     const float fwd_re = av.x * c - av.y * s;
     const float fwd_im = av.x * s + av.y * c;
     const float bwd_re = b_re * c + b_im * s;
     const float bwd_im = b_im * c - b_re * s;
-    const float hr = fwd_re + bwd_re;
-    const float hi = fwd_im + bwd_im;
-    const float ki = wk.y;
+    return {fwd_re + bwd_re, fwd_im + bwd_im, fwd_re - bwd_re, fwd_im - bwd_im};
+}
+
+// The cell's eight real spectra, packed two per complex field (A + iB): fields
+// 0 and 1, 2 and 3, and the velocity fields 4 and 5. ki = 1/|k|.
+__device__ __forceinline__ void evolve_pair0(float hr, float hi, float ki, float kx, float kz, float2& p0, float2& p1)
+{
     const float sx = kx * ki;
     const float sz = kz * ki;
     const float dx_re = sx * hi, dx_im = -sx * hr;
     const float dz_re = sz * hi, dz_im = -sz * hr;
     const float hx_re = -kx * hi, hx_im = kx * hr;
+    p0 = make_float2(hr - dx_im, hi + dx_re);
+    p1 = make_float2(dz_re - hx_im, dz_im + hx_re);
+}
+__device__ __forceinline__ void evolve_pair1(float hr, float hi, float ki, float kx, float kz, float2& p2, float2& p3)
+{
+    const float sx = kx * ki;
+    const float sz = kz * ki;
     const float hz_re = -kz * hi, hz_im = kz * hr;
     const float jxx = kx * sx, jzz = kz * sz, jxz = kx * sz;
     const float jxx_re = jxx * hr, jxx_im = jxx * hi;
     const float jzz_re = jzz * hr, jzz_im = jzz * hi;
     const float jxz_re = jxz * hr, jxz_im = jxz * hi;
+    p2 = make_float2(hz_re - jxx_im, hz_im + jxx_re);
+    p3 = make_float2(jzz_re - jxz_im, jzz_im + jxz_re);
+}
+__device__ __forceinline__ void evolve_pair2(float dr, float di, float omega, float ki, float kx, float kz, float2& p4,
+                                             float2& p5)
+{
+    const float sx = kx * ki;
+    const float sz = kz * ki;
+    const float wsx = omega * sx, wsz = omega * sz;
+    const float ux_re = -wsx * dr, ux_im = -wsx * di;
+    const float uz_re = -wsz * dr, uz_im = -wsz * di;
+    const float uy_re = -omega * di, uy_im = omega * dr;
+    p4 = make_float2(ux_re - uy_im, ux_im + uy_re);
+    p5 = make_float2(uz_re, uz_im);
+}
 
-    p[0] = make_float2(hr - dx_im, hi + dx_re);
-    p[1] = make_float2(dz_re - hx_im, dz_im + hx_re);
-    p[2] = make_float2(hz_re - jxx_im, hz_im + jxx_re);
-    p[3] = make_float2(jzz_re - jxz_im, jzz_im + jxz_re);
-    if constexpr (NF == 6) {
-        const float dr = fwd_re - bwd_re;
-        const float di = fwd_im - bwd_im;
-        const float w = wk.x;
-        const float wsx = w * sx, wsz = w * sz;
-        const float ux_re = -wsx * dr, ux_im = -wsx * di;
-        const float uz_re = -wsz * dr, uz_im = -wsz * di;
-        const float uy_re = -w * di, uy_im = w * dr;
-        p[4] = make_float2(ux_re - uy_im, ux_im + uy_re);
-        p[5] = make_float2(uz_re, uz_im);
-    }
+// All NF fields of one cell, wk = (omega, 1/|k|).
+template <int NF>
+__device__ __forceinline__ void evolve_cell(float2 av, float2 bm, float2 wk, float kx, float kz, double top,
+                                            float2 (&p)[NF])
+{
+    const Amplitude a = evolve_amplitude(av, bm, wk.x, top);
+    evolve_pair0(a.hr, a.hi, wk.y, kx, kz, p[0], p[1]);
+    evolve_pair1(a.hr, a.hi, wk.y, kx, kz, p[2], p[3]);
+    if constexpr (NF == 6) evolve_pair2(a.dr, a.di, wk.x, wk.y, kx, kz, p[4], p[5]);
 }
 
 // Displacement (lambda Dx, h, lambda Dz, foam) and normal (n, Jacobian) of one
@@ -102,12 +123,11 @@ __device__ __forceinline__ FoamTaps foam_fetch(float u, float v, int n, Get&& ge
     const float fu = floorf(u), fv = floorf(v);
     t.tu = u - fu;
     t.tv = v - fv;
-    int x0 = __float2int_rz(fu) % n;
-    if (x0 < 0) x0 += n;
-    int z0 = __float2int_rz(fv) % n;
-    if (z0 < 0) z0 += n;
-    const int x1 = (x0 + 1) % n;
-    const int z1 = (z0 + 1) % n;
+    // n is a power of two: masking wraps negative indices too.
+    const int x0 = __float2int_rz(fu) & (n - 1);
+    const int z0 = __float2int_rz(fv) & (n - 1);
+    const int x1 = (x0 + 1) & (n - 1);
+    const int z1 = (z0 + 1) & (n - 1);
     t.fa = get(z0, x0);
     t.fb = get(z0, x1);
     t.fc = get(z1, x0);

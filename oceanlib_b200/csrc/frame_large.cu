@@ -3,28 +3,55 @@
 // The persistent frame kernel (frame.cu) keeps every field of a row pair, or
 // of a strip of columns, in one CTA's shared memory. Above N = 1024 that no
 // longer fits: six 4096-point sequences alone are 209 KB. These sizes (the
-// reference accepts N up to 4096, src/ocean.cpp:28-59) run three passes per
-// chunk of oceans instead, through a field-major intermediate
-// inter[ocean][field][y][x]:
+// reference accepts N up to 4096, src/ocean.cpp:28-59) run two passes per
+// chunk of oceans instead, through an intermediate that crosses HBM once each
+// way (800 MB at 4096 with velocity, beyond the L2):
 //
-//   rows      row y per task: evolve the row's cells once for all NF fields
-//             (src/core/evolve.cpp:28-184; h0(-k) read from the mirrored row
-//             in global memory, which the neighbouring task has just read),
-//             field pair 0 into shared memory and the other pairs straight
-//             into their rows of the intermediate; transform pair 0, then
-//             each other pair from its row (just written, so read from L2)
-//             back in place.
-//   columns   four columns of one field per task, transformed in place.
-//   finalize  one thread per cell: the NF fields to the RGBA32F outputs
-//             (src/core/evolve.cpp:186-327) and, with persistent foam, the
-//             first foam substep (src/foam.cpp:89-139).
+//   rows      two neighbouring rows per task: evolve the rows' cells once
+//             (src/core/evolve.cpp:28-184), then field pair by field pair
+//             transform the rows and write them to the intermediate;
+//   columns   two neighbouring columns per task: field pair by field pair
+//             read and transform the columns, then finalize every cell
+//             (src/core/evolve.cpp:186-327) into the RGBA32F outputs.
 //
-// A sequence spans N/16 lanes holding 16 values each (4-stage blocks, three
-// passes through shared memory at both sizes), i.e. several warps, which
-// synchronise with the CTA barrier. Evolve, butterflies, twiddles, finalize
-// and foam are the persistent kernel's own functions (frame_cells.cuh,
-// ocean_device.cuh), so these sizes match the reference bit for bit too.
-// A CTA runs several tasks so that each twiddle table load serves them all.
+// Persistent foam runs every substep as its own launch at these sizes: a
+// column strip's foam taps are scattered four-byte reads (4096^2 with velocity
+// and foam: 1448 us fused, 1151 us apart).
+//
+// What bounds a pass is shared memory (capacity and wavefronts) and the phases
+// between barriers, so values stay in registers wherever a thread needs them
+// again:
+//   * A sequence pair (fields 2q and 2q+1, packed f32x2 arithmetic) spans
+//     N / 16 lanes of 16 indices each: 4-stage register blocks, and only the
+//     two exchanges between the three blocks go through shared memory, real
+//     and imaginary parts one after the other in the same 8 bytes per index.
+//     The first block takes its values straight from evolve or from global
+//     memory (index c + j N/16 in lane c), and the last leaves the same
+//     indices in the same lane, straight for the intermediate or finalize.
+//   * The evolved amplitudes (rows) and the transformed first field pair
+//     (columns) wait for the later pairs in their own thread's slots of
+//     shared memory. The velocity pair goes first: nothing of it is needed
+//     afterwards.
+// The intermediate is inter[ocean][x / 2][pair][y][x & 1], 16 bytes (a.re,
+// b.re, a.im, b.im) a cell and pair: a column task's pair is one contiguous
+// run, which a bulk prefetch brings into the L2 while the pair before it is
+// transformed. Threads 2c and 2c + 1 are lane c of the task's two rows
+// (columns), so a warp's stores to the intermediate are 64-byte runs and those
+// to the outputs whole 32-byte sectors.
+//
+// Measured, one ocean with velocity: 4096^2 1618 -> 960 us, 2048^2 376 -> 260 us
+// a frame against rows, columns and finalize as three passes that each moved
+// every field through HBM; without velocity 1081 -> 667 and 253 -> 190 us;
+// the precise form at 4096^2 with velocity 2524 -> 1590 us. What is left at
+// 4096^2: FP32 pipe time of about 23k of a task's 63k cycles, exchanges 14k
+// (16 warps in one phase), loads from the L2 and stores 12k each. Without the
+// output stores 837 us, without the prefetches 1055 us. Keeping the second
+// exchange inside a warp by regrouping the lanes (no CTA barrier) was slower
+// (978 -> 1063 us): it halves the runs that the rows store.
+//
+// Evolve, butterflies, twiddles and finalize are the persistent kernel's own
+// functions (frame_cells.cuh, ocean_device.cuh), so these sizes match the
+// reference bit for bit too.
 #include "frame_cells.cuh"
 #include "ocean_device.cuh"
 #include "spectrum.h"
@@ -37,187 +64,367 @@ namespace {
 template <int LOG_N>
 struct Large {
     static constexpr int N = 1 << LOG_N;
-    static constexpr int G = N / 16;               // lanes per sequence
-    static constexpr int SEQ = padded_len(N) + 4;  // sequence stride (float2)
-    static constexpr int W = 4;                    // columns per column task
-    static constexpr int ROW_T = 2 * G;            // threads: two sequences
-    static constexpr int COL_T = W * G;            // threads: W sequences
-    static constexpr int ROW_TASKS = 2;            // rows per row CTA (a row and its mirror)
-    // Resident row CTAs per SM the registers are capped for: two at N = 4096
-    // (512 threads, 102 KB each; 7% faster than one), three at 2048 (256
-    // threads, 51 KB each).
-    static constexpr int ROW_BLOCKS = LOG_N >= 12 ? 2 : 3;
-    static constexpr int COL_TASKS = 2;            // tasks per column CTA
-    static constexpr size_t ROW_SMEM = sizeof(float2) * (2 * SEQ + N - 1);
-    static constexpr size_t COL_SMEM = sizeof(float2) * (W * SEQ + N - 1);
-    static_assert(COL_SMEM <= 227 * 1024, "a column CTA fits in shared memory");
+    static constexpr int G = N / 16;                // lanes per sequence pair
+    static constexpr int THREADS = 2 * G;           // two rows (columns) per task
+    static constexpr int CTAS = 512 / THREADS;      // resident per SM: 128 registers a thread
+    static constexpr int TASKS = N / 2;             // per ocean and pass
+    static constexpr int SEQ = padded_len(N) + 8;   // exchange stride (f32x2): the two rows 8 bank pairs apart
+    static constexpr int HELD = 15;                 // of a thread's 16 cells, those the column stash holds
+    static constexpr int BUF = 2 * SEQ;
+    static constexpr size_t EXCHANGE = sizeof(f32x2) * BUF;
+    static constexpr size_t TWIDDLES = sizeof(float2) * N;
+    static constexpr size_t ROW_SMEM = EXCHANGE + TWIDDLES + (sizeof(float2) + sizeof(float)) * 16 * THREADS + sizeof(float) * N;
+    static constexpr size_t COL_SMEM = EXCHANGE + TWIDDLES + sizeof(float4) * HELD * THREADS;
+    static_assert((COL_SMEM + 1024) * CTAS <= 228 * 1024 && COL_SMEM <= 227 * 1024, "the column CTAs fit on an SM");
+    static_assert((ROW_SMEM + 1024) * CTAS <= 228 * 1024 && ROW_SMEM <= 227 * 1024, "the row CTAs fit on an SM");
 };
 
-template <int LOG_N, int NF, int AR>
-__global__ void __launch_bounds__(Large<LOG_N>::ROW_T, Large<LOG_N>::ROW_BLOCKS)
-large_row_kernel(FrameArgs a)
-{
-    using S = Large<LOG_N>;
-    constexpr int N = S::N, NT = S::ROW_T, SEQ = S::SEQ, G = S::G;
-    constexpr int NG = NF / 2;  // field pairs per row
-    extern __shared__ float4 smem4[];
-    float2* data = reinterpret_cast<float2*>(smem4);  // the task's two sequences
-    float2* tws = data + 2 * SEQ;
-    const int tid = threadIdx.x;
-    const int o = blockIdx.y;
-    const int ocean = a.ocean_base + o;
-    const OceanConsts cst = a.consts[ocean];
-    const size_t cells = static_cast<size_t>(N) * N;
-    const float2* h0 = a.h0 + static_cast<size_t>(ocean) * cells;
-    const float2* geom = a.omega_kinv + static_cast<size_t>(cst.geom) * cells;
-    const float* kvec = a.kvec + static_cast<size_t>(cst.geom) * N;
-    const double top = a.t_over_2pi[ocean];
-    float2* inter = a.inter + static_cast<size_t>(o) * NF * cells;
-    for (int i = tid; i < N - 1; i += NT) tws[i] = __ldg(&a.twiddles[i]);
+// A thread's place: row (column) r of the task's two, lane c of its pair, and
+// that row's exchange buffer.
+template <int LOG_N>
+struct Place {
+    int r, c;
+    f32x2* buf;
 
-#pragma unroll 1
-    for (int k = 0; k < S::ROW_TASKS; ++k) {
-        // Task t: row slot t, whose two members (p, N - p), or (0, N/2) for
-        // p = 0, are each other's h0(-k) rows, so consecutive tasks reuse
-        // what the L2 just fetched.
-        const int j = blockIdx.x * S::ROW_TASKS + k;
-        const int p = j >> 1, r = j & 1;
-        const int y = p == 0 ? (r ? N / 2 : 0) : (r ? N - p : p);
-        const int my = (N - y) & (N - 1);
-        const float kz = __ldg(&kvec[y]);
-        const size_t row = static_cast<size_t>(y) * N;
-        __syncthreads();  // the twiddles are complete; the last task's reads are done
-        // Evolve once: pair 0 to shared memory, pairs 1.. to their rows of
-        // the intermediate (coalesced float2 stores, read back below).
-        for (int x = tid; x < N; x += NT) {
-            const float2 av = __ldg(&h0[row + x]);
-            const float2 bm = __ldg(&h0[static_cast<size_t>(my) * N + ((N - x) & (N - 1))]);
-            float2 pv[NF];
-            evolve_cell<NF>(av, bm, __ldg(&geom[row + x]), __ldg(&kvec[x]), kz, top, pv);
-            data[pad_idx(x)] = pv[0];
-            data[SEQ + pad_idx(x)] = pv[1];
+    __device__ __forceinline__ explicit Place(void* smem)
+        : r(threadIdx.x & 1), c(threadIdx.x >> 1), buf(static_cast<f32x2*>(smem) + r * Large<LOG_N>::SEQ)
+    {
+    }
+};
+
+// The unnormalised inverse transform of a pair of sequences whose index
+// c + j N/16 is in slot j; afterwards slot j holds index(j).
+template <int LOG_N, int AR>
+struct LargeFft {
+    static constexpr int G = Large<LOG_N>::G;
+    using B0 = PairBlock<LOG_N, G, 0, AR>;
+    using B1 = PairBlock<LOG_N, G, 4, AR>;
+    using B2 = PairBlock<LOG_N, G, 8, AR>;
+    static_assert(B0::r == 4 && B1::r == 4 && 8 + B2::r == LOG_N, "three blocks cover the stages");
+
+    // Hands 8 bytes of every slot from one block to the next: a part of the
+    // pair, or both parts of one sequence.
+    template <class From, class To>
+    __device__ __forceinline__ static void exchange(f32x2 (&v)[16], f32x2* buf, int c)
+    {
+        static_assert(From::C * From::RR == 16 && To::C * To::RR == 16, "16 slots");
+        __syncthreads();  // the buffer's last readers are done
 #pragma unroll
-            for (int f = 2; f < NF; ++f) inter[static_cast<size_t>(f) * cells + row + x] = pv[f];
-        }
+        for (int j = 0; j < 16; ++j) buf[pad_idx(From::index_after(j / From::RR, j % From::RR, c))] = v[j];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = buf[pad_idx(To::index_before(j / To::RR, j % To::RR, c))];
+    }
+    template <class From, class To>
+    __device__ __forceinline__ static void exchange(float (&x)[16], float (&y)[16], f32x2* buf, int c)
+    {
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            buf[pad_idx(From::index_after(j / From::RR, j % From::RR, c))] = px_pack(x[j], y[j]);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) px_unpack(buf[pad_idx(To::index_before(j / To::RR, j % To::RR, c))], x[j], y[j]);
+    }
+
+    template <class B>
+    __device__ __forceinline__ static void block(f32x2 (&re)[16], f32x2 (&im)[16], const float2* tw, int c)
+    {
+        B::compute(reinterpret_cast<f32x2(&)[B::C][B::RR]>(re), reinterpret_cast<f32x2(&)[B::C][B::RR]>(im), tw, c);
+    }
+    template <class B>
+    __device__ __forceinline__ static void block(float (&x)[16], float (&y)[16], const float2* tw, int c)
+    {
+        B::compute_f64(reinterpret_cast<float(&)[B::C][B::RR]>(x), reinterpret_cast<float(&)[B::C][B::RR]>(y), tw, c);
+    }
+
+    __device__ __forceinline__ static void run(f32x2 (&re)[16], f32x2 (&im)[16], const float2* tw, const Place<LOG_N>& p)
+    {
+        if constexpr (AR == kArPrecise) {
+            // The two sequences one after the other, so that the FP64 values
+            // of one block (64 registers) and the other sequence's FP32 values
+            // (32) are all a lane holds.
+            float ax[16], ay[16], bx[16], by[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                px_unpack(re[j], ax[j], bx[j]);
+                px_unpack(im[j], ay[j], by[j]);
+            }
 #pragma unroll 1
-        for (int g = 0; g < NG; ++g) {
-            if (g > 0) {
-                __syncthreads();  // the last pair's outputs are read out of shared memory
-                // This CTA wrote the pair's row above; the barrier makes its
-                // stores visible, and the loads go to L2.
-                for (int i = tid; i < 2 * N; i += NT) {
-                    const int s = i >> LOG_N, x = i & (N - 1);
-                    data[s * SEQ + pad_idx(x)] = __ldcg(&inter[static_cast<size_t>(2 * g + s) * cells + row + x]);
+            for (int h = 0; h < 2; ++h) {
+                block<B0>(ax, ay, tw, p.c);
+                exchange<B0, B1>(ax, ay, p.buf, p.c);
+                block<B1>(ax, ay, tw, p.c);
+                exchange<B1, B2>(ax, ay, p.buf, p.c);
+                block<B2>(ax, ay, tw, p.c);
+                // The sequences change places: twice round is the original order.
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float tx = ax[j], ty = ay[j];
+                    ax[j] = bx[j];
+                    ay[j] = by[j];
+                    bx[j] = tx;
+                    by[j] = ty;
                 }
             }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                re[j] = px_pack(ax[j], bx[j]);
+                im[j] = px_pack(ay[j], by[j]);
+            }
+        } else {
+            block<B0>(re, im, tw, p.c);
+            exchange<B0, B1>(re, p.buf, p.c);
+            exchange<B0, B1>(im, p.buf, p.c);
+            block<B1>(re, im, tw, p.c);
+            exchange<B1, B2>(re, p.buf, p.c);
+            exchange<B1, B2>(im, p.buf, p.c);
+            block<B2>(re, im, tw, p.c);
+        }
+    }
+    __device__ __forceinline__ static int index(int j, const Place<LOG_N>& p)
+    {
+        return B2::index_after(j / B2::RR, j % B2::RR, p.c);
+    }
+};
+
+// Brings `bytes` (a multiple of 16 KB) at `p` into the L2: threads
+// [first, first + bytes / 16 KB) of the CTA take a piece each.
+__device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes, int first)
+{
+    constexpr unsigned kPiece = 16384;
+    const unsigned k = threadIdx.x - first;
+    if (k < bytes / kPiece)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(static_cast<const char*>(p) + k * kPiece),
+                     "r"(kPiece)
+                     : "memory");
+}
+
+template <int LOG_N>
+__device__ __forceinline__ void load_twiddles(float2* tws, const float2* __restrict__ src)
+{
+    for (int i = threadIdx.x; i < Large<LOG_N>::N - 1; i += Large<LOG_N>::THREADS) tws[i] = __ldg(&src[i]);
+}
+
+// A read-only load that stays where it is written.
+__device__ __forceinline__ float2 load_now(const float2* p)
+{
+    float2 v;
+    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+
+template <int LOG_N, int NF, int AR>
+__global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) large_row_kernel(FrameArgs a)
+{
+    using S = Large<LOG_N>;
+    using Fft = LargeFft<LOG_N, AR>;
+    constexpr int N = S::N, G = S::G, Q = NF / 2, NT = S::THREADS;
+    extern __shared__ float4 smem4[];
+    const int tid = threadIdx.x;
+    const Place<LOG_N> p(smem4);
+    float2* tws = reinterpret_cast<float2*>(smem4) + S::BUF;
+    float* kv = reinterpret_cast<float*>(tws + N);
+    float2* held_h = reinterpret_cast<float2*>(kv + N) + tid;                   // (hr, hi) of cell j at [j * NT]
+    float* held_k = reinterpret_cast<float*>(held_h - tid + 16 * NT) + tid;     // its 1/|k|
+    load_twiddles<LOG_N>(tws, a.twiddles);
+
+    const size_t cells = static_cast<size_t>(N) * N;
+    const int tasks = S::TASKS * a.chunk;
+    // Task t's rows are y and y + 1. Rows 2k, 2k + 1 and the rows with their
+    // mirrors are neighbouring tasks, which share what the L2 fetched.
+    auto first_row = [](int t) { return 2 * ((t & 1) ? S::TASKS - 1 - (t >> 1) : (t >> 1)); };
+    int kv_of = -1;
+#pragma unroll 1
+    for (int task = blockIdx.x; task < tasks; task += gridDim.x) {
+        const int o = task / S::TASKS;
+        const int y = first_row(task % S::TASKS) + p.r;
+        const int ocean = a.ocean_base + o;
+        const int geom_of = a.consts[ocean].geom;
+        const float2* h0 = a.h0 + static_cast<size_t>(ocean) * cells;
+        const float2* h0_row = h0 + static_cast<size_t>(y) * N;
+        const float2* h0_mirror = h0 + static_cast<size_t>((N - y) & (N - 1)) * N;
+        const float2* geom = a.omega_kinv + static_cast<size_t>(geom_of) * cells + static_cast<size_t>(y) * N;
+        if (geom_of != kv_of) {
+            __syncthreads();  // the table's last readers are done
+            for (int i = tid; i < N; i += NT) kv[i] = __ldg(&a.kvec[static_cast<size_t>(geom_of) * N + i]);
             __syncthreads();
-            fft_sequence<LOG_N, G, AR>(data + (tid / G) * SEQ, tws, tid % G);  // ends with a CTA barrier
-            float2* out = inter + static_cast<size_t>(2 * g) * cells + row;
-            for (int i = tid; i < 2 * N; i += NT) {
-                const int s = i >> LOG_N, x = i & (N - 1);
-                out[static_cast<size_t>(s) * cells + x] = data[s * SEQ + pad_idx(x)];
+            kv_of = geom_of;
+        }
+        const float kz = kv[y];
+        const double top = a.t_over_2pi[ocean];
+        ulonglong2* out = reinterpret_cast<ulonglong2*>(a.inter + static_cast<size_t>(o) * NF * cells) + 2 * y;
+#pragma unroll 1
+        for (int k = 0; k < Q; ++k) {
+            const int q = Q == 3 ? (k + 2) % 3 : k;  // the velocity pair first
+            f32x2 re[16], im[16];
+            if (k == 0) {
+                // Every cell's loads before the first is evolved: 96 registers
+                // that the fields then take over.
+                float2 av[16], bm[16], wks[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const int x = p.c + G * j;
+                    av[j] = load_now(&h0_row[x]);
+                    bm[j] = load_now(&h0_mirror[(N - x) & (N - 1)]);
+                    wks[j] = load_now(&geom[x]);
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const int x = p.c + G * j;
+                    const float2 wk = wks[j];
+                    const Amplitude e = evolve_amplitude(av[j], bm[j], wk.x, top);
+                    held_h[j * NT] = make_float2(e.hr, e.hi);
+                    held_k[j * NT] = wk.y;
+                    float2 pa, pb;
+                    if constexpr (Q == 3) {
+                        evolve_pair2(e.dr, e.di, wk.x, wk.y, kv[x], kz, pa, pb);
+                    } else {
+                        evolve_pair0(e.hr, e.hi, wk.y, kv[x], kz, pa, pb);
+                    }
+                    re[j] = px_pack(pa.x, pb.x);
+                    im[j] = px_pack(pa.y, pb.y);
+                }
+                // The next task's rows while this one's are transformed.
+                if (task + static_cast<int>(gridDim.x) < tasks) {
+                    const int next = task + gridDim.x, no = a.ocean_base + next / S::TASKS;
+                    const int ny = first_row(next % S::TASKS);
+                    const float2* nh = a.h0 + static_cast<size_t>(no) * cells;
+                    const float2* ng = a.omega_kinv + static_cast<size_t>(a.consts[no].geom) * cells;
+                    constexpr unsigned kRows = 2u * N * sizeof(float2);
+                    prefetch_l2(nh + static_cast<size_t>(ny) * N, kRows, 0);
+                    prefetch_l2(ng + static_cast<size_t>(ny) * N, kRows, 32);
+                    // Rows N - y - 1 and N - y; row N - 1 alone for y = 0.
+                    prefetch_l2(nh + static_cast<size_t>(N - ny - 1) * N, ny == 0 ? kRows / 2 : kRows, 64);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float kx = kv[p.c + G * j];
+                    const float2 h = held_h[j * NT];
+                    const float ki = held_k[j * NT];
+                    float2 pa, pb;
+                    if (Q == 3 && q == 0) {
+                        evolve_pair0(h.x, h.y, ki, kx, kz, pa, pb);
+                    } else {
+                        evolve_pair1(h.x, h.y, ki, kx, kz, pa, pb);
+                    }
+                    re[j] = px_pack(pa.x, pb.x);
+                    im[j] = px_pack(pa.y, pb.y);
+                }
+            }
+            Fft::run(re, im, tws, p);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const int x = Fft::index(j, p);
+                out[(static_cast<size_t>(x >> 1) * Q + q) * 2 * N + (x & 1)] = make_ulonglong2(re[j], im[j]);
             }
         }
     }
 }
 
-template <int LOG_N, int AR>
-__global__ void __launch_bounds__(Large<LOG_N>::COL_T) large_col_kernel(FrameArgs a, int nf)
+template <int LOG_N, int NF, int AR>
+__global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) large_col_kernel(FrameArgs a)
 {
     using S = Large<LOG_N>;
-    constexpr int N = S::N, NT = S::COL_T, SEQ = S::SEQ, G = S::G, W = S::W;
-    constexpr int H = W / 2;  // float4 (two columns) per row of a strip
+    using Fft = LargeFft<LOG_N, AR>;
+    constexpr int N = S::N, Q = NF / 2, NT = S::THREADS;
+    constexpr unsigned kPairBytes = 2u * N * sizeof(float4);  // a task's pair
     extern __shared__ float4 smem4[];
-    float2* data = reinterpret_cast<float2*>(smem4);  // the task's W sequences
-    float2* tws = data + W * SEQ;
     const int tid = threadIdx.x;
-    const int o = blockIdx.y;
-    const size_t cells = static_cast<size_t>(N) * N;
-    for (int i = tid; i < N - 1; i += NT) tws[i] = __ldg(&a.twiddles[i]);
+    const Place<LOG_N> p(smem4);
+    float2* tws = reinterpret_cast<float2*>(smem4) + S::BUF;
+    ulonglong2* held = reinterpret_cast<ulonglong2*>(tws + N) + tid;  // pair 0 of cell j at [j * NT]
+    load_twiddles<LOG_N>(tws, a.twiddles);
+    __syncthreads();
 
+    const size_t cells = static_cast<size_t>(N) * N;
+    const int tasks = S::TASKS * a.chunk;
+    // Pair q of a task's two columns; the chunk's oceans follow each other.
+    auto pair_at = [&](int task, int q) {
+        return reinterpret_cast<const float4*>(a.inter) + (static_cast<size_t>(task) * Q + q) * 2 * N;
+    };
 #pragma unroll 1
-    for (int k = 0; k < S::COL_TASKS; ++k) {
-        // Task t: strip t % (N / W) of field t / (N / W); neighbouring CTAs
-        // take neighbouring strips, which share the rows' cache lines.
-        const int t = blockIdx.x * S::COL_TASKS + k;
-        const int f = t / (N / W);
-        const int x0 = (t % (N / W)) * W;
-        float2* plane = a.inter + (static_cast<size_t>(o) * nf + f) * cells;
-        __syncthreads();  // the twiddles are complete; the last task's reads are done
-        for (int i = tid; i < N * H; i += NT) {
-            const int y = i / H, h = i % H;
-            const float4 v = reinterpret_cast<const float4*>(plane + static_cast<size_t>(y) * N + x0)[h];
-            data[(2 * h) * SEQ + pad_idx(y)] = make_float2(v.x, v.y);
-            data[(2 * h + 1) * SEQ + pad_idx(y)] = make_float2(v.z, v.w);
-        }
-        __syncthreads();
-        fft_sequence<LOG_N, G, AR>(data + (tid / G) * SEQ, tws, tid % G);  // ends with a CTA barrier
-        for (int i = tid; i < N * H; i += NT) {
-            const int y = i / H, h = i % H;
-            const float2 u = data[(2 * h) * SEQ + pad_idx(y)];
-            const float2 v = data[(2 * h + 1) * SEQ + pad_idx(y)];
-            reinterpret_cast<float4*>(plane + static_cast<size_t>(y) * N + x0)[h] = make_float4(u.x, u.y, v.x, v.y);
+    for (int task = blockIdx.x; task < tasks; task += gridDim.x) {
+        ulonglong2 last;  // pair 0 of the 16th cell
+#pragma unroll 1
+        for (int k = 0; k < Q; ++k) {
+            // The velocity pair first, the pair that completes the cell last.
+            const int q = Q == 3 ? (k + 2) % 3 : k;
+            if (k + 1 < Q) {
+                prefetch_l2(pair_at(task, Q == 3 ? k : k + 1), kPairBytes, 0);
+            } else if (task + static_cast<int>(gridDim.x) < tasks) {
+                prefetch_l2(pair_at(task + gridDim.x, Q == 3 ? 2 : 0), kPairBytes, 0);
+            }
+            const float4* src = pair_at(task, q) + tid;
+            f32x2 re[16], im[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const float4 v = __ldcs(src + NT * j);
+                re[j] = px_pack(v.x, v.y);
+                im[j] = px_pack(v.z, v.w);
+            }
+            Fft::run(re, im, tws, p);
+            const int ocean = a.ocean_base + task / S::TASKS;
+            const size_t base = static_cast<size_t>(ocean) * cells + 2 * (task % S::TASKS) + p.r;
+            if (Q == 3 && q == 2) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float ux, uz, uy, zero;
+                    px_unpack(re[j], ux, uz);
+                    px_unpack(im[j], uy, zero);
+                    __stcs(&a.velocity[base + static_cast<size_t>(Fft::index(j, p)) * N], make_float4(ux, uy, uz, 0.0f));
+                }
+            } else if (q == 0) {
+#pragma unroll
+                for (int j = 0; j < S::HELD; ++j) held[j * NT] = make_ulonglong2(re[j], im[j]);
+                last = make_ulonglong2(re[15], im[15]);
+            } else {
+                const OceanConsts cst = a.consts[ocean];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const ulonglong2 h = j < S::HELD ? held[j * NT] : last;
+                    float2 f0, f1, f2, f3;
+                    px_unpack(h.x, f0.x, f1.x);
+                    px_unpack(h.y, f0.y, f1.y);
+                    px_unpack(re[j], f2.x, f3.x);
+                    px_unpack(im[j], f2.y, f3.y);
+                    const CellOut c = finalize_cell(f0, f1, f2, f3, cst.lambda, cst.foam_threshold, cst.inv_threshold);
+                    const size_t idx = base + static_cast<size_t>(Fft::index(j, p)) * N;
+                    __stcs(&a.disp[idx], c.disp);
+                    __stcs(&a.normal[idx], c.normal);
+                }
+            }
         }
     }
 }
 
-template <int NF, bool FOAM>
-__global__ void __launch_bounds__(256) large_finalize_kernel(FrameArgs a, int log_n)
+template <typename Kernel>
+cudaError_t launch(Kernel k, int tasks, int threads, int ctas, size_t smem, const FrameArgs& a, cudaStream_t st)
 {
-    const int n = 1 << log_n;
-    const size_t cells = static_cast<size_t>(n) * n;
-    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= cells) return;
-    const int o = blockIdx.y;
-    const int ocean = a.ocean_base + o;
-    const OceanConsts cst = a.consts[ocean];
-    const float2* in = a.inter + static_cast<size_t>(o) * NF * cells + i;
-    float2 f[NF];
-#pragma unroll
-    for (int k = 0; k < NF; ++k) f[k] = __ldcs(in + k * cells);
-    const CellOut c = finalize_cell(f[0], f[1], f[2], f[3], cst.lambda, cst.foam_threshold, cst.inv_threshold);
-    const size_t idx = static_cast<size_t>(ocean) * cells + i;
-    __stcs(&a.disp[idx], c.disp);
-    __stcs(&a.normal[idx], c.normal);
-    if constexpr (NF == 6) {
-        __stcs(&a.velocity[idx], make_float4(f[4].x, f[4].y, f[5].x, 0.0f));
-        if constexpr (FOAM) {
-            const int x = static_cast<int>(i & (n - 1));
-            const int z = static_cast<int>(i >> log_n);
-            __stcs(&a.foam_next[idx],
-                   foam_cell(a.foam_cur + static_cast<size_t>(ocean) * cells, n, x, z, f[4].x, f[5].x, c.disp.w,
-                             a.foam_dt, a.foam_decay, a.foam_gain, a.foam_scale, a.foam_drift_x, a.foam_drift_z,
-                             a.foam_inv_cell));
-        }
-    }
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    int dev = 0, sms = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    // One wave of CTAs, each walking over tasks: a twiddle table load serves them all.
+    const int grid = tasks < sms * ctas ? tasks : sms * ctas;
+    k<<<grid, threads, smem, st>>>(a);
+    return cudaGetLastError();
 }
 
 template <int LOG_N, int NF, int AR>
 cudaError_t rows_launch(const FrameArgs& a, cudaStream_t st)
 {
     using S = Large<LOG_N>;
-    auto k = large_row_kernel<LOG_N, NF, AR>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(S::ROW_SMEM));
-    if (e != cudaSuccess) return e;
-    static_assert(S::N % S::ROW_TASKS == 0, "row tasks divide evenly among CTAs");
-    const dim3 grid(S::N / S::ROW_TASKS, a.chunk);
-    k<<<grid, S::ROW_T, S::ROW_SMEM, st>>>(a);
-    return cudaGetLastError();
+    return launch(large_row_kernel<LOG_N, NF, AR>, S::TASKS * a.chunk, S::THREADS, S::CTAS, S::ROW_SMEM, a, st);
 }
 
-template <int LOG_N, int AR>
-cudaError_t cols_launch(int nf, const FrameArgs& a, cudaStream_t st)
+template <int LOG_N, int NF, int AR>
+cudaError_t cols_launch(const FrameArgs& a, cudaStream_t st)
 {
     using S = Large<LOG_N>;
-    auto k = large_col_kernel<LOG_N, AR>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(S::COL_SMEM));
-    if (e != cudaSuccess) return e;
-    static_assert((S::N / S::W) % S::COL_TASKS == 0, "column tasks divide evenly among CTAs");
-    const dim3 grid((S::N / S::W) * nf / S::COL_TASKS, a.chunk);
-    k<<<grid, S::COL_T, S::COL_SMEM, st>>>(a, nf);
-    return cudaGetLastError();
+    return launch(large_col_kernel<LOG_N, NF, AR>, S::TASKS * a.chunk, S::THREADS, S::CTAS, S::COL_SMEM, a, st);
 }
 
 // The arithmetic `ar` (kArExact, kArFast, kArPrecise) as a compile-time
@@ -239,6 +446,15 @@ cudaError_t rows_n(int nf, int ar, const FrameArgs& a, cudaStream_t st)
     });
 }
 
+template <int LOG_N>
+cudaError_t cols_n(int nf, int ar, const FrameArgs& a, cudaStream_t st)
+{
+    return with_arith(ar, [&](auto A) {
+        constexpr int AR = decltype(A)::value;
+        return nf == 4 ? cols_launch<LOG_N, 4, AR>(a, st) : cols_launch<LOG_N, 6, AR>(a, st);
+    });
+}
+
 }  // namespace
 
 cudaError_t launch_large_rows(int log_n, int nf, int ar, const FrameArgs& a, cudaStream_t st)
@@ -254,34 +470,11 @@ cudaError_t launch_large_rows(int log_n, int nf, int ar, const FrameArgs& a, cud
 cudaError_t launch_large_cols(int log_n, int nf, int ar, const FrameArgs& a, cudaStream_t st)
 {
     if (nf != 4 && nf != 6) return cudaErrorInvalidValue;
-    return with_arith(ar, [&](auto A) {
-        constexpr int AR = decltype(A)::value;
-        switch (log_n) {
-            case 11: return cols_launch<11, AR>(nf, a, st);
-            case 12: return cols_launch<12, AR>(nf, a, st);
-            default: return cudaErrorInvalidValue;
-        }
-    });
-}
-
-cudaError_t launch_large_finalize(int log_n, int nf, bool fuse_foam, const FrameArgs& a, cudaStream_t st)
-{
-    if (log_n != 11 && log_n != 12) return cudaErrorInvalidValue;
-    if (fuse_foam && nf != 6) return cudaErrorInvalidValue;
-    const size_t cells = size_t(1) << (2 * log_n);
-    const dim3 grid(static_cast<unsigned>(cells / 256), a.chunk);
-    if (nf == 4) {
-        large_finalize_kernel<4, false><<<grid, 256, 0, st>>>(a, log_n);
-    } else if (nf == 6) {
-        if (fuse_foam) {
-            large_finalize_kernel<6, true><<<grid, 256, 0, st>>>(a, log_n);
-        } else {
-            large_finalize_kernel<6, false><<<grid, 256, 0, st>>>(a, log_n);
-        }
-    } else {
-        return cudaErrorInvalidValue;
+    switch (log_n) {
+        case 11: return cols_n<11>(nf, ar, a, st);
+        case 12: return cols_n<12>(nf, ar, a, st);
+        default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 }  // namespace ocean_b200

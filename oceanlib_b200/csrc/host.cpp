@@ -423,6 +423,7 @@ public:
             }
         }
         if (steps > 0) {
+            if (large()) foam_substep(st);
             foam_cur_ ^= 1;
             for (uint32_t s = 1; s < steps; ++s) {
                 foam_substep(st);
@@ -495,9 +496,9 @@ public:
         const uint32_t steps = foam_on_ ? foam_accumulate(foam_dt) : 0u;
         FrameArgs a = frame_args(dev);
         if (steps > 0) set_foam_args(a);
-        // Foam beyond the first substep needs every ocean's previous state,
-        // so copies start per chunk only when the frame has one substep.
-        const bool pipelined = steps <= 1;
+        // Foam beyond the fused substep (all of it above N = 1024) comes after
+        // every ocean's frame, so copies start per chunk only without it.
+        const bool pipelined = steps == 0 || (steps == 1 && !large());
         const size_t bytes4 = cells_ * sizeof(float4);
         uint32_t c = 0;
         for (uint32_t base = 0; base < count_; base += chunk_, ++c) {
@@ -517,6 +518,7 @@ public:
             }
         }
         if (steps > 0) {
+            if (large()) foam_substep(stream_);
             foam_cur_ ^= 1;
             for (uint32_t s = 1; s < steps; ++s) {
                 foam_substep(stream_);
@@ -709,7 +711,6 @@ private:
         const int ar = arith_of_form(form_);
         if (large()) {
             timed(1, st, [&] { check(launch_large_cols(log_n_, nf_, ar, a, st), "column pass"); });
-            timed(1, st, [&] { check(launch_large_finalize(log_n_, nf_, foam, a, st), "finalize"); });
             return;
         }
         timed(1, st, [&] { check(launch_col_pass(log_n_, nf_, ar, foam, a, st), "column pass"); });

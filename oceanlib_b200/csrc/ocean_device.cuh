@@ -346,20 +346,11 @@ struct PairBlock {
     static constexpr int C = (N >> r) / G2;
     static constexpr int w = LOG_N - r - L0;
 
-    __device__ __forceinline__ static void run(ulonglong2* seq, const float2* tw, int lane, int bar_id)
+    // The block's butterflies on values in registers: slot [k][t] holds the
+    // element T = t of combination c = lane + G2 k, and afterwards the one that
+    // belongs at index_after(k, slot, lane).
+    __device__ __forceinline__ static void compute(f32x2 (&re)[C][RR], f32x2 (&im)[C][RR], const float2* tw, int lane)
     {
-        f32x2 re[C][RR], im[C][RR];
-#pragma unroll
-        for (int k = 0; k < C; ++k) {
-            const int c = lane + G2 * k;
-#pragma unroll
-            for (int t = 0; t < RR; ++t) {
-                const ulonglong2 v = seq[pad4((t << (LOG_N - r)) | c)];
-                re[k][t] = v.x;
-                im[k][t] = v.y;
-            }
-        }
-        pair_sync<G2>(bar_id);
         if constexpr (AR == kArPrecise) {
             // The pair's two sequences one after the other, each as doubles
             // (8 complex values: 32 registers), rounded back into its half
@@ -402,38 +393,89 @@ struct PairBlock {
             }
         } else {
 #pragma unroll
-        for (int k = 0; k < C; ++k) {
-            const int c = lane + G2 * k;
-            const int P = c >> L0;
+            for (int k = 0; k < C; ++k) {
+                const int c = lane + G2 * k;
+                const int P = c >> L0;
 #pragma unroll
-            for (int s = 0; s < r; ++s) {
-                const int half = RR >> (s + 1);
-                const int l = L0 + s;
-                const float2* twl = tw + (N - (N >> l));
+                for (int s = 0; s < r; ++s) {
+                    const int half = RR >> (s + 1);
+                    const int l = L0 + s;
+                    const float2* twl = tw + (N - (N >> l));
 #pragma unroll
-                for (int S = 0; S < RR; ++S) {
-                    if (S & half) continue;
-                    const int Rk = S & (half - 1);
-                    // One 8-byte load, duplicated into both lanes of each
-                    // f32x2 in registers (a 16-byte (wx, wx, wy, wy) table
-                    // entry costs twice the shared-memory wavefronts).
-                    const float2 wv = twl[(Rk << w) | P];
-                    butterfly_pair<AR>(re[k][S], im[k][S], re[k][S + half], im[k][S + half], px_pack(wv.x, wv.x),
-                                       px_pack(wv.y, wv.y));
+                    for (int S = 0; S < RR; ++S) {
+                        if (S & half) continue;
+                        const int Rk = S & (half - 1);
+                        // One 8-byte load, duplicated into both lanes of each
+                        // f32x2 in registers (a 16-byte (wx, wx, wy, wy) table
+                        // entry costs twice the shared-memory wavefronts).
+                        const float2 wv = twl[(Rk << w) | P];
+                        butterfly_pair<AR>(re[k][S], im[k][S], re[k][S + half], im[k][S + half], px_pack(wv.x, wv.x),
+                                           px_pack(wv.y, wv.y));
+                    }
                 }
             }
         }
-        }
+    }
+
+    // The same on one sequence of the pair, in FP64, rounded to FP32 once.
+    __device__ __forceinline__ static void compute_f64(float (&x)[C][RR], float (&y)[C][RR], const float2* tw, int lane)
+    {
 #pragma unroll
         for (int k = 0; k < C; ++k) {
-            const int c = lane + G2 * k;
-            const int P = c >> L0;
-            const int q = c & ((1 << L0) - 1);
+            const int P = (lane + G2 * k) >> L0;
+            double xr[RR], xi[RR];
 #pragma unroll
-            for (int S = 0; S < RR; ++S) {
-                const int out = (P << (L0 + r)) | (bitrev<r>(S) << L0) | q;
-                seq[pad4(out)] = make_ulonglong2(re[k][S], im[k][S]);
+            for (int t = 0; t < RR; ++t) {
+                xr[t] = x[k][t];
+                xi[t] = y[k][t];
             }
+#pragma unroll
+            for (int s = 0; s < r; ++s) {
+                const int half = RR >> (s + 1);
+                const float2* twl = tw + (N - (N >> (L0 + s)));
+#pragma unroll
+                for (int S = 0; S < RR; ++S) {
+                    if (S & half) continue;
+                    butterfly_f64(xr[S], xi[S], xr[S + half], xi[S + half], twl[((S & (half - 1)) << w) | P]);
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < RR; ++t) {
+                x[k][t] = __double2float_rn(xr[t]);
+                y[k][t] = __double2float_rn(xi[t]);
+            }
+        }
+    }
+
+    // Where slot [k][t] comes from before the block, and goes after it.
+    __device__ __forceinline__ static int index_before(int k, int t, int lane)
+    {
+        return (t << (LOG_N - r)) | (lane + G2 * k);
+    }
+    __device__ __forceinline__ static int index_after(int k, int S, int lane)
+    {
+        const int c = lane + G2 * k;
+        return ((c >> L0) << (L0 + r)) | (bitrev<r>(S) << L0) | (c & ((1 << L0) - 1));
+    }
+
+    __device__ __forceinline__ static void run(ulonglong2* seq, const float2* tw, int lane, int bar_id)
+    {
+        f32x2 re[C][RR], im[C][RR];
+#pragma unroll
+        for (int k = 0; k < C; ++k) {
+#pragma unroll
+            for (int t = 0; t < RR; ++t) {
+                const ulonglong2 v = seq[pad4(index_before(k, t, lane))];
+                re[k][t] = v.x;
+                im[k][t] = v.y;
+            }
+        }
+        pair_sync<G2>(bar_id);
+        compute(re, im, tw, lane);
+#pragma unroll
+        for (int k = 0; k < C; ++k) {
+#pragma unroll
+            for (int S = 0; S < RR; ++S) seq[pad4(index_after(k, S, lane))] = make_ulonglong2(re[k][S], im[k][S]);
         }
         pair_sync<G2>(bar_id);
         if constexpr (L0 + r < LOG_N) PairBlock<LOG_N, G2, L0 + r, AR>::run(seq, tw, lane, bar_id);

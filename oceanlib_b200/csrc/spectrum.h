@@ -149,17 +149,14 @@ cudaError_t launch_col_pass(int log_n, int nf, int ar, bool fuse_foam,
                             const FrameArgs& args, cudaStream_t stream);
 
 // The frame at N = 2048 and 4096 (log_n 11, 12; frame_large.cu), for
-// `args.chunk` oceans from args.ocean_base, in three launches: rows (evolve +
-// row FFTs), column FFTs in place, finalize (+ the first foam substep when
-// fuse_foam; nf = 6). The intermediate is field-major: field f of chunk ocean
-// o at args.inter + (o * nf + f) * N * N. args.table must be null.
+// `args.chunk` oceans from args.ocean_base, in two launches: rows (evolve +
+// row FFTs) and columns (column FFTs + finalize), through nf * N * N float2 of
+// args.inter an ocean of the chunk. args.table must be null.
 cudaError_t launch_large_rows(int log_n, int nf, int ar, const FrameArgs& args, cudaStream_t stream);
 cudaError_t launch_large_cols(int log_n, int nf, int ar, const FrameArgs& args, cudaStream_t stream);
-cudaError_t launch_large_finalize(int log_n, int nf, bool fuse_foam, const FrameArgs& args,
-                                  cudaStream_t stream);
 
 // Stand-alone foam substep for oceans [0, count) (used for substeps after the
-// first in one update).
+// first in one update, and above N = 1024 for the first too).
 cudaError_t launch_foam_step(int n, int count, const float4* disp, const float4* velocity,
                              const float* cur, float* next, float dt, float decay, float gain,
                              float scale, float drift_x, float drift_z, float inv_cell,
