@@ -364,7 +364,7 @@ __device__ __forceinline__ void row_task(const FrameArgs& a, int ocean, int grou
         kvec = a.kvec + static_cast<size_t>(cst.geom) * N;
         h0 = a.h0 + static_cast<size_t>(ocean) * N * N;
     }
-    const double top = a.t_over_2pi[ocean];
+    const double top = frame_time(a, ocean);
 
     // Row of slot jr: pair p = (jr's pair index) covers (p, N-p), or (0, N/2)
     // for p = 0. Paired tasks hold whole pairs (slot jr = 2 j + r); single-row
@@ -758,6 +758,12 @@ __host__ __device__ constexpr size_t frame_engine_offset()
            128 * 128;
 }
 
+// Zeroes the next launch's queue words, each CTA its share (QueueArgs).
+__device__ __forceinline__ void clear_words(unsigned* words, uint32_t count, int tid, int nt)
+{
+    for (uint32_t i = blockIdx.x * nt + tid; i < count; i += gridDim.x * nt) words[i] = 0u;
+}
+
 template <class P, int NF, int AR, bool FOAM>
 __global__ void __launch_bounds__(P::template threads<NF>(), frame_min_blocks<P, NF>())
 frame_kernel(FrameArgs a, QueueArgs q)
@@ -792,6 +798,7 @@ frame_kernel(FrameArgs a, QueueArgs q)
     uint32_t h0_parity = 0;
 
     const int tid = threadIdx.x;
+    clear_words(q.clear, q.clear_words, tid, NT);
     if constexpr (!TC) load_twiddles<P>(tws, a.twiddles, tid, NT);
     TcEngineOf<LOG_N, NF> eng{reinterpret_cast<unsigned char*>(smem4) + frame_engine_offset<LOG_N, NF>(), 0};
     if constexpr (TC) {
@@ -1032,7 +1039,9 @@ __global__ void __launch_bounds__(64 * NF, 768 / (64 * NF)) mixed_frame_kernel(M
     }
     static_assert(sizeof(MixedGroup) % sizeof(unsigned) == 0, "the group table copies as words");
 
+    if (blockIdx.x == 0 && tid == 0 && m.clear_ticket != nullptr) *m.clear_ticket = 0u;
     for (int gi = 0; gi < m.groups; ++gi) {
+        clear_words(m.g[gi].clear, m.g[gi].clear_words, tid, NT);
         const float2* src = m.g[gi].a.twiddles;
         switch (m.g[gi].log_n) {
             case 5: mix_load_twiddles<5, NF>(tw_area, src, tid, NT); break;

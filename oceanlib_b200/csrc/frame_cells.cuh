@@ -5,8 +5,15 @@
 #pragma once
 
 #include "ocean_device.cuh"
+#include "spectrum.h"
 
 namespace ocean_b200 {
+
+// t / 2 pi of an ocean of the frame.
+__device__ __forceinline__ double frame_time(const FrameArgs& a, int ocean)
+{
+    return a.t_over_2pi != nullptr ? a.t_over_2pi[ocean] : a.t_uniform;
+}
 
 // The evolved amplitude of one cell (src/core/evolve.cpp:28-121, and :123-184
 // for the velocity fields): h0(k) = av, h0(-k) = bm (conjugated here), the

@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) lar
             kv_of = geom_of;
         }
         const float kz = kv[y];
-        const double top = a.t_over_2pi[ocean];
+        const double top = frame_time(a, ocean);
         ulonglong2* out = reinterpret_cast<ulonglong2*>(a.inter + static_cast<size_t>(o) * NF * cells) + 2 * y;
 #pragma unroll 1
         for (int k = 0; k < Q; ++k) {

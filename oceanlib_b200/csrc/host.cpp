@@ -255,12 +255,14 @@ public:
         const uint32_t inter_oceans =
             large() ? chunk_ : std::max<uint32_t>(chunk_, static_cast<uint32_t>(slots_));
         inter_ = DevBuf<float2>(cells_ * nf_ * inter_oceans);
-        queue_ = DevBuf<unsigned>(1 + 2 * size_t(count_));
+        queue_ = FrameQueue(count_, stream_);
         error_ = DevBuf<unsigned>(1);
         check(cudaMemsetAsync(error_.p, 0, sizeof(unsigned), stream_), "memset");
-        disp_ = DevBuf<float4>(cells_ * count_);
-        normal_ = DevBuf<float4>(cells_ * count_);
-        if (velocity_) velocity_buf_ = DevBuf<float4>(cells_ * count_);
+        // One block, so that a single ocean's outputs are one copy to the host.
+        out_ = DevBuf<float4>(cells_ * count_ * (velocity_ ? 3 : 2));
+        disp_ = out_.p;
+        normal_ = disp_ + cells_ * count_;
+        if (velocity_) velocity_buf_ = normal_ + cells_ * count_;
         if (foam_on_) {
             foam_a_ = DevBuf<float>(cells_ * count_);
             foam_b_ = DevBuf<float>(cells_ * count_);
@@ -381,9 +383,9 @@ public:
     }
     size_t cells() const { return cells_; }
 
-    float4* disp(uint32_t i) const { return disp_.p + i * cells_; }
-    float4* normal(uint32_t i) const { return normal_.p + i * cells_; }
-    float4* velocity_ptr(uint32_t i) const { return velocity_ ? velocity_buf_.p + i * cells_ : nullptr; }
+    float4* disp(uint32_t i) const { return disp_ + i * cells_; }
+    float4* normal(uint32_t i) const { return normal_ + i * cells_; }
+    float4* velocity_ptr(uint32_t i) const { return velocity_ ? velocity_buf_ + i * cells_ : nullptr; }
     float* foam_ptr(uint32_t i) const
     {
         if (!foam_on_) return nullptr;
@@ -395,22 +397,8 @@ public:
     void update(const double* times, bool per_ocean, float foam_dt, cudaStream_t st)
     {
         if (st == nullptr) st = stream_;
-        // Per-ocean t/(2pi), hoisted exactly as src/core/evolve.cpp:33 does.
-        const int slot = slot_next_;
-        slot_next_ = (slot_next_ + 1) % kTimeSlots;
-        check(cudaEventSynchronize(slot_done_[slot]), "time slot");
-        double* host = top_host_.p + static_cast<size_t>(slot) * count_;
-        for (uint32_t i = 0; i < count_; ++i) {
-            const double t = per_ocean ? times[i] : times[0];
-            host[i] = t * kInvTwoPi;
-        }
-        double* dev = top_.p + static_cast<size_t>(slot) * count_;
-        check(cudaMemcpyAsync(dev, host, count_ * sizeof(double), cudaMemcpyHostToDevice, st),
-              "upload times");
-        check(cudaEventRecord(slot_done_[slot], st), "event");
-
+        FrameArgs a = frame_args_at(times, per_ocean, st);
         const uint32_t steps = foam_on_ ? foam_accumulate(foam_dt) : 0u;
-        FrameArgs a = frame_args(dev);
         if (steps > 0) set_foam_args(a);
         if (persistent_) {
             run_frame(a, 0, count_, steps > 0, st);
@@ -456,25 +444,12 @@ public:
     // the row pass of every chunk, stage 1 the column pass (plus foam).
     void update_stage(int stage, const double* times, cudaStream_t st)
     {
+        FrameArgs a = frame_args_at(times, false, st);
+        a.ocean_base = 0;
+        a.chunk = static_cast<int32_t>(count_);
         if (stage == 0) {
-            const int slot = slot_next_;
-            slot_next_ = (slot_next_ + 1) % kTimeSlots;
-            check(cudaEventSynchronize(slot_done_[slot]), "time slot");
-            double* host = top_host_.p + static_cast<size_t>(slot) * count_;
-            for (uint32_t i = 0; i < count_; ++i) host[i] = times[0] * kInvTwoPi;
-            staged_top_ = top_.p + static_cast<size_t>(slot) * count_;
-            check(cudaMemcpyAsync(staged_top_, host, count_ * sizeof(double),
-                                  cudaMemcpyHostToDevice, st), "upload times");
-            check(cudaEventRecord(slot_done_[slot], st), "event");
-            // One chunk only on this path (a single ocean).
-            FrameArgs a = frame_args(staged_top_);
-            a.ocean_base = 0;
-            a.chunk = static_cast<int32_t>(count_);
-            run_row(a, st);
+            run_row(a, st);  // one chunk only on this path (a single ocean)
         } else {
-            FrameArgs a = frame_args(staged_top_);
-            a.ocean_base = 0;
-            a.chunk = static_cast<int32_t>(count_);
             run_col(a, st, false);
         }
     }
@@ -484,17 +459,8 @@ public:
     void update_host(const double* times, bool per_ocean, float foam_dt, float* h_disp,
                      float* h_normal, float* h_vel, float* h_foam)
     {
-        const int slot = slot_next_;
-        slot_next_ = (slot_next_ + 1) % kTimeSlots;
-        check(cudaEventSynchronize(slot_done_[slot]), "time slot");
-        double* host = top_host_.p + static_cast<size_t>(slot) * count_;
-        for (uint32_t i = 0; i < count_; ++i) host[i] = (per_ocean ? times[i] : times[0]) * kInvTwoPi;
-        double* dev = top_.p + static_cast<size_t>(slot) * count_;
-        check(cudaMemcpyAsync(dev, host, count_ * sizeof(double), cudaMemcpyHostToDevice, stream_),
-              "upload times");
-        check(cudaEventRecord(slot_done_[slot], stream_), "event");
+        FrameArgs a = frame_args_at(times, per_ocean, stream_);
         const uint32_t steps = foam_on_ ? foam_accumulate(foam_dt) : 0u;
-        FrameArgs a = frame_args(dev);
         if (steps > 0) set_foam_args(a);
         // Foam beyond the fused substep (all of it above N = 1024) comes after
         // every ocean's frame, so copies start per chunk only without it.
@@ -555,15 +521,15 @@ public:
         ushort4* hv = hn + texels;
         const size_t bytes = texels * sizeof(ushort4);
         if (h_disp) {
-            check(launch_pack_rgba16(disp_.p, foam_on_ ? foam_ptr(0) : nullptr, texels, hd, stream_), "pack");
+            check(launch_pack_rgba16(disp_, foam_on_ ? foam_ptr(0) : nullptr, texels, hd, stream_), "pack");
             check(cudaMemcpyAsync(h_disp, hd, bytes, cudaMemcpyDeviceToHost, stream_), "copy displacement");
         }
         if (h_normal) {
-            check(launch_pack_rgba16(normal_.p, nullptr, texels, hn, stream_), "pack");
+            check(launch_pack_rgba16(normal_, nullptr, texels, hn, stream_), "pack");
             check(cudaMemcpyAsync(h_normal, hn, bytes, cudaMemcpyDeviceToHost, stream_), "copy normal");
         }
         if (h_vel && velocity_) {
-            check(launch_pack_rgba16(velocity_buf_.p, nullptr, texels, hv, stream_), "pack");
+            check(launch_pack_rgba16(velocity_buf_, nullptr, texels, hv, stream_), "pack");
             check(cudaMemcpyAsync(h_vel, hv, bytes, cudaMemcpyDeviceToHost, stream_), "copy velocity");
         }
         check(cudaStreamSynchronize(stream_), "frame");
@@ -680,16 +646,18 @@ private:
     }
 
     // One persistent launch for oceans [base, base + k) (csrc/frame.cu
-    // frame_kernel): reset its work queue, then launch one wave of resident CTAs.
+    // frame_kernel): one wave of resident CTAs.
     void run_frame(FrameArgs a, uint32_t base, uint32_t k, bool foam, cudaStream_t st)
     {
         a.ocean_base = static_cast<int32_t>(base);
         a.chunk = static_cast<int32_t>(k);
-        check(cudaMemsetAsync(queue_.p, 0, (1 + 2 * size_t(k)) * sizeof(unsigned), st), "queue reset");
         QueueArgs q;
-        q.ticket = queue_.p;
-        q.rows_done = queue_.p + 1;
-        q.cols_done = queue_.p + 1 + k;
+        const FrameQueue::Set set = queue_.take(st);
+        q.ticket = set.ticket;
+        q.rows_done = set.counters;
+        q.cols_done = set.counters + k;
+        q.clear = set.clear;
+        q.clear_words = set.words;
         q.error = error_.p;
         q.count = static_cast<int32_t>(k);
         q.slots = slots_;
@@ -704,6 +672,7 @@ private:
             check(launch_frame(log_n_, nf_, form_, foam, a, q, launch_grid, st, plan_),
                   "frame kernel");
         });
+        queue_.launched(set);
     }
 
     void run_col(const FrameArgs& a, cudaStream_t st, bool foam)
@@ -848,22 +817,27 @@ public:
     int nf() const { return nf_; }
     int form() const { return form_; }
 
-    // The batch as one group of a mixed-size launch, with the per-ocean
-    // t / 2 pi at `top` on the device; its queue counters are zeroed on `st`.
-    MixedGroup mixed_group(const double* top, cudaStream_t st)
+    // The batch as one group of a mixed-size launch on `st`, every ocean at
+    // t / 2 pi; mixed_launched() once that is queued.
+    MixedGroup mixed_group(double t_over_2pi, cudaStream_t st)
     {
         MixedGroup g{};
-        g.a = frame_args(top);
+        g.a = frame_args(nullptr);
+        g.a.t_uniform = t_over_2pi;
         g.a.ocean_base = 0;
         g.a.chunk = static_cast<int32_t>(count_);
-        check(cudaMemsetAsync(queue_.p, 0, (1 + 2 * size_t(count_)) * sizeof(unsigned), st), "queue reset");
-        g.rows_done = queue_.p + 1;
-        g.cols_done = queue_.p + 1 + count_;
+        mixed_set_ = queue_.take(st);
+        g.rows_done = mixed_set_.counters;
+        g.cols_done = mixed_set_.counters + count_;
+        g.clear = mixed_set_.clear;
+        g.clear_words = mixed_set_.words;
         g.count = static_cast<int32_t>(count_);
         g.slots = slots_;
         g.log_n = log_n_;
         return g;
     }
+
+    void mixed_launched() { queue_.launched(mixed_set_); }
 
     // Settles the launch shapes, so a capture issues launches only.
     void prime_shapes()
@@ -872,6 +846,27 @@ public:
     }
 
 private:
+
+    // The frame's arguments with t / 2 pi hoisted exactly as
+    // src/core/evolve.cpp:33 does: one time for every ocean travels with the
+    // launch, a time per ocean through a pinned slot, copied on `st`.
+    FrameArgs frame_args_at(const double* times, bool per_ocean, cudaStream_t st)
+    {
+        if (!per_ocean) {
+            FrameArgs a = frame_args(nullptr);
+            a.t_uniform = times[0] * kInvTwoPi;
+            return a;
+        }
+        const int slot = slot_next_;
+        slot_next_ = (slot_next_ + 1) % kTimeSlots;
+        check(cudaEventSynchronize(slot_done_[slot]), "time slot");
+        double* host = top_host_.p + static_cast<size_t>(slot) * count_;
+        for (uint32_t i = 0; i < count_; ++i) host[i] = times[i] * kInvTwoPi;
+        double* dev = top_.p + static_cast<size_t>(slot) * count_;
+        check(cudaMemcpyAsync(dev, host, count_ * sizeof(double), cudaMemcpyHostToDevice, st), "upload times");
+        check(cudaEventRecord(slot_done_[slot], st), "event");
+        return frame_args(dev);
+    }
 
     FrameArgs frame_args(const double* top) const
     {
@@ -883,9 +878,9 @@ private:
         a.consts = consts_.p;
         a.t_over_2pi = top;
         a.inter = inter_.p;
-        a.disp = disp_.p;
-        a.normal = normal_.p;
-        a.velocity = velocity_buf_.p;
+        a.disp = disp_;
+        a.normal = normal_;
+        a.velocity = velocity_buf_;
         a.error = error_.p;
         return a;
     }
@@ -910,8 +905,8 @@ private:
         FrameArgs a = frame_args(nullptr);
         set_foam_args(a);
         timed(2, st, [&] {
-            check(launch_foam_step(static_cast<int>(n_), static_cast<int>(count_), disp_.p,
-                                   velocity_buf_.p, a.foam_cur, a.foam_next, a.foam_dt,
+            check(launch_foam_step(static_cast<int>(n_), static_cast<int>(count_), disp_,
+                                   velocity_buf_, a.foam_cur, a.foam_next, a.foam_dt,
                                    a.foam_decay, a.foam_gain, a.foam_scale, a.foam_drift_x,
                                    a.foam_drift_z, a.foam_inv_cell, st), "foam step");
         });
@@ -982,17 +977,19 @@ private:
     int frame_grid_[kMaxFramePlans][2] = {};  // [plan][foam]: CTAs of one wave
     int plan_ = 0;  // the persistent kernel's task plan (frame_plan_count)
     double grid_share_ = 1.0;
-    DevBuf<unsigned> queue_, error_;
+    FrameQueue queue_;
+    FrameQueue::Set mixed_set_{};
+    DevBuf<unsigned> error_;
     uint64_t launches_ = 0;
     int slot_next_ = 0;
-    double* staged_top_ = nullptr;
 
     DevBuf<float2> h0_, geom_, tw_, inter_;
     DevBuf<float> kvec_;
     DevBuf<OceanConsts> consts_;
     DevBuf<double> top_;
     HostBuf<double> top_host_;
-    DevBuf<float4> disp_, normal_, velocity_buf_;
+    DevBuf<float4> out_;  // displacement, normal and velocity of every ocean
+    float4 *disp_ = nullptr, *normal_ = nullptr, *velocity_buf_ = nullptr;
     DevBuf<ushort4> half_;  // RGBA16F staging of update_host_rgba16 (allocated on first use)
     DevBuf<float> foam_a_, foam_b_;
     int foam_cur_ = 0;
@@ -1015,9 +1012,9 @@ public:
         : desc_(d), batch_(&desc_, 1, g_form.load(), false, foam_defaults(), 1)
     {
         const size_t cells = batch_.cells();
-        disp_ = HostBuf<float>(cells * 4);
-        normal_ = HostBuf<float>(cells * 4);
-        if (batch_.velocity()) vel_ = HostBuf<float>(cells * 4);
+        // Displacement, normal and velocity one after the other, as the batch
+        // holds them: the mirror is one copy.
+        mirror_ = HostBuf<float>(cells * 4 * (batch_.velocity() ? 3 : 2));
         q_in_ = DevBuf<float2>(1);
         q_out_ = DevBuf<SurfaceEx>(1);
         q_host_in_ = HostBuf<float2>(1);
@@ -1053,13 +1050,8 @@ public:
 
     void refresh()
     {
-        const size_t bytes = batch_.cells() * sizeof(float4);
         cudaStream_t st = batch_.stream();
-        check(cudaMemcpyAsync(disp_.p, batch_.disp(0), bytes, cudaMemcpyDeviceToHost, st), "copy");
-        check(cudaMemcpyAsync(normal_.p, batch_.normal(0), bytes, cudaMemcpyDeviceToHost, st), "copy");
-        if (vel_.p)
-            check(cudaMemcpyAsync(vel_.p, batch_.velocity_ptr(0), bytes, cudaMemcpyDeviceToHost, st),
-                  "copy");
+        check(cudaMemcpyAsync(mirror_.p, batch_.disp(0), mirror_.n * sizeof(float), cudaMemcpyDeviceToHost, st), "copy");
         check(cudaStreamSynchronize(st), "refresh");
     }
 
@@ -1096,9 +1088,9 @@ public:
 
     const ocean_desc& desc() const { return desc_; }
     double time() const { return time_; }
-    const float* host_disp() const { return disp_.p; }
-    const float* host_normal() const { return normal_.p; }
-    const float* host_velocity() const { return vel_.p; }
+    float* host_disp() const { return mirror_.p; }
+    float* host_normal() const { return mirror_.p + 4 * batch_.cells(); }
+    float* host_velocity() const { return batch_.velocity() ? mirror_.p + 8 * batch_.cells() : nullptr; }
     Batch& batch() { return batch_; }
     const Batch& batch() const { return batch_; }
 
@@ -1128,14 +1120,14 @@ private:
                 case 0: m.batch_.update_stage(0, &c->t, st); break;
                 case 1: m.batch_.update_stage(1, &c->t, st); break;
                 case 2:
-                    check(cudaMemcpyAsync(m.disp_.p, m.batch_.disp(0), bytes, cudaMemcpyDeviceToHost, st),
+                    check(cudaMemcpyAsync(m.host_disp(), m.batch_.disp(0), bytes, cudaMemcpyDeviceToHost, st),
                           "copy");
                     break;
                 default:
-                    check(cudaMemcpyAsync(m.normal_.p, m.batch_.normal(0), bytes,
+                    check(cudaMemcpyAsync(m.host_normal(), m.batch_.normal(0), bytes,
                                           cudaMemcpyDeviceToHost, st), "copy");
-                    if (m.vel_.p)
-                        check(cudaMemcpyAsync(m.vel_.p, m.batch_.velocity_ptr(0), bytes,
+                    if (m.batch_.velocity())
+                        check(cudaMemcpyAsync(m.host_velocity(), m.batch_.velocity_ptr(0), bytes,
                                               cudaMemcpyDeviceToHost, st), "copy");
                     break;
             }
@@ -1150,7 +1142,7 @@ private:
     ocean_desc desc_;
     Batch batch_;
     double time_ = 0.0;
-    HostBuf<float> disp_, normal_, vel_;
+    HostBuf<float> mirror_;
     mutable std::mutex query_mutex_;
     mutable DevBuf<float2> q_in_, many_in_;
     mutable DevBuf<SurfaceEx> q_out_, many_out_;
@@ -1379,8 +1371,10 @@ public:
             mixed_ok_ = mixed_ok_ && b->mixable() && b->nf() == batches_[0]->nf() && b->form() == batches_[0]->form();
         if (mixed_ok_) {
             mix_defer_ = batches_[0]->nf() == 6;
-            mix_words_ = DevBuf<unsigned>(2);  // ticket, error word
-            check(cudaMemsetAsync(mix_words_.p, 0, 2 * sizeof(unsigned), stream_), "memset");
+            mix_ticket_ = FrameQueue(0, stream_);
+            mix_error_ = DevBuf<unsigned>(1);
+            check(cudaMemsetAsync(mix_error_.p, 0, sizeof(unsigned), stream_), "memset");
+            check(cudaStreamSynchronize(stream_), "memset");  // updates may come on any stream
             for (size_t g = 0; g < batches_.size(); ++g) mix_order_.push_back(g);
             // Largest tasks first, so the short ones fill the wave's tail.
             std::stable_sort(mix_order_.begin(), mix_order_.end(),
@@ -1419,6 +1413,10 @@ public:
     void update(double t, cudaStream_t st)
     {
         if (st == nullptr) st = stream_;
+        if (mixed_) {
+            enqueue_mixed(Batch::time_over_2pi(t), st);  // one launch, the time among its arguments
+            return;
+        }
         if (use_graph_) {
             // The whole frame - time upload, fork, every size's persistent
             // launch, join - is one CUDA graph, captured once and replayed.
@@ -1427,11 +1425,6 @@ public:
             const double top = Batch::time_over_2pi(t);
             for (size_t i = 0; i < gtimes_.n; ++i) gtimes_.p[i] = top;
             check(cudaGraphLaunch(exec_, st), "graph launch");
-            return;
-        }
-        if (mixed_) {
-            stage_times(t, st);
-            enqueue_mixed(dtimes_.p, st);
             return;
         }
         if (!concurrent_) {
@@ -1481,10 +1474,10 @@ public:
     {
         if (!mixed_ok_) return;
         unsigned w = 0;
-        check(cudaMemcpyAsync(&w, mix_words_.p + 1, sizeof(w), cudaMemcpyDeviceToHost, stream_), "error word");
+        check(cudaMemcpyAsync(&w, mix_error_.p, sizeof(w), cudaMemcpyDeviceToHost, stream_), "error word");
         check(cudaStreamSynchronize(stream_), "error word");
         if (w != 0) {
-            check(cudaMemsetAsync(mix_words_.p + 1, 0, sizeof(unsigned), stream_), "memset");
+            check(cudaMemsetAsync(mix_error_.p, 0, sizeof(unsigned), stream_), "memset");
             check(cudaStreamSynchronize(stream_), "error word");
             throw TimeoutError();
         }
@@ -1501,8 +1494,8 @@ public:
     const std::string& form_note() const { return form_note_; }
 
 private:
-    // Captures one frame under the chosen schedule: the upload of the pinned
-    // times, an event marking them read, then (concurrent) a fork onto one
+    // Captures one frame under the chosen schedule (the one launch needs no
+    // graph): the upload of the pinned times, an event marking them read, then (concurrent) a fork onto one
     // stream per size, each size's frame, and the join.
     void build_graph()
     {
@@ -1516,9 +1509,7 @@ private:
             // between replays; a plain record inside a capture only orders
             // the capture's own streams.
             check(cudaEventRecordWithFlags(copied_, stream_, cudaEventRecordExternal), "event");
-            if (mixed_) {
-                enqueue_mixed(dtimes_.p, stream_);
-            } else if (concurrent_) {
+            if (concurrent_) {
                 check(cudaEventRecord(fork_, stream_), "event");
                 for (size_t g = 0; g < batches_.size(); ++g) {
                     check(cudaStreamWaitEvent(streams_[g], fork_, 0), "wait");
@@ -1539,41 +1530,30 @@ private:
         check(cudaGraphInstantiate(&exec_, graph_, 0), "graph instantiate");
     }
 
-    // The host's t / 2 pi for every ocean into the pinned block (once the
-    // previous upload has read it), then uploaded on `st`.
-    void stage_times(double t, cudaStream_t st)
-    {
-        check(cudaEventSynchronize(copied_), "time staging");
-        const double top = Batch::time_over_2pi(t);
-        for (size_t i = 0; i < gtimes_.n; ++i) gtimes_.p[i] = top;
-        check(cudaMemcpyAsync(dtimes_.p, gtimes_.p, gtimes_.n * sizeof(double), cudaMemcpyHostToDevice, st),
-              "times");
-        check(cudaEventRecord(copied_, st), "event");
-    }
-
-    // Every size's frame as one mixed_frame_kernel launch on `st`: the groups'
-    // counters and the ticket reset, then the launch (device work only, so a
-    // capture can hold it).
-    void enqueue_mixed(const double* dtimes, cudaStream_t st)
+    // Every size's frame as one mixed_frame_kernel launch on `st`.
+    void enqueue_mixed(double t_over_2pi, cudaStream_t st)
     {
         MixedArgs m{};
         m.groups = static_cast<int32_t>(mix_order_.size());
         uint32_t first = 0;
         for (size_t k = 0; k < mix_order_.size(); ++k) {
             const size_t g = mix_order_[k];
-            m.g[k] = batches_[g]->mixed_group(dtimes + toff_[g], st);
+            m.g[k] = batches_[g]->mixed_group(t_over_2pi, st);
             m.g[k].first = first;
             first += mixed_tasks(m.g[k].log_n, m.g[k].count);
         }
         m.total = first;
-        m.ticket = mix_words_.p;
-        m.error = mix_words_.p + 1;
+        const FrameQueue::Set ticket = mix_ticket_.take(st);
+        m.ticket = ticket.ticket;
+        m.clear_ticket = ticket.clear;
+        m.error = mix_error_.p;
         m.wait_ns = 1000000000ull;
         m.defer = mix_defer_ ? 1 : 0;
-        check(cudaMemsetAsync(mix_words_.p, 0, sizeof(unsigned), st), "ticket reset");
         const int grid = static_cast<int>(std::min<uint64_t>(static_cast<uint64_t>(mix_grid_), first));
         check(launch_mixed_frame(batches_[0]->nf(), arith_of_form(batches_[0]->form()), m, grid, st),
               "mixed frame kernel");
+        mix_ticket_.launched(ticket);
+        for (size_t g : mix_order_) batches_[g]->mixed_launched();
     }
 
     void drop_graph()
@@ -1744,7 +1724,8 @@ private:
     bool mix_defer_ = false;      // MixedArgs::defer (default: with velocity)
     int mix_grid_ = 0;
     std::vector<size_t> mix_order_;
-    DevBuf<unsigned> mix_words_;
+    FrameQueue mix_ticket_;
+    DevBuf<unsigned> mix_error_;
     std::string describe_;
     int form_ = OCEAN_FFT_EXACT;
     std::string form_note_;

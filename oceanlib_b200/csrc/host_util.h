@@ -102,4 +102,52 @@ struct HostBuf {
     ~HostBuf() { if (p) cudaFreeHost(p); }
 };
 
+// The queue words (a ticket, then rows_done[count] and cols_done[count]) of a
+// batch's persistent launches. Two sets take turns: a launch works on one and
+// zeroes the other for the launch after it, so that no memset stands in front
+// of a frame. It would pay to clear a launch's own words at its end, but its
+// last CTA must then know that all others are done, a fence and an atomic
+// round trip in each (3 x 256^2 cascade levels: 0.7 us a frame). While a
+// stream is captured the launch gets a third set, zeroed by a memset in the
+// same graph: a graph may be launched any number of times in a row, so its
+// launches cannot take turns.
+class FrameQueue {
+public:
+    struct Set {
+        unsigned* ticket;
+        unsigned* counters;  // rows_done, then cols_done
+        unsigned* clear;     // the next launch's words, or null
+        uint32_t words;      // of the next launch
+        bool turn;           // call launched() once the launch is queued
+    };
+
+    FrameQueue() = default;
+    // Zeroed on `st`: later launches come after that.
+    FrameQueue(size_t count, cudaStream_t st) : words_(1 + 2 * count), w_(3 * words_)
+    {
+        check(cudaMemsetAsync(w_.p, 0, w_.n * sizeof(unsigned), st), "queue");
+    }
+    Set take(cudaStream_t st) const
+    {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        check(cudaStreamIsCapturing(st, &cap), "capture status");
+        if (cap != cudaStreamCaptureStatusNone) {
+            unsigned* own = w_.p + 2 * words_;
+            check(cudaMemsetAsync(own, 0, words_ * sizeof(unsigned), st), "queue reset");
+            return {own, own + 1, nullptr, 0u, false};
+        }
+        unsigned* own = w_.p + turn_ * words_;
+        return {own, own + 1, w_.p + (turn_ ^ 1) * words_, static_cast<uint32_t>(words_), true};
+    }
+    void launched(const Set& s)
+    {
+        if (s.turn) turn_ ^= 1;
+    }
+
+private:
+    size_t words_ = 0;
+    DevBuf<unsigned> w_;
+    int turn_ = 0;
+};
+
 }  // namespace ocean_b200

@@ -156,7 +156,7 @@ struct OceanKind {
     int log_n = 0, nf = 4;
     int grid = 0;
     DevBuf<float2> tw, inter;
-    unsigned* queue = nullptr;  // pool allocation, 1 + 2 * queue_cap
+    FrameQueue queue;
     size_t queue_cap = 0;
     size_t bytes = 0;
 };
@@ -250,7 +250,7 @@ public:
         uint64_t keep = UINT64_MAX;  // keep freed memory cached in the pool
         check(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep), "pool attribute");
         error_ = DevBuf<unsigned>(1);
-        mix_ticket_ = DevBuf<unsigned>(1);
+        mix_ticket_ = FrameQueue(0, stream_);
         check(cudaMemsetAsync(error_.p, 0, sizeof(unsigned), stream_), "memset");
         ctxs_.resize(desc_.max_inflight);
         // Staging for a full batch of query points plus the tables and sources
@@ -282,8 +282,6 @@ public:
         cudaStreamSynchronize(stream_);
         for (auto& kv : sessions_)
             if (kv.second->block) cudaFreeAsync(kv.second->block, stream_);
-        for (auto& k : ocean_kinds_)
-            if (k->queue) cudaFreeAsync(k->queue, stream_);
         for (auto& c : ctxs_) {
             if (c->dev) cudaFreeAsync(c->dev, stream_);
             if (c->start) cudaEventDestroy(c->start);
@@ -549,6 +547,7 @@ private:
         const size_t cells = static_cast<size_t>(k->n) * k->n;
         k->tw = DevBuf<float2>(k->n - 1);
         k->inter = DevBuf<float2>(3 * cells * k->nf);
+        ensure_queue(k.get(), 1024);  // sessions updating in one batch before the words have to grow
         const std::vector<float2> tw = stage_twiddles(k->n);
         check(cudaMemcpyAsync(k->tw.p, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, stream_),
               "twiddles");
@@ -794,10 +793,7 @@ private:
     {
         if (count <= k->queue_cap) return;
         const size_t cap = std::max(count, k->queue_cap * 2);
-        if (k->queue) check(cudaFreeAsync(k->queue, stream_), "free queue");
-        k->queue = nullptr;
-        check(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&k->queue), (1 + 2 * cap) * sizeof(unsigned), pool_,
-                                      stream_), "queue");
+        k->queue = FrameQueue(cap, stream_);  // (freeing the old words waits for their last launch)
         k->queue_cap = cap;
     }
 
@@ -918,10 +914,12 @@ private:
         for (const OceanPart& p : oparts)
             one_launch = one_launch && mixed_size_ok(p.k->log_n) && p.k->nf == oparts[0].k->nf;
         MixedArgs m{};
+        std::vector<FrameQueue::Set> sets;
         for (const OceanPart& p : oparts) {
             OceanKind* k = p.k;
             const int count = static_cast<int>(p.count);
-            check(cudaMemsetAsync(k->queue, 0, (1 + 2 * p.count) * sizeof(unsigned), stream_), "queue reset");
+            const FrameQueue::Set set = k->queue.take(stream_);
+            sets.push_back(set);
             FrameArgs a{};
             a.twiddles = k->tw.p;
             a.t_over_2pi = reinterpret_cast<const double*>(d + p.top);
@@ -932,17 +930,21 @@ private:
             if (one_launch) {
                 MixedGroup& g = m.g[m.groups++];
                 g.a = a;
-                g.rows_done = k->queue + 1;
-                g.cols_done = k->queue + 1 + p.count;
+                g.rows_done = set.counters;
+                g.cols_done = set.counters + p.count;
+                g.clear = set.clear;
+                g.clear_words = set.words;
                 g.count = count;
                 g.slots = std::min(count, 3);
                 g.log_n = k->log_n;
                 continue;
             }
             QueueArgs q;
-            q.ticket = k->queue;
-            q.rows_done = k->queue + 1;
-            q.cols_done = k->queue + 1 + p.count;
+            q.ticket = set.ticket;
+            q.rows_done = set.counters;
+            q.cols_done = set.counters + p.count;
+            q.clear = set.clear;
+            q.clear_words = set.words;
             q.error = error_.p;
             q.count = count;
             q.slots = std::min(count, 3);
@@ -950,6 +952,7 @@ private:
             q.defer = k->nf == 6 ? 1 : 0;
             const int grid = static_cast<int>(std::min<uint64_t>(k->grid, uint64_t(count) * k->n));
             check(launch_frame(k->log_n, k->nf, desc_.fft_form, false, a, q, grid, stream_), "frame kernel");
+            k->queue.launched(set);
             ++kernels;
         }
         if (one_launch) {
@@ -961,7 +964,9 @@ private:
                 first += mixed_tasks(m.g[i].log_n, m.g[i].count);
             }
             m.total = first;
-            m.ticket = mix_ticket_.p;
+            const FrameQueue::Set ticket = mix_ticket_.take(stream_);
+            m.ticket = ticket.ticket;
+            m.clear_ticket = ticket.clear;
             m.error = error_.p;
             m.wait_ns = 1000000000ull;
             const int nf = oparts[0].k->nf;
@@ -973,9 +978,10 @@ private:
                 if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "mixed frame occupancy");
                 grid = per_sm * sms_;
             }
-            check(cudaMemsetAsync(mix_ticket_.p, 0, sizeof(unsigned), stream_), "ticket reset");
             check(launch_mixed_frame(nf, ar, m, static_cast<int>(std::min<uint64_t>(grid, first)), stream_),
                   "mixed frame kernel");
+            mix_ticket_.launched(ticket);
+            for (size_t i = 0; i < oparts.size(); ++i) oparts[i].k->queue.launched(sets[i]);
             ++kernels;
         }
         const IWaveSource* dev_src = reinterpret_cast<const IWaveSource*>(d + src_off);
@@ -1212,7 +1218,7 @@ private:
     cudaStream_t stream_ = nullptr;
     cudaMemPool_t pool_ = nullptr;
     DevBuf<unsigned> error_;
-    DevBuf<unsigned> mix_ticket_;  // the one-launch frame's ticket
+    FrameQueue mix_ticket_;  // the one-launch frame's ticket
     int mix_grid_[2] = {0, 0};     // its resident grid, by field count (4, 6)
     std::vector<std::unique_ptr<BatchCtx>> ctxs_;
     std::deque<BatchCtx*> free_ctx_, inflight_;

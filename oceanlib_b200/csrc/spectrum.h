@@ -47,7 +47,8 @@ struct FrameArgs {
     const float* kvec;         // [geoms][N]
     const float2* twiddles;    // [N-1] per-stage inverse twiddles
     const OceanConsts* consts; // [count]
-    const double* t_over_2pi;  // [count]
+    const double* t_over_2pi;  // [count], or null: every ocean at t_uniform
+    double t_uniform;          // t / 2 pi of every ocean (t_over_2pi null)
     float2* inter;             // [chunk][N][N][NF] row-pass output
     float4* disp;              // [count][N*N]
     float4* normal;            // [count][N*N]
@@ -69,7 +70,9 @@ struct FrameArgs {
 };
 
 // Work queue of the persistent frame kernel. `ticket`, `rows_done[count]` and
-// `cols_done[count]` must be zero at launch (one contiguous block).
+// `cols_done[count]` must be zero at launch. The launch itself zeroes
+// clear[0 .. clear_words), the words of the next launch's queue (FrameQueue in
+// host_util.h keeps two in turn), so a frame needs no reset in front of it.
 struct QueueArgs {
     unsigned* ticket;
     unsigned* rows_done;
@@ -78,6 +81,8 @@ struct QueueArgs {
     int32_t count;        // oceans in the frame (inter holds `slots` of them)
     int32_t slots;        // intermediate ring slots
     unsigned long long wait_ns;
+    unsigned* clear;
+    uint32_t clear_words;
     // 1: a row task's counter add waits until the CTA's next task has staged
     // its inputs (when that task waits on nothing), so its release does not
     // stall the CTA; 0: the add comes before the next task. Either way a
@@ -115,7 +120,8 @@ cudaError_t launch_wait_probe(const unsigned* counter, unsigned target, unsigned
 // .. 1024 (log_n 5..10), one field count for all groups, FP32 forms, no
 // persistent foam. Group g's tickets are [first, first + tasks), tasks =
 // mixed_tasks(log_n, count); its rows_done / cols_done (count each) and the
-// ticket must be zero at launch.
+// ticket must be zero at launch, which clears the next launch's words, each
+// group's and `clear_ticket`, as QueueArgs says.
 constexpr int kMaxMixedGroups = 6;
 struct MixedGroup {
     FrameArgs a;          // the group's arrays, or its pointer table (ocean_base 0)
@@ -125,12 +131,15 @@ struct MixedGroup {
     int32_t count;        // oceans
     int32_t slots;        // intermediate ring slots (a.inter holds them)
     int32_t log_n;
+    unsigned* clear;      // next launch's words of this group
+    uint32_t clear_words;
 };
 struct MixedArgs {
     MixedGroup g[kMaxMixedGroups];
     int32_t groups;
     uint32_t total;       // tickets of all groups
     unsigned* ticket;
+    unsigned* clear_ticket;  // may be null
     unsigned* error;      // sticky: set when a bounded wait gives up
     unsigned long long wait_ns;
     int32_t defer;        // as QueueArgs::defer, for every group
