@@ -22,6 +22,7 @@
 // the other row already in shared memory, so h0 is read from HBM once.
 #include "frame_cells.cuh"
 #include "ocean_device.cuh"
+#include "queue_device.cuh"
 #include "spectrum.h"
 #include "tc_dft.cuh"
 #include "tc_dft_small.cuh"
@@ -245,11 +246,6 @@ __device__ __forceinline__ void transform_all(float2* data, const float2* tws, i
 // ---------------------------------------------------------------------------
 constexpr unsigned long long kH0WaitNs = 1000000000ull;  // 1 s
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p)
-{
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
 // Once per CTA (thread 0), before the CTA's first barrier.
 __device__ __forceinline__ void h0_bar_init(uint64_t* bar)
 {
@@ -298,20 +294,6 @@ __device__ __forceinline__ void h0_rows_wait(uint64_t* bar, uint32_t parity, uns
             return;
         }
     }
-}
-
-// Release add at GPU scope: every write that happens before it (the CTA's,
-// through the preceding barrier) is visible to an acquirer that sees the sum.
-__device__ __forceinline__ void red_release_add(unsigned* p, unsigned v)
-{
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
 }
 
 // The persistent queues' counter adds that a task makes once its inputs are
@@ -701,31 +683,6 @@ col_pass_kernel(FrameArgs a)
 // and leaves, and the others give up in turn.
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ unsigned long long global_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Spin until *counter >= target or the error word is set or limit_ns passes.
-// Returns false on timeout / abort.
-__device__ bool wait_at_least(const unsigned* counter, unsigned target, unsigned* error,
-                              unsigned long long limit_ns)
-{
-    if (ld_acquire(counter) >= target) return true;
-    const unsigned long long t0 = global_ns();
-    while (true) {
-        __nanosleep(64);
-        if (ld_acquire(counter) >= target) return true;
-        if (ld_acquire(error) != 0u) return false;
-        if (global_ns() - t0 > limit_ns) {
-            atomicCAS(error, 0u, 1u);
-            return false;
-        }
-    }
-}
-
 // Resident CTAs the persistent kernel is compiled for: 768 threads per SM
 // (at N = 1024, whose 32 values per lane need the registers, two CTAs of
 // single rows).
@@ -756,12 +713,6 @@ __host__ __device__ constexpr size_t frame_engine_offset()
 {
     return ((frame_data_float2<FramePlan<LOG_N, true>, NF>() + (size_t(1) << LOG_N)) * sizeof(float2) + 127) /
            128 * 128;
-}
-
-// Zeroes the next launch's queue words, each CTA its share (QueueArgs).
-__device__ __forceinline__ void clear_words(unsigned* words, uint32_t count, int tid, int nt)
-{
-    for (uint32_t i = blockIdx.x * nt + tid; i < count; i += gridDim.x * nt) words[i] = 0u;
 }
 
 template <class P, int NF, int AR, bool FOAM>
@@ -1365,8 +1316,8 @@ cudaError_t col_dispatch_n(int nf, int ar, bool foam, const FrameArgs& a, cudaSt
 
 }  // namespace
 
-static_assert(frame_plan_count<8>(false) <= kMaxFramePlans && frame_plan_count<9>(false) <= kMaxFramePlans &&
-                  frame_plan_count<10>(false) <= kMaxFramePlans,
+static_assert(frame_plan_count<8>(false) <= kPairPlan && frame_plan_count<9>(false) <= kPairPlan &&
+                  frame_plan_count<10>(false) <= kPairPlan && kPairPlan < kMaxFramePlans,
               "the host sizes its per-plan tables by kMaxFramePlans");
 
 int frame_plan_count(int log_n, int form)
@@ -1375,10 +1326,22 @@ int frame_plan_count(int log_n, int form)
     return (form != 2 && log_n >= 8) ? 2 : 1;
 }
 
+int kernel_plan(int log_n, int form, int plan, int count)
+{
+    return plan == 0 && form != 2 && pair_frame_ok(log_n, count) ? kPairPlan : plan;
+}
+
+int frame_ring_slots(int log_n, int form, int slots, int count)
+{
+    const int ring = kernel_plan(log_n, form, 0, count) == kPairPlan ? pair_frame_ring(slots) : slots;
+    return ring < count ? ring : count;
+}
+
 int frame_blocks_per_sm(int log_n, int nf, int form, bool fuse_foam, int plan)
 {
     if (log_n < 4 || log_n > 10) return 0;
     if (form == 2 && (log_n < 6 || log_n > 9)) return 0;
+    if (plan == kPairPlan) return form == 2 ? 0 : pair_frame_blocks_per_sm(log_n, nf, arith_of_form(form), fuse_foam);
     if (plan < 0 || plan >= frame_plan_count(log_n, form)) return 0;
     return frame_dispatch(log_n, nf, form, fuse_foam, plan, [](auto L) { return decltype(L)::blocks_per_sm(); });
 }
@@ -1388,6 +1351,10 @@ cudaError_t launch_frame(int log_n, int nf, int form, bool fuse_foam, const Fram
 {
     if (log_n < 4 || log_n > 10) return cudaErrorInvalidValue;
     if (form == 2 && (log_n < 6 || log_n > 9)) return cudaErrorInvalidValue;
+    if (plan == kPairPlan) {
+        if (form == 2) return cudaErrorInvalidValue;
+        return launch_pair_frame(log_n, nf, arith_of_form(form), fuse_foam, a, q, grid, st);
+    }
     if (plan < 0 || plan >= frame_plan_count(log_n, form)) return cudaErrorInvalidValue;
     return frame_dispatch(log_n, nf, form, fuse_foam, plan,
                           [&](auto L) { return decltype(L)::launch(a, q, grid, st); });

@@ -68,7 +68,7 @@ struct Large {
     static constexpr int THREADS = 2 * G;           // two rows (columns) per task
     static constexpr int CTAS = 512 / THREADS;      // resident per SM: 128 registers a thread
     static constexpr int TASKS = N / 2;             // per ocean and pass
-    static constexpr int SEQ = padded_len(N) + 8;   // exchange stride (f32x2): the two rows 8 bank pairs apart
+    static constexpr int SEQ = seq_stride_bytes(N, 16, 2, false) / 8;  // exchange stride (f32x2)
     static constexpr int HELD = 15;                 // of a thread's 16 cells, those the column stash holds
     static constexpr int BUF = 2 * SEQ;
     static constexpr size_t EXCHANGE = sizeof(f32x2) * BUF;
@@ -92,102 +92,6 @@ struct Place {
     }
 };
 
-// The unnormalised inverse transform of a pair of sequences whose index
-// c + j N/16 is in slot j; afterwards slot j holds index(j).
-template <int LOG_N, int AR>
-struct LargeFft {
-    static constexpr int G = Large<LOG_N>::G;
-    using B0 = PairBlock<LOG_N, G, 0, AR>;
-    using B1 = PairBlock<LOG_N, G, 4, AR>;
-    using B2 = PairBlock<LOG_N, G, 8, AR>;
-    static_assert(B0::r == 4 && B1::r == 4 && 8 + B2::r == LOG_N, "three blocks cover the stages");
-
-    // Hands 8 bytes of every slot from one block to the next: a part of the
-    // pair, or both parts of one sequence.
-    template <class From, class To>
-    __device__ __forceinline__ static void exchange(f32x2 (&v)[16], f32x2* buf, int c)
-    {
-        static_assert(From::C * From::RR == 16 && To::C * To::RR == 16, "16 slots");
-        __syncthreads();  // the buffer's last readers are done
-#pragma unroll
-        for (int j = 0; j < 16; ++j) buf[pad_idx(From::index_after(j / From::RR, j % From::RR, c))] = v[j];
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = buf[pad_idx(To::index_before(j / To::RR, j % To::RR, c))];
-    }
-    template <class From, class To>
-    __device__ __forceinline__ static void exchange(float (&x)[16], float (&y)[16], f32x2* buf, int c)
-    {
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            buf[pad_idx(From::index_after(j / From::RR, j % From::RR, c))] = px_pack(x[j], y[j]);
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) px_unpack(buf[pad_idx(To::index_before(j / To::RR, j % To::RR, c))], x[j], y[j]);
-    }
-
-    template <class B>
-    __device__ __forceinline__ static void block(f32x2 (&re)[16], f32x2 (&im)[16], const float2* tw, int c)
-    {
-        B::compute(reinterpret_cast<f32x2(&)[B::C][B::RR]>(re), reinterpret_cast<f32x2(&)[B::C][B::RR]>(im), tw, c);
-    }
-    template <class B>
-    __device__ __forceinline__ static void block(float (&x)[16], float (&y)[16], const float2* tw, int c)
-    {
-        B::compute_f64(reinterpret_cast<float(&)[B::C][B::RR]>(x), reinterpret_cast<float(&)[B::C][B::RR]>(y), tw, c);
-    }
-
-    __device__ __forceinline__ static void run(f32x2 (&re)[16], f32x2 (&im)[16], const float2* tw, const Place<LOG_N>& p)
-    {
-        if constexpr (AR == kArPrecise) {
-            // The two sequences one after the other, so that the FP64 values
-            // of one block (64 registers) and the other sequence's FP32 values
-            // (32) are all a lane holds.
-            float ax[16], ay[16], bx[16], by[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                px_unpack(re[j], ax[j], bx[j]);
-                px_unpack(im[j], ay[j], by[j]);
-            }
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                block<B0>(ax, ay, tw, p.c);
-                exchange<B0, B1>(ax, ay, p.buf, p.c);
-                block<B1>(ax, ay, tw, p.c);
-                exchange<B1, B2>(ax, ay, p.buf, p.c);
-                block<B2>(ax, ay, tw, p.c);
-                // The sequences change places: twice round is the original order.
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float tx = ax[j], ty = ay[j];
-                    ax[j] = bx[j];
-                    ay[j] = by[j];
-                    bx[j] = tx;
-                    by[j] = ty;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                re[j] = px_pack(ax[j], bx[j]);
-                im[j] = px_pack(ay[j], by[j]);
-            }
-        } else {
-            block<B0>(re, im, tw, p.c);
-            exchange<B0, B1>(re, p.buf, p.c);
-            exchange<B0, B1>(im, p.buf, p.c);
-            block<B1>(re, im, tw, p.c);
-            exchange<B1, B2>(re, p.buf, p.c);
-            exchange<B1, B2>(im, p.buf, p.c);
-            block<B2>(re, im, tw, p.c);
-        }
-    }
-    __device__ __forceinline__ static int index(int j, const Place<LOG_N>& p)
-    {
-        return B2::index_after(j / B2::RR, j % B2::RR, p.c);
-    }
-};
-
 // Brings `bytes` (a multiple of 16 KB) at `p` into the L2: threads
 // [first, first + bytes / 16 KB) of the CTA take a piece each.
 __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes, int first)
@@ -206,19 +110,11 @@ __device__ __forceinline__ void load_twiddles(float2* tws, const float2* __restr
     for (int i = threadIdx.x; i < Large<LOG_N>::N - 1; i += Large<LOG_N>::THREADS) tws[i] = __ldg(&src[i]);
 }
 
-// A read-only load that stays where it is written.
-__device__ __forceinline__ float2 load_now(const float2* p)
-{
-    float2 v;
-    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
-    return v;
-}
-
 template <int LOG_N, int NF, int AR>
 __global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) large_row_kernel(FrameArgs a)
 {
     using S = Large<LOG_N>;
-    using Fft = LargeFft<LOG_N, AR>;
+    using Fft = RegFft<LOG_N, 16, AR, false>;
     constexpr int N = S::N, G = S::G, Q = NF / 2, NT = S::THREADS;
     extern __shared__ float4 smem4[];
     const int tid = threadIdx.x;
@@ -313,10 +209,10 @@ __global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) lar
                     im[j] = px_pack(pa.y, pb.y);
                 }
             }
-            Fft::run(re, im, tws, p);
+            Fft::run(re, im, p.buf, tws, p.c);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                const int x = Fft::index(j, p);
+                const int x = Fft::index(j, p.c);
                 out[(static_cast<size_t>(x >> 1) * Q + q) * 2 * N + (x & 1)] = make_ulonglong2(re[j], im[j]);
             }
         }
@@ -327,7 +223,7 @@ template <int LOG_N, int NF, int AR>
 __global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) large_col_kernel(FrameArgs a)
 {
     using S = Large<LOG_N>;
-    using Fft = LargeFft<LOG_N, AR>;
+    using Fft = RegFft<LOG_N, 16, AR, false>;
     constexpr int N = S::N, Q = NF / 2, NT = S::THREADS;
     constexpr unsigned kPairBytes = 2u * N * sizeof(float4);  // a task's pair
     extern __shared__ float4 smem4[];
@@ -364,7 +260,7 @@ __global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) lar
                 re[j] = px_pack(v.x, v.y);
                 im[j] = px_pack(v.z, v.w);
             }
-            Fft::run(re, im, tws, p);
+            Fft::run(re, im, p.buf, tws, p.c);
             const int ocean = a.ocean_base + task / S::TASKS;
             const size_t base = static_cast<size_t>(ocean) * cells + 2 * (task % S::TASKS) + p.r;
             if (Q == 3 && q == 2) {
@@ -373,7 +269,7 @@ __global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) lar
                     float ux, uz, uy, zero;
                     px_unpack(re[j], ux, uz);
                     px_unpack(im[j], uy, zero);
-                    __stcs(&a.velocity[base + static_cast<size_t>(Fft::index(j, p)) * N], make_float4(ux, uy, uz, 0.0f));
+                    __stcs(&a.velocity[base + static_cast<size_t>(Fft::index(j, p.c)) * N], make_float4(ux, uy, uz, 0.0f));
                 }
             } else if (q == 0) {
 #pragma unroll
@@ -390,7 +286,7 @@ __global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) lar
                     px_unpack(re[j], f2.x, f3.x);
                     px_unpack(im[j], f2.y, f3.y);
                     const CellOut c = finalize_cell(f0, f1, f2, f3, cst.lambda, cst.foam_threshold, cst.inv_threshold);
-                    const size_t idx = base + static_cast<size_t>(Fft::index(j, p)) * N;
+                    const size_t idx = base + static_cast<size_t>(Fft::index(j, p.c)) * N;
                     __stcs(&a.disp[idx], c.disp);
                     __stcs(&a.normal[idx], c.normal);
                 }

@@ -1,0 +1,416 @@
+// oceanlib-b200: the persistent frame with its transforms in registers.
+//
+// The same frame, queue protocol and arithmetic as frame_kernel (frame.cu), for
+// the sizes where it is the faster one (pair_frame_ok). There, a task's every
+// field sat in shared memory and each step of the frame - evolve, three stage
+// blocks, the store - read and wrote all of it: the shared-memory pipe was the
+// frame's busiest unit (71% of 64 x 512^2 with velocity and foam). Here a task
+// takes ROWS neighbouring rows (columns) through the field pairs one after the
+// other, E indices of a pair a lane, and a value passes through shared memory
+// only between two stage blocks:
+//
+//   rows     evolve straight into the first block's registers; the last block's
+//            registers go to the intermediate. The evolved amplitudes and 1/|k|
+//            wait in the thread's own shared memory for the later pairs; the
+//            velocity pair, which needs more of the cell, goes first.
+//   columns  the first block reads the intermediate; the last block's registers
+//            are finalized and stored. The first pair waits in the thread's own
+//            shared memory until the second completes the cell; the velocity
+//            pair goes last, with the foam step, which needs the cell's foam
+//            source (kept in the same place) and velocity.
+//
+// Neighbouring threads are the same lane of the task's ROWS rows (columns), and
+// the intermediate is inter[x / ROWS][pair][y][x % ROWS], 16 bytes (a.re, b.re,
+// a.im, b.im) a cell and pair: a warp reads it in whole 512-byte runs, writes it
+// in runs of ROWS^2 x 16 bytes and writes the outputs in runs of ROWS x 16.
+//
+// A CTA has T = 256 threads and three are resident, so three times as many rows
+// are in flight as with a task's pairs side by side. So that a column task does
+// not wait for rows still in flight, the queue runs the rows `ahead` oceans
+// before the columns, R(0) .. R(ahead - 1) | R(ahead) C(0) | R(ahead + 1) C(1) |
+// .. | C(count - 1), through a ring of `ring` slots: 4 and 8 at three ring slots
+// of the batch's own count, 2 and 5 at two. Every awaited task holds an earlier
+// ticket, as in frame_kernel, since the ring has more slots than rows run ahead.
+// 64 x 512^2 with velocity, us a frame by (ahead, ring): (2, 4) 983, (2, 5) 810,
+// (3, 6) 740, (3, 7) 715, (4, 8) 672, (5, 10) 664.
+#include "frame_cells.cuh"
+#include "ocean_device.cuh"
+#include "queue_device.cuh"
+#include "spectrum.h"
+
+#include <type_traits>
+
+namespace ocean_b200 {
+namespace {
+
+// E indices of a pair a lane, ROWS rows (columns) a task.
+template <int LOG_N_, int E_, int ROWS_>
+struct RegPlan {
+    static constexpr int LOG_N = LOG_N_, N = 1 << LOG_N, E = E_, ROWS = ROWS_;
+    static constexpr int G = N / E;             // lanes per pair
+    static constexpr int T = ROWS * G;          // threads
+    static constexpr int CTAS = 768 / T;        // resident per SM: 80 registers a thread
+    static constexpr int TASKS = N / ROWS;      // per ocean, rows and columns alike
+    static constexpr int SEQ = seq_stride_bytes(N, E, ROWS, false);
+    // Shared memory, in bytes from the start: exchange buffers, twiddles, the
+    // threads' own values (16 bytes a cell in a column task).
+    static constexpr size_t TW = ROWS * SEQ;
+    static constexpr size_t HELD = TW + sizeof(float2) * N;
+    static constexpr size_t SMEM = HELD + sizeof(float4) * E * T;
+    static_assert(E * T == ROWS * N && TW % 16 == 0 && HELD % 16 == 0, "a thread holds E cells");
+    static_assert(CTAS * (SMEM + 1280) <= 228 * 1024, "the resident CTAs fit on an SM");
+};
+template <int LOG_N>
+using PairPlan = RegPlan<LOG_N, 8, 4>;
+
+// Ring slots of a launch with q.slots = slots (see above).
+__host__ __device__ constexpr unsigned ring_of(unsigned slots) { return 3u * slots - 1u; }
+static_assert(ring_of(3) > 4 && ring_of(2) > 2 && ring_of(1) > 1, "more slots than rows run ahead");
+
+// Adds this CTA's finished row task (pub[0]) or its own column task (pub[1]).
+__device__ __forceinline__ void publish(unsigned* counter, int tid)
+{
+    if (tid == 0 && counter != nullptr) red_release_add(counter, 1u);
+}
+
+template <class P, int NF, int AR>
+__device__ __forceinline__ void pair_row_task(const FrameArgs& a, int ocean, int task, float2* inter_slot,
+                                              unsigned char* smem, int tid, unsigned* const* pub)
+{
+    using Fft = RegFft<P::LOG_N, P::E, AR, false>;
+    constexpr int N = P::N, G = P::G, E = P::E, ROWS = P::ROWS, T = P::T, Q = NF / 2;
+    const int r = tid % ROWS, c = tid / ROWS;
+    void* buf = smem + r * P::SEQ;
+    const float2* tws = reinterpret_cast<const float2*>(smem + P::TW);
+    float2* held_h = reinterpret_cast<float2*>(smem + P::HELD) + tid;                         // (hr, hi) of cell j at [j * T]
+    float* held_k = reinterpret_cast<float*>(smem + P::HELD + sizeof(float2) * E * T) + tid;  // its 1/|k|
+
+    // Rows and the rows with their mirrors are neighbouring tasks: the second
+    // read of h0 finds it in the L2.
+    const int y = ROWS * ((task & 1) ? P::TASKS - 1 - (task >> 1) : (task >> 1)) + r;
+    const float2 *geom, *h0;
+    const float* kvec;
+    if (a.table != nullptr) {
+        const OceanSlot& s = a.table[ocean];
+        geom = s.omega_kinv;
+        kvec = s.kvec;
+        h0 = s.h0;
+    } else {
+        const int g = a.consts[ocean].geom;
+        geom = a.omega_kinv + static_cast<size_t>(g) * N * N;
+        kvec = a.kvec + static_cast<size_t>(g) * N;
+        h0 = a.h0 + static_cast<size_t>(ocean) * N * N;
+    }
+    const double top = frame_time(a, ocean);
+    const float kz = __ldg(&kvec[y]);
+    const float2* h0_row = h0 + y * N;
+    const float2* h0_mirror = h0 + ((N - y) & (N - 1)) * N;
+    geom += y * N;
+    ulonglong2* out = reinterpret_cast<ulonglong2*>(inter_slot) + y * ROWS;
+#pragma unroll 1
+    for (int k = 0; k < Q; ++k) {
+        const int q = Q == 3 ? (k + 2) % 3 : k;  // the velocity pair first
+        f32x2 re[E], im[E];
+        if (k == 0) {
+            float2 av[E], bm[E], wk[E];
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                const int x = c + G * j;
+                av[j] = load_now(&h0_row[x]);
+                bm[j] = load_now(&h0_mirror[(N - x) & (N - 1)]);
+                wk[j] = load_now(&geom[x]);
+            }
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                const float kx = __ldg(&kvec[c + G * j]);
+                const Amplitude e = evolve_amplitude(av[j], bm[j], wk[j].x, top);
+                held_h[j * T] = make_float2(e.hr, e.hi);
+                held_k[j * T] = wk[j].y;
+                float2 pa, pb;
+                if constexpr (Q == 3) {
+                    evolve_pair2(e.dr, e.di, wk[j].x, wk[j].y, kx, kz, pa, pb);
+                } else {
+                    evolve_pair0(e.hr, e.hi, wk[j].y, kx, kz, pa, pb);
+                }
+                re[j] = px_pack(pa.x, pb.x);
+                im[j] = px_pack(pa.y, pb.y);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                const float kx = __ldg(&kvec[c + G * j]);
+                const float2 h = held_h[j * T];
+                const float ki = held_k[j * T];
+                float2 pa, pb;
+                if (Q == 3 && q == 0) {
+                    evolve_pair0(h.x, h.y, ki, kx, kz, pa, pb);
+                } else {
+                    evolve_pair1(h.x, h.y, ki, kx, kz, pa, pb);
+                }
+                re[j] = px_pack(pa.x, pb.x);
+                im[j] = px_pack(pa.y, pb.y);
+            }
+        }
+        Fft::run(re, im, buf, tws, c);
+        if (k == 0) publish(pub[0], tid);  // the CTA's previous row task, whose stores have drained by now
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const int x = Fft::index(j, c);
+            out[((x / ROWS) * Q + q) * N * ROWS + x % ROWS] = make_ulonglong2(re[j], im[j]);
+        }
+    }
+}
+
+template <class P, int NF, int AR, bool FOAM>
+__device__ __forceinline__ void pair_col_task(const FrameArgs& a, int ocean, int strip, const float2* inter_slot,
+                                              unsigned char* smem, int tid, unsigned* const* pub)
+{
+    using Fft = RegFft<P::LOG_N, P::E, AR, false>;
+    constexpr int N = P::N, E = P::E, ROWS = P::ROWS, T = P::T, Q = NF / 2;
+    const int w = tid % ROWS, c = tid / ROWS;
+    void* buf = smem + w * P::SEQ;
+    const float2* tws = reinterpret_cast<const float2*>(smem + P::TW);
+    ulonglong2* held = reinterpret_cast<ulonglong2*>(smem + P::HELD) + tid;  // pair 0 of cell j at [j * T]
+    float* src = reinterpret_cast<float*>(held);                             // later its foam source, at [4 T j]
+    const int x0 = strip * ROWS;
+    const size_t base = static_cast<size_t>(ocean) * N * N;
+#pragma unroll 1
+    for (int q = 0; q < Q; ++q) {
+        const float4* in = reinterpret_cast<const float4*>(inter_slot) + (strip * Q + q) * N * ROWS + tid;
+        f32x2 re[E], im[E];
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const float4 v = __ldcg(in + T * j);
+            re[j] = px_pack(v.x, v.y);
+            im[j] = px_pack(v.z, v.w);
+        }
+        Fft::run(re, im, buf, tws, c);
+        if (q == 0) publish(pub[0], tid);
+        // Every thread's values of the last pair were in registers before the
+        // transform's first barrier: the slot is free.
+        if (q == Q - 1) publish(pub[1], tid);
+        float4 *out_disp, *out_normal, *out_vel;
+        OceanConsts cst;
+        if (a.table != nullptr) {
+            const OceanSlot& s = a.table[ocean];
+            out_disp = s.disp;
+            out_normal = s.normal;
+            out_vel = s.velocity;
+            cst = s.cst;
+        } else {
+            out_disp = a.disp + base;
+            out_normal = a.normal + base;
+            out_vel = a.velocity + base;
+            cst = a.consts[ocean];
+        }
+        if (q == 0) {
+#pragma unroll
+            for (int j = 0; j < E; ++j) held[j * T] = make_ulonglong2(re[j], im[j]);
+        } else if (q == 1) {
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                const ulonglong2 h = held[j * T];
+                float2 f0, f1, f2, f3;
+                px_unpack(h.x, f0.x, f1.x);
+                px_unpack(h.y, f0.y, f1.y);
+                px_unpack(re[j], f2.x, f3.x);
+                px_unpack(im[j], f2.y, f3.y);
+                const CellOut o = finalize_cell(f0, f1, f2, f3, cst.lambda, cst.foam_threshold, cst.inv_threshold);
+                const int idx = Fft::index(j, c) * N + x0 + w;
+                __stcs(&out_disp[idx], o.disp);
+                __stcs(&out_normal[idx], o.normal);
+                if constexpr (FOAM) src[4 * T * j] = o.disp.w;
+            }
+        } else {
+            // The foam step's taps, within a cell or so of the strip, straight
+            // from memory: staging the strip's surroundings in shared memory,
+            // four bytes a copy, cost more than the loads (921 us against 881
+            // for 64 x 512^2).
+            const float* cur = a.foam_cur + base;
+            auto foam_get = [&](int zz, int xx) { return __ldg(&cur[zz * N + xx]); };
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                float ux, uz, uy, zero;
+                px_unpack(re[j], ux, uz);
+                px_unpack(im[j], uy, zero);
+                const int y = Fft::index(j, c);
+                const int idx = y * N + x0 + w;
+                __stcs(&out_vel[idx], make_float4(ux, uy, uz, 0.0f));
+                if constexpr (FOAM) {
+                    const FoamTaps t = foam_taps(N, x0 + w, y, ux, uz, a.foam_dt, a.foam_scale, a.foam_drift_x,
+                                                 a.foam_drift_z, a.foam_inv_cell, foam_get);
+                    __stcs(&a.foam_next[base + idx],
+                           foam_finish(t, src[4 * T * j], a.foam_decay, a.foam_gain));
+                }
+            }
+        }
+    }
+}
+
+template <int LOG_N, int NF, int AR, bool FOAM>
+__global__ void __launch_bounds__(PairPlan<LOG_N>::T, PairPlan<LOG_N>::CTAS) pair_frame_kernel(FrameArgs a, QueueArgs q)
+{
+    using P = PairPlan<LOG_N>;
+    constexpr int N = P::N;
+    constexpr unsigned TASKS = P::TASKS;
+    extern __shared__ float4 smem4[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(smem4);
+    // Thread 0's queue state between tasks, as in frame_kernel.
+    __shared__ unsigned s_ticket;
+    __shared__ int s_ok;
+    __shared__ unsigned* s_publish;
+    __shared__ unsigned* s_pub[2];
+    unsigned r_next = 0;  // thread 0: the ticket drawn one task ahead
+    int r_have_next = 0;
+
+    const int tid = threadIdx.x;
+    clear_words(q.clear, q.clear_words, tid, P::T);
+    float2* tws = reinterpret_cast<float2*>(smem + P::TW);
+    for (int i = tid; i < N - 1; i += P::T) tws[i] = a.twiddles[i];
+
+    const unsigned count = static_cast<unsigned>(q.count);
+    const unsigned slots = static_cast<unsigned>(q.slots);
+    const unsigned ring = min(ring_of(slots), count);
+    const unsigned ahead = min(max(2u * slots, 3u) - 2u, count);
+    const unsigned total = 2u * count * TASKS;
+    // Ticket -> (row?, ocean, task index) for the queue order above.
+    auto decode = [&](unsigned t, bool& row, unsigned& ocean, unsigned& idx) {
+        idx = t % TASKS;
+        unsigned b = t / TASKS;  // R(0 .. ahead - 1), then R(ahead + i), C(i) in turn, then the last C's
+        if (b < ahead) {
+            row = true, ocean = b;
+            return;
+        }
+        b -= ahead;
+        const unsigned pairs = count - ahead;
+        row = b < 2u * pairs && (b & 1u) == 0u;
+        ocean = b < 2u * pairs ? (b >> 1) + (row ? ahead : 0u) : b - pairs;
+    };
+    if (tid == 0) {
+        s_publish = nullptr;
+        r_next = atomicAdd(q.ticket, 1u);
+        r_have_next = 1;
+    }
+    // frame_kernel's protocol: a ticket drawn one task ahead far from the end,
+    // the finished row task published by the next task unless that has to wait.
+    while (true) {
+        __syncthreads();  // previous task's writes issued; shared memory free
+        if (tid == 0) {
+            unsigned* prev = s_publish;
+            const unsigned t = r_have_next ? r_next : atomicAdd(q.ticket, 1u);
+            r_have_next = 0;
+            int ok = 1;
+            unsigned* pub = nullptr;
+            unsigned* self = nullptr;
+            const unsigned* dep = nullptr;
+            if (t < total) {
+                if (t + 2u * gridDim.x < total) {
+                    r_next = atomicAdd(q.ticket, 1u);
+                    r_have_next = 1;
+                }
+                bool row;
+                unsigned ocean, idx;
+                decode(t, row, ocean, idx);
+                if (row) {
+                    if (ocean >= ring) dep = q.cols_done + (ocean - ring);
+                    pub = q.rows_done + ocean;
+                } else {
+                    dep = q.rows_done + ocean;
+                    self = q.cols_done + ocean;
+                }
+            }
+            if (t >= total || !q.defer || (dep != nullptr && ld_acquire(dep) < TASKS)) {
+                if (prev != nullptr) red_release_add(prev, 1u);
+                prev = nullptr;
+                if (dep != nullptr) ok = wait_at_least(dep, TASKS, q.error, q.wait_ns);
+            }
+            s_pub[0] = prev;
+            s_pub[1] = self;
+            s_publish = pub;
+            s_ticket = t;
+            s_ok = ok;
+        }
+        __syncthreads();
+        const unsigned t = s_ticket;
+        if (t >= total || !s_ok) break;
+        bool row;
+        unsigned ocean, idx;
+        decode(t, row, ocean, idx);
+        float2* inter = a.inter + static_cast<size_t>(ocean % ring) * N * N * NF;
+        const int abs_ocean = a.ocean_base + static_cast<int>(ocean);
+        if (row) {
+            pair_row_task<P, NF, AR>(a, abs_ocean, static_cast<int>(idx), inter, smem, tid, s_pub);
+        } else {
+            pair_col_task<P, NF, AR, FOAM>(a, abs_ocean, static_cast<int>(idx), inter, smem, tid, s_pub);
+        }
+    }
+}
+
+template <int LOG_N, int NF, int AR, bool FOAM>
+struct PairLaunch {
+    using P = PairPlan<LOG_N>;
+    static constexpr size_t SMEM = P::SMEM;
+
+    static cudaError_t prepare()
+    {
+        return cudaFuncSetAttribute(pair_frame_kernel<LOG_N, NF, AR, FOAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(SMEM));
+    }
+    static int blocks_per_sm()
+    {
+        int n = 0;
+        if (prepare() != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pair_frame_kernel<LOG_N, NF, AR, FOAM>, P::T, SMEM) !=
+            cudaSuccess)
+            return 0;
+        return n;
+    }
+    static cudaError_t launch(const FrameArgs& a, const QueueArgs& q, int grid, cudaStream_t st)
+    {
+        cudaError_t e = prepare();
+        if (e != cudaSuccess) return e;
+        pair_frame_kernel<LOG_N, NF, AR, FOAM><<<grid, P::T, SMEM, st>>>(a, q);
+        return cudaGetLastError();
+    }
+};
+
+// The variant of (log_n, nf, ar, foam) for `fn`.
+template <int LOG_N, int AR, typename Fn>
+auto variant_ar(int nf, bool foam, Fn&& fn)
+{
+    if (nf == 4) return fn(PairLaunch<LOG_N, 4, AR, false>{});
+    if (foam) return fn(PairLaunch<LOG_N, 6, AR, true>{});
+    return fn(PairLaunch<LOG_N, 6, AR, false>{});
+}
+template <int LOG_N, typename Fn>
+auto variant(int nf, int ar, bool foam, Fn&& fn)
+{
+    if (ar == kArFast) return variant_ar<LOG_N, kArFast>(nf, foam, fn);
+    if (ar == kArPrecise) return variant_ar<LOG_N, kArPrecise>(nf, foam, fn);
+    return variant_ar<LOG_N, kArExact>(nf, foam, fn);
+}
+
+}  // namespace
+
+// A task takes its pairs one after the other, so a frame of few oceans, whose
+// tasks do not fill the GPU, is a longer chain here than with a task's pairs side
+// by side (frame_kernel): 512^2 with velocity, us a frame here / there: one ocean
+// 43.0 / 27.2, two 43.2 / 41.0, three 43.1 / 54.5.
+bool pair_frame_ok(int log_n, int count) { return log_n == 9 && count >= 3; }
+
+int pair_frame_ring(int slots) { return static_cast<int>(ring_of(static_cast<unsigned>(slots))); }
+
+int pair_frame_blocks_per_sm(int log_n, int nf, int ar, bool fuse_foam)
+{
+    if (log_n != 9) return 0;
+    return variant<9>(nf, ar, fuse_foam, [](auto L) { return decltype(L)::blocks_per_sm(); });
+}
+
+cudaError_t launch_pair_frame(int log_n, int nf, int ar, bool fuse_foam, const FrameArgs& a, const QueueArgs& q, int grid,
+                              cudaStream_t st)
+{
+    if (log_n != 9) return cudaErrorInvalidValue;
+    return variant<9>(nf, ar, fuse_foam, [&](auto L) { return decltype(L)::launch(a, q, grid, st); });
+}
+
+}  // namespace ocean_b200

@@ -250,10 +250,10 @@ public:
         slots_ = static_cast<int>(std::min<uint32_t>(count_, 3));
         max_slots_ = slots_;
         defer_ = nf_ == 6;
-        // The persistent kernel's ring needs `slots_` oceans; the row/column
+        // The persistent kernels' ring needs `ring` oceans; the row/column
         // passes one per chunk ocean (all a batch above N = 1024 ever uses).
-        const uint32_t inter_oceans =
-            large() ? chunk_ : std::max<uint32_t>(chunk_, static_cast<uint32_t>(slots_));
+        const uint32_t ring = static_cast<uint32_t>(frame_ring_slots(log_n_, form_, slots_, static_cast<int>(count_)));
+        const uint32_t inter_oceans = large() ? chunk_ : std::max(chunk_, ring);
         inter_ = DevBuf<float2>(cells_ * nf_ * inter_oceans);
         queue_ = FrameQueue(count_, stream_);
         error_ = DevBuf<unsigned>(1);
@@ -663,13 +663,14 @@ private:
         q.slots = slots_;
         q.wait_ns = 1000000000ull;
         q.defer = defer_ ? 1 : 0;
-        const int grid = frame_grid(foam);
+        const int plan = kernel_plan(log_n_, form_, plan_, static_cast<int>(k));
+        const int grid = frame_grid(plan, foam);
         // A share below 1 leaves SMs to batches of other sizes running
         // concurrently (the ensemble's schedule).
         const int shared = std::max(1, static_cast<int>(std::lround(grid * grid_share_)));
         const int launch_grid = static_cast<int>(std::min<uint64_t>(shared, uint64_t(k) * n_));
         timed(3, st, [&] {
-            check(launch_frame(log_n_, nf_, form_, foam, a, q, launch_grid, st, plan_),
+            check(launch_frame(log_n_, nf_, form_, foam, a, q, launch_grid, st, plan),
                   "frame kernel");
         });
         queue_.launched(set);
@@ -686,14 +687,14 @@ private:
     }
     static constexpr double kInvTwoPi = 0.159154943091895335769;
 
-    // One wave of resident CTAs of the persistent kernel (computed once).
-    int frame_grid(bool foam)
+    // One wave of resident CTAs of a kernel plan (computed once).
+    int frame_grid(int plan, bool foam)
     {
-        int& grid = frame_grid_[plan_][foam ? 1 : 0];
+        int& grid = frame_grid_[plan][foam ? 1 : 0];
         if (grid == 0) {
             int sms = 0;
             check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "SM count");
-            const int per_sm = frame_blocks_per_sm(log_n_, nf_, form_, foam, plan_);
+            const int per_sm = frame_blocks_per_sm(log_n_, nf_, form_, foam, plan);
             if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "frame occupancy");
             grid = per_sm * sms;
         }
@@ -842,7 +843,7 @@ public:
     // Settles the launch shapes, so a capture issues launches only.
     void prime_shapes()
     {
-        if (persistent_) (void)frame_grid(false);
+        if (persistent_) (void)frame_grid(kernel_plan(log_n_, form_, plan_, static_cast<int>(count_)), false);
     }
 
 private:

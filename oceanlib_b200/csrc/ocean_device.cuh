@@ -489,5 +489,152 @@ __device__ __forceinline__ void fft_pair(ulonglong2* seq, const float2* tw, int 
     PairBlock<LOG_N, G2, 0, AR>::run(seq, tw, lane, bar_id);
 }
 
+// ---------------------------------------------------------------------------
+// Sequence pairs that stay in registers: the transform of a pair over G = N / E
+// lanes, lane c holding the E indices c + j G in slots j (real parts f32x2 in
+// re, imaginary parts in im). The blocks' butterflies are PairBlock's; between
+// two blocks the values pass through `buf`, which the lanes of one CTA share
+// (CTA barriers: every thread of the CTA runs the same transforms, each pair
+// its own buf). WHOLE: 16 bytes an index, two barriers an exchange; else 8
+// bytes - the real parts, then the imaginary parts - and four. Afterwards slot
+// j holds index(j, c). One element of padding after every E keeps a block's
+// stores and loads free of bank conflicts when neighbouring threads are the
+// same lane of neighbouring pairs and the pairs' buffers lie STRIDE bytes apart.
+// ---------------------------------------------------------------------------
+// Bytes from one pair's buffer to the next of `pairs` (a power of two up to 8):
+// the lanes of each pair that one wavefront serves fall into different banks.
+__host__ __device__ constexpr int seq_stride_bytes(int n, int e, int pairs, bool whole)
+{
+    return whole ? ((n + n / e + 7) / 8 * 8 + 8 / pairs) * 16 : ((n + n / e + 15) / 16 * 16 + 16 / pairs) * 8;
+}
+
+template <int LOG_N, int E, int AR, bool WHOLE>
+struct RegFft {
+    static constexpr int N = 1 << LOG_N;
+    static constexpr int G = N / E;
+    static constexpr int LANE_LOG = ilog2c(E);
+    template <int L0>
+    using Block = PairBlock<LOG_N, G, L0, AR>;
+    static constexpr int LAST = (LOG_N - 1) / LANE_LOG * LANE_LOG;  // the last block's first stage
+
+    __device__ __forceinline__ static int pad(int i) { return i + (i >> LANE_LOG); }
+
+    // Hands every slot's value from one block to the next.
+    template <class From, class To>
+    __device__ __forceinline__ static void exchange_part(f32x2 (&v)[E], void* buf, int c)
+    {
+        f32x2* p = static_cast<f32x2*>(buf);
+        __syncthreads();  // the buffer's last readers are done
+#pragma unroll
+        for (int j = 0; j < E; ++j) p[pad(From::index_after(j / From::RR, j % From::RR, c))] = v[j];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = p[pad(To::index_before(j / To::RR, j % To::RR, c))];
+    }
+    template <class From, class To>
+    __device__ __forceinline__ static void exchange(f32x2 (&re)[E], f32x2 (&im)[E], void* buf, int c)
+    {
+        if constexpr (!WHOLE) {
+            exchange_part<From, To>(re, buf, c);
+            exchange_part<From, To>(im, buf, c);
+        } else {
+            ulonglong2* p = static_cast<ulonglong2*>(buf);
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < E; ++j)
+                p[pad(From::index_after(j / From::RR, j % From::RR, c))] = make_ulonglong2(re[j], im[j]);
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                const ulonglong2 v = p[pad(To::index_before(j / To::RR, j % To::RR, c))];
+                re[j] = v.x;
+                im[j] = v.y;
+            }
+        }
+    }
+    template <class From, class To>
+    __device__ __forceinline__ static void exchange(float (&x)[E], float (&y)[E], void* buf, int c)
+    {
+        f32x2* p = static_cast<f32x2*>(buf);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < E; ++j)
+            p[pad(From::index_after(j / From::RR, j % From::RR, c))] = px_pack(x[j], y[j]);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < E; ++j) px_unpack(p[pad(To::index_before(j / To::RR, j % To::RR, c))], x[j], y[j]);
+    }
+
+    template <int L0>
+    __device__ __forceinline__ static void blocks(f32x2 (&re)[E], f32x2 (&im)[E], void* buf, const float2* tw, int c)
+    {
+        using B = Block<L0>;
+        static_assert(B::C * B::RR == E, "a lane holds E indices");
+        B::compute(reinterpret_cast<f32x2(&)[B::C][B::RR]>(re), reinterpret_cast<f32x2(&)[B::C][B::RR]>(im), tw, c);
+        if constexpr (L0 + B::r < LOG_N) {
+            exchange<B, Block<L0 + B::r>>(re, im, buf, c);
+            blocks<L0 + B::r>(re, im, buf, tw, c);
+        }
+    }
+    template <int L0>
+    __device__ __forceinline__ static void blocks(float (&x)[E], float (&y)[E], void* buf, const float2* tw, int c)
+    {
+        using B = Block<L0>;
+        B::compute_f64(reinterpret_cast<float(&)[B::C][B::RR]>(x), reinterpret_cast<float(&)[B::C][B::RR]>(y), tw, c);
+        if constexpr (L0 + B::r < LOG_N) {
+            exchange<B, Block<L0 + B::r>>(x, y, buf, c);
+            blocks<L0 + B::r>(x, y, buf, tw, c);
+        }
+    }
+
+    __device__ __forceinline__ static void run(f32x2 (&re)[E], f32x2 (&im)[E], void* buf, const float2* tw, int c)
+    {
+        if constexpr (AR == kArPrecise) {
+            // The two sequences one after the other, so that the FP64 values
+            // of one block and the other sequence's FP32 values are all a lane
+            // holds (96 registers at E = 16).
+            float ax[E], ay[E], bx[E], by[E];
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                px_unpack(re[j], ax[j], bx[j]);
+                px_unpack(im[j], ay[j], by[j]);
+            }
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                blocks<0>(ax, ay, buf, tw, c);
+                // The sequences change places: twice round is the original order.
+#pragma unroll
+                for (int j = 0; j < E; ++j) {
+                    const float tx = ax[j], ty = ay[j];
+                    ax[j] = bx[j];
+                    ay[j] = by[j];
+                    bx[j] = tx;
+                    by[j] = ty;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                re[j] = px_pack(ax[j], bx[j]);
+                im[j] = px_pack(ay[j], by[j]);
+            }
+        } else {
+            blocks<0>(re, im, buf, tw, c);
+        }
+    }
+    __device__ __forceinline__ static int index(int j, int c)
+    {
+        using B = Block<LAST>;
+        return B::index_after(j / B::RR, j % B::RR, c);
+    }
+};
+
+// A read-only load that stays where it is written: a batch of them is in
+// flight before the first value is used.
+__device__ __forceinline__ float2 load_now(const float2* p)
+{
+    float2 v;
+    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
 
 }  // namespace ocean_b200

@@ -154,7 +154,7 @@ struct OceanKind {
     uint32_t n = 0;
     bool velocity = false;
     int log_n = 0, nf = 4;
-    int grid = 0;
+    int grid[kMaxFramePlans] = {};  // CTAs of one wave by kernel plan
     DevBuf<float2> tw, inter;
     FrameQueue queue;
     size_t queue_cap = 0;
@@ -521,12 +521,18 @@ private:
         return field_kinds_.back().get();
     }
 
+    // Oceans that the frame kernels of a kind hold in its intermediate ring.
+    size_t ring_oceans(const ocean_desc& od) const
+    {
+        return static_cast<size_t>(std::max(3, frame_ring_slots(ilog2u(od.size), desc_.fft_form, 3, 64)));
+    }
+
     // Bytes a new ocean / field kind would add (shared tables).
     size_t ocean_kind_bytes(const ocean_desc& od) const
     {
         const size_t cells = static_cast<size_t>(od.size) * od.size;
         const int nf = od.compute_velocity ? 6 : 4;
-        return round_up((od.size - 1) * sizeof(float2), kAlign) + round_up(3 * cells * nf * sizeof(float2), kAlign);
+        return round_up((od.size - 1) * sizeof(float2), kAlign) + round_up(ring_oceans(od) * cells * nf * sizeof(float2), kAlign);
     }
 
     OceanKind* find_ocean_kind(const ocean_desc& od)
@@ -546,14 +552,17 @@ private:
         k->nf = k->velocity ? 6 : 4;
         const size_t cells = static_cast<size_t>(k->n) * k->n;
         k->tw = DevBuf<float2>(k->n - 1);
-        k->inter = DevBuf<float2>(3 * cells * k->nf);
+        k->inter = DevBuf<float2>(ring_oceans(od) * cells * k->nf);
         ensure_queue(k.get(), 1024);  // sessions updating in one batch before the words have to grow
         const std::vector<float2> tw = stage_twiddles(k->n);
         check(cudaMemcpyAsync(k->tw.p, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, stream_),
               "twiddles");
-        const int per_sm = frame_blocks_per_sm(k->log_n, k->nf, desc_.fft_form, false);
-        if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "frame occupancy");
-        k->grid = per_sm * sms_;
+        // The kernel plans of a few sessions and of many.
+        for (int plan : {kernel_plan(k->log_n, desc_.fft_form, 0, 1), kernel_plan(k->log_n, desc_.fft_form, 0, 64)}) {
+            const int per_sm = frame_blocks_per_sm(k->log_n, k->nf, desc_.fft_form, false, plan);
+            if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "frame occupancy");
+            k->grid[plan] = per_sm * sms_;
+        }
         k->bytes = ocean_kind_bytes(od);
         check(cudaStreamSynchronize(stream_), "twiddles");
         ocean_kinds_.push_back(std::move(k));
@@ -950,8 +959,9 @@ private:
             q.slots = std::min(count, 3);
             q.wait_ns = 1000000000ull;
             q.defer = k->nf == 6 ? 1 : 0;
-            const int grid = static_cast<int>(std::min<uint64_t>(k->grid, uint64_t(count) * k->n));
-            check(launch_frame(k->log_n, k->nf, desc_.fft_form, false, a, q, grid, stream_), "frame kernel");
+            const int plan = kernel_plan(k->log_n, desc_.fft_form, 0, count);
+            const int grid = static_cast<int>(std::min<uint64_t>(k->grid[plan], uint64_t(count) * k->n));
+            check(launch_frame(k->log_n, k->nf, desc_.fft_form, false, a, q, grid, stream_, plan), "frame kernel");
             k->queue.launched(set);
             ++kernels;
         }

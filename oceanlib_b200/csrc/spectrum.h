@@ -97,17 +97,31 @@ struct QueueArgs {
 inline int arith_of_form(int form) { return form == 1 ? 1 : (form == 3 ? 2 : 0); }
 
 // One persistent launch for the whole frame of `q.count` oceans (foam fused
-// when fuse_foam). `form` is an ocean_fft_form (the tensor form: N = 64 to 512).
-// `grid` = CTAs to launch (0 = one wave of resident CTAs).
-// `plan` picks the task plan (0: the default; 1: the alternative of N = 256,
-// 512 and 1024, see frame_plan_count).
+// when fuse_foam). `form` is an ocean_fft_form (the tensor form: N = 64 to 512),
+// `plan` a kernel plan (kernel_plan), `grid` the CTAs to launch.
 cudaError_t launch_frame(int log_n, int nf, int form, bool fuse_foam, const FrameArgs& args,
-                         const QueueArgs& q, int grid, cudaStream_t stream, int plan = 0);
+                         const QueueArgs& q, int grid, cudaStream_t stream, int plan);
 // Resident CTAs per SM of the persistent frame kernel (0: no such variant).
-int frame_blocks_per_sm(int log_n, int nf, int form, bool fuse_foam, int plan = 0);
-// Task plans the persistent kernel has for a size and form (1 or 2).
+int frame_blocks_per_sm(int log_n, int nf, int form, bool fuse_foam, int plan);
+// Task plans a caller may choose for a size and form (1 or 2): 0 the default,
+// 1 the alternative of N = 256, 512 and 1024.
 int frame_plan_count(int log_n, int form);
-constexpr int kMaxFramePlans = 2;  // frame_plan_count never exceeds it
+// The kernel plan of a launch of `count` oceans under task plan `plan`: the
+// plan itself, or kPairPlan, the register-resident frame (frame_pairs.cu), where
+// plan 0 takes that.
+constexpr int kPairPlan = 2;
+constexpr int kMaxFramePlans = 3;  // kernel plans are below it
+int kernel_plan(int log_n, int form, int plan, int count);
+// Ocean slots of `inter` that launches of up to `count` oceans with
+// q.slots <= slots use, whatever the plan.
+int frame_ring_slots(int log_n, int form, int slots, int count);
+// The register-resident persistent frame, as frame_blocks_per_sm and
+// launch_frame call it for kPairPlan.
+bool pair_frame_ok(int log_n, int count);
+int pair_frame_ring(int slots);
+int pair_frame_blocks_per_sm(int log_n, int nf, int ar, bool fuse_foam);
+cudaError_t launch_pair_frame(int log_n, int nf, int ar, bool fuse_foam, const FrameArgs& args, const QueueArgs& q,
+                              int grid, cudaStream_t stream);
 // Bounded waits that nothing completes (tests the timeout paths): on
 // `counter`, which nothing increments, setting *error, and on an mbarrier
 // nothing arrives at, setting *bar_error.
