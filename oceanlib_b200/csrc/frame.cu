@@ -1328,13 +1328,31 @@ int frame_plan_count(int log_n, int form)
 
 int kernel_plan(int log_n, int form, int plan, int count)
 {
-    return plan == 0 && form != 2 && pair_frame_ok(log_n, count) ? kPairPlan : plan;
+    return plan == 0 && form != 2 && pair_frame_ok(log_n, arith_of_form(form), count) ? kPairPlan : plan;
 }
 
 int frame_ring_slots(int log_n, int form, int slots, int count)
 {
-    const int ring = kernel_plan(log_n, form, 0, count) == kPairPlan ? pair_frame_ring(slots) : slots;
+    int ring = slots;
+    if (kernel_plan(log_n, form, 0, count) == kPairPlan) {
+        const int r = pair_frame_ring(log_n, arith_of_form(form), slots);
+        ring = ring > r ? ring : r;
+    }
     return ring < count ? ring : count;
+}
+
+int frame_grid(int log_n, int nf, int form, bool fuse_foam, int plan, int count, int wave, int sms)
+{
+    long tasks;  // row tasks of the frame, and as many column tasks
+    if (plan == kPairPlan) {
+        tasks = static_cast<long>(count) * pair_frame_tasks(log_n, arith_of_form(form), fuse_foam);
+    } else {
+        if (plan < 0 || plan >= frame_plan_count(log_n, form)) return 0;
+        tasks = static_cast<long>(count) *
+                frame_dispatch(log_n, nf, form, fuse_foam, plan, [](auto L) { return decltype(L)::P::RT; });
+    }
+    const long even = (tasks + sms - 1) / sms * sms;
+    return static_cast<int>(even < wave ? even : wave);
 }
 
 int frame_blocks_per_sm(int log_n, int nf, int form, bool fuse_foam, int plan)

@@ -68,7 +68,7 @@ struct Large {
     static constexpr int THREADS = 2 * G;           // two rows (columns) per task
     static constexpr int CTAS = 512 / THREADS;      // resident per SM: 128 registers a thread
     static constexpr int TASKS = N / 2;             // per ocean and pass
-    static constexpr int SEQ = seq_stride_bytes(N, 16, 2, false) / 8;  // exchange stride (f32x2)
+    static constexpr int SEQ = seq_stride_bytes(N, 16, 2) / 8;  // exchange stride (f32x2)
     static constexpr int HELD = 15;                 // of a thread's 16 cells, those the column stash holds
     static constexpr int BUF = 2 * SEQ;
     static constexpr size_t EXCHANGE = sizeof(f32x2) * BUF;
@@ -114,7 +114,7 @@ template <int LOG_N, int NF, int AR>
 __global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) large_row_kernel(FrameArgs a)
 {
     using S = Large<LOG_N>;
-    using Fft = RegFft<LOG_N, 16, AR, false>;
+    using Fft = RegFft<LOG_N, 16, AR>;
     constexpr int N = S::N, G = S::G, Q = NF / 2, NT = S::THREADS;
     extern __shared__ float4 smem4[];
     const int tid = threadIdx.x;
@@ -223,7 +223,7 @@ template <int LOG_N, int NF, int AR>
 __global__ void __launch_bounds__(Large<LOG_N>::THREADS, Large<LOG_N>::CTAS) large_col_kernel(FrameArgs a)
 {
     using S = Large<LOG_N>;
-    using Fft = RegFft<LOG_N, 16, AR, false>;
+    using Fft = RegFft<LOG_N, 16, AR>;
     constexpr int N = S::N, Q = NF / 2, NT = S::THREADS;
     constexpr unsigned kPairBytes = 2u * N * sizeof(float4);  // a task's pair
     extern __shared__ float4 smem4[];

@@ -1,7 +1,7 @@
 // oceanlib-b200: the persistent frame with its transforms in registers.
 //
 // The same frame, queue protocol and arithmetic as frame_kernel (frame.cu), for
-// the sizes where it is the faster one (pair_frame_ok). There, a task's every
+// the batches where it is the faster one (pair_frame_ok). There, a task's every
 // field sat in shared memory and each step of the frame - evolve, three stage
 // blocks, the store - read and wrote all of it: the shared-memory pipe was the
 // frame's busiest unit (71% of 64 x 512^2 with velocity and foam). Here a task
@@ -24,15 +24,16 @@
 // a.im, b.im) a cell and pair: a warp reads it in whole 512-byte runs, writes it
 // in runs of ROWS^2 x 16 bytes and writes the outputs in runs of ROWS x 16.
 //
-// A CTA has T = 256 threads and three are resident, so three times as many rows
-// are in flight as with a task's pairs side by side. So that a column task does
-// not wait for rows still in flight, the queue runs the rows `ahead` oceans
-// before the columns, R(0) .. R(ahead - 1) | R(ahead) C(0) | R(ahead + 1) C(1) |
-// .. | C(count - 1), through a ring of `ring` slots: 4 and 8 at three ring slots
-// of the batch's own count, 2 and 5 at two. Every awaited task holds an earlier
-// ticket, as in frame_kernel, since the ring has more slots than rows run ahead.
-// 64 x 512^2 with velocity, us a frame by (ahead, ring): (2, 4) 983, (2, 5) 810,
-// (3, 6) 740, (3, 7) 715, (4, 8) 672, (5, 10) 664.
+// A resident wave of CTAs holds several oceans' worth of tasks (3.5 at 512^2, 222
+// at 64^2). So that a column task does not wait for rows still in flight, nor a
+// row task for its ring slot, the queue runs the rows `ahead` oceans before the
+// columns, R(0) .. R(ahead - 1) | R(ahead) C(0) | R(ahead + 1) C(1) | .. |
+// C(count - 1), with ahead = that many oceans and a ring of twice as many slots.
+// (frame_kernel's ring of three keeps a large batch of small oceans to a few
+// CTAs.) Every awaited task holds an earlier ticket, as in frame_kernel, since
+// the ring has more slots than rows run ahead. 64 x 512^2 with velocity, us a
+// frame by (ahead, ring): (2, 4) 983, (2, 5) 810, (3, 6) 740, (3, 7) 715,
+// (4, 8) 672, (5, 10) 664.
 #include "frame_cells.cuh"
 #include "ocean_device.cuh"
 #include "queue_device.cuh"
@@ -49,23 +50,41 @@ struct RegPlan {
     static constexpr int LOG_N = LOG_N_, N = 1 << LOG_N, E = E_, ROWS = ROWS_;
     static constexpr int G = N / E;             // lanes per pair
     static constexpr int T = ROWS * G;          // threads
-    static constexpr int CTAS = 768 / T;        // resident per SM: 80 registers a thread
+    static constexpr int CTAS = (E == 16 ? 512 : 768) / T;  // resident per SM: 128 or 80 registers a thread
     static constexpr int TASKS = N / ROWS;      // per ocean, rows and columns alike
-    static constexpr int SEQ = seq_stride_bytes(N, E, ROWS, false);
+    static constexpr int SEQ = seq_stride_bytes(N, E, ROWS);
     // Shared memory, in bytes from the start: exchange buffers, twiddles, the
     // threads' own values (16 bytes a cell in a column task).
     static constexpr size_t TW = ROWS * SEQ;
     static constexpr size_t HELD = TW + sizeof(float2) * N;
     static constexpr size_t SMEM = HELD + sizeof(float4) * E * T;
+    // Oceans that the rows run ahead of the columns and slots of the ring, at
+    // q.slots = slots (see above).
+    static constexpr int WAVE = (148 * CTAS + TASKS - 1) / TASKS;  // oceans' worth of tasks on the GPU
+    static constexpr int IN_FLIGHT = WAVE > 2 ? WAVE : 2;
+    __host__ __device__ static constexpr unsigned ahead(unsigned slots)
+    {
+        return slots >= 3 ? IN_FLIGHT : (IN_FLIGHT + 1) / 2;
+    }
+    __host__ __device__ static constexpr unsigned ring(unsigned slots) { return 2 * ahead(slots) + (slots >= 3 ? 0 : 1); }
     static_assert(E * T == ROWS * N && TW % 16 == 0 && HELD % 16 == 0, "a thread holds E cells");
     static_assert(CTAS * (SMEM + 1280) <= 228 * 1024, "the resident CTAs fit on an SM");
 };
-template <int LOG_N>
-using PairPlan = RegPlan<LOG_N, 8, 4>;
-
-// Ring slots of a launch with q.slots = slots (see above).
-__host__ __device__ constexpr unsigned ring_of(unsigned slots) { return 3u * slots - 1u; }
-static_assert(ring_of(3) > 4 && ring_of(2) > 2 && ring_of(1) > 1, "more slots than rows run ahead");
+// Eight indices a lane (80 registers); a task takes as many rows as 128 threads
+// hold, but at least two (1024^2), and four with foam at 512^2: two columns' foam
+// is 8 bytes a row (64 oceans: 829 us against 745; without foam four rows cost
+// 670 against 651). The precise form rounds where a stage block ends, so it
+// keeps the blocks it always had: 3 + 3 + .. stages at N = 32, 64 and 512, 4 + 3
+// and 4 + 4 (16 indices a lane) at 128 and 256, and at 1024, whose blocks of
+// five would take 32 indices a lane, and 16, one block of four, frame_kernel.
+template <int LOG_N, int AR, bool FOAM>
+struct PairPlanOf {
+    static constexpr int E = AR == kArPrecise && (LOG_N == 7 || LOG_N == 8) ? 16 : 8;
+    static constexpr int T = LOG_N == 4 ? 32 : (LOG_N == 10 || (LOG_N == 9 && FOAM) ? 256 : 128);
+    using type = RegPlan<LOG_N, E, T * E / (1 << LOG_N)>;
+};
+template <int LOG_N, int AR, bool FOAM>
+using PairPlan = typename PairPlanOf<LOG_N, AR, FOAM>::type;
 
 // Adds this CTA's finished row task (pub[0]) or its own column task (pub[1]).
 __device__ __forceinline__ void publish(unsigned* counter, int tid)
@@ -77,7 +96,7 @@ template <class P, int NF, int AR>
 __device__ __forceinline__ void pair_row_task(const FrameArgs& a, int ocean, int task, float2* inter_slot,
                                               unsigned char* smem, int tid, unsigned* const* pub)
 {
-    using Fft = RegFft<P::LOG_N, P::E, AR, false>;
+    using Fft = RegFft<P::LOG_N, P::E, AR>;
     constexpr int N = P::N, G = P::G, E = P::E, ROWS = P::ROWS, T = P::T, Q = NF / 2;
     const int r = tid % ROWS, c = tid / ROWS;
     void* buf = smem + r * P::SEQ;
@@ -165,7 +184,7 @@ template <class P, int NF, int AR, bool FOAM>
 __device__ __forceinline__ void pair_col_task(const FrameArgs& a, int ocean, int strip, const float2* inter_slot,
                                               unsigned char* smem, int tid, unsigned* const* pub)
 {
-    using Fft = RegFft<P::LOG_N, P::E, AR, false>;
+    using Fft = RegFft<P::LOG_N, P::E, AR>;
     constexpr int N = P::N, E = P::E, ROWS = P::ROWS, T = P::T, Q = NF / 2;
     const int w = tid % ROWS, c = tid / ROWS;
     void* buf = smem + w * P::SEQ;
@@ -247,10 +266,9 @@ __device__ __forceinline__ void pair_col_task(const FrameArgs& a, int ocean, int
     }
 }
 
-template <int LOG_N, int NF, int AR, bool FOAM>
-__global__ void __launch_bounds__(PairPlan<LOG_N>::T, PairPlan<LOG_N>::CTAS) pair_frame_kernel(FrameArgs a, QueueArgs q)
+template <class P, int NF, int AR, bool FOAM>
+__global__ void __launch_bounds__(P::T, P::CTAS) pair_frame_kernel(FrameArgs a, QueueArgs q)
 {
-    using P = PairPlan<LOG_N>;
     constexpr int N = P::N;
     constexpr unsigned TASKS = P::TASKS;
     extern __shared__ float4 smem4[];
@@ -270,8 +288,8 @@ __global__ void __launch_bounds__(PairPlan<LOG_N>::T, PairPlan<LOG_N>::CTAS) pai
 
     const unsigned count = static_cast<unsigned>(q.count);
     const unsigned slots = static_cast<unsigned>(q.slots);
-    const unsigned ring = min(ring_of(slots), count);
-    const unsigned ahead = min(max(2u * slots, 3u) - 2u, count);
+    const unsigned ring = min(P::ring(slots), count);
+    const unsigned ahead = min(P::ahead(slots), count);
     const unsigned total = 2u * count * TASKS;
     // Ticket -> (row?, ocean, task index) for the queue order above.
     auto decode = [&](unsigned t, bool& row, unsigned& ocean, unsigned& idx) {
@@ -348,19 +366,19 @@ __global__ void __launch_bounds__(PairPlan<LOG_N>::T, PairPlan<LOG_N>::CTAS) pai
 
 template <int LOG_N, int NF, int AR, bool FOAM>
 struct PairLaunch {
-    using P = PairPlan<LOG_N>;
+    using P = PairPlan<LOG_N, AR, FOAM>;
     static constexpr size_t SMEM = P::SMEM;
 
     static cudaError_t prepare()
     {
-        return cudaFuncSetAttribute(pair_frame_kernel<LOG_N, NF, AR, FOAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        return cudaFuncSetAttribute(pair_frame_kernel<P, NF, AR, FOAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(SMEM));
     }
     static int blocks_per_sm()
     {
         int n = 0;
         if (prepare() != cudaSuccess) return 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pair_frame_kernel<LOG_N, NF, AR, FOAM>, P::T, SMEM) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pair_frame_kernel<P, NF, AR, FOAM>, P::T, SMEM) !=
             cudaSuccess)
             return 0;
         return n;
@@ -369,7 +387,7 @@ struct PairLaunch {
     {
         cudaError_t e = prepare();
         if (e != cudaSuccess) return e;
-        pair_frame_kernel<LOG_N, NF, AR, FOAM><<<grid, P::T, SMEM, st>>>(a, q);
+        pair_frame_kernel<P, NF, AR, FOAM><<<grid, P::T, SMEM, st>>>(a, q);
         return cudaGetLastError();
     }
 };
@@ -385,32 +403,87 @@ auto variant_ar(int nf, bool foam, Fn&& fn)
 template <int LOG_N, typename Fn>
 auto variant(int nf, int ar, bool foam, Fn&& fn)
 {
+    if constexpr (LOG_N != 4 && LOG_N != 10) {
+        if (ar == kArPrecise) return variant_ar<LOG_N, kArPrecise>(nf, foam, fn);
+    }
     if (ar == kArFast) return variant_ar<LOG_N, kArFast>(nf, foam, fn);
-    if (ar == kArPrecise) return variant_ar<LOG_N, kArPrecise>(nf, foam, fn);
     return variant_ar<LOG_N, kArExact>(nf, foam, fn);
+}
+template <typename Fn>
+auto dispatch(int log_n, int nf, int ar, bool foam, Fn&& fn)
+{
+    switch (log_n) {
+        case 4: return variant<4>(nf, ar, foam, fn);
+        case 5: return variant<5>(nf, ar, foam, fn);
+        case 6: return variant<6>(nf, ar, foam, fn);
+        case 7: return variant<7>(nf, ar, foam, fn);
+        case 8: return variant<8>(nf, ar, foam, fn);
+        case 9: return variant<9>(nf, ar, foam, fn);
+        default: return variant<10>(nf, ar, foam, fn);
+    }
+}
+
+// Whether the size has a plan in this arithmetic.
+bool has_plan(int log_n, int ar)
+{
+    return log_n >= 4 && log_n <= 10 && (ar != kArPrecise || (log_n != 4 && log_n != 10));
 }
 
 }  // namespace
 
 // A task takes its pairs one after the other, so a frame of few oceans, whose
 // tasks do not fill the GPU, is a longer chain here than with a task's pairs side
-// by side (frame_kernel): 512^2 with velocity, us a frame here / there: one ocean
-// 43.0 / 27.2, two 43.2 / 41.0, three 43.1 / 54.5.
-bool pair_frame_ok(int log_n, int count) { return log_n == 9 && count >= 3; }
+// by side (frame_kernel). From the fourth ocean on that kernel waits for the three
+// slots of its ring; at 512^2 and above a frame fills the GPU sooner. us a frame
+// there / here, with velocity unless "-":
+//   N = 16   4 oceans 14.4 / 12.4, 64- 112 / 12, 4096- 6843 / 50
+//   N = 32   2 14.4 / 15.8, 4- 19.5 / 13.4, 2048- 5119 / 82
+//   N = 64   2 13.4 / 16.2, 3- 11.3 / 13.4, 4 21.3 / 16.5, 1024- 2625 / 143
+//   N = 128  3- 12.8 / 14.4, 4 24.6 / 18.5, 256- 1019 / 140
+//   N = 256  2 14.4 / 18.5, 3 20.5 / 20.8, 4 30.9 / 20.8, 64 414 / 165
+//   N = 512  1 22.6 / 22.6, 2 36.2 / 32.8, 64 854 / 651
+//   N = 1024 1- 61 / 57, 2- 111 / 78, 16 1137 / 793
+// The precise form's blocks of 16 indices (N = 128 and 256) leave four CTAs of 128
+// threads on an SM, and its chain is longest:
+//   N = 128  4 28.7 / 45, 8 40.2 / 47.0, 64 335 / 104
+//   N = 256  6 55.5 / 62.2, 10- 68.2 / 57.6, 21 168 / 141
+bool pair_frame_ok(int log_n, int ar, int count)
+{
+    if (!has_plan(log_n, ar)) return false;
+    if (ar == kArPrecise && log_n == 7) return count >= 12;
+    if (ar == kArPrecise && log_n == 8) return count >= 8;
+    return count >= (log_n >= 10 ? 1 : log_n == 9 ? 2 : 4);
+}
 
-int pair_frame_ring(int slots) { return static_cast<int>(ring_of(static_cast<unsigned>(slots))); }
+int pair_frame_ring(int log_n, int ar, int slots)
+{
+    if (!has_plan(log_n, ar)) return 0;
+    const unsigned s = static_cast<unsigned>(slots);
+    int ring = 0;
+    for (bool foam : {false, true}) {
+        const int r = dispatch(log_n, 6, ar, foam, [&](auto L) { return static_cast<int>(decltype(L)::P::ring(s)); });
+        ring = ring > r ? ring : r;
+    }
+    return ring;
+}
+
+int pair_frame_tasks(int log_n, int ar, bool fuse_foam)
+{
+    if (!has_plan(log_n, ar)) return 0;
+    return dispatch(log_n, fuse_foam ? 6 : 4, ar, fuse_foam, [](auto L) { return decltype(L)::P::TASKS; });
+}
 
 int pair_frame_blocks_per_sm(int log_n, int nf, int ar, bool fuse_foam)
 {
-    if (log_n != 9) return 0;
-    return variant<9>(nf, ar, fuse_foam, [](auto L) { return decltype(L)::blocks_per_sm(); });
+    if (!has_plan(log_n, ar)) return 0;
+    return dispatch(log_n, nf, ar, fuse_foam, [](auto L) { return decltype(L)::blocks_per_sm(); });
 }
 
 cudaError_t launch_pair_frame(int log_n, int nf, int ar, bool fuse_foam, const FrameArgs& a, const QueueArgs& q, int grid,
                               cudaStream_t st)
 {
-    if (log_n != 9) return cudaErrorInvalidValue;
-    return variant<9>(nf, ar, fuse_foam, [&](auto L) { return decltype(L)::launch(a, q, grid, st); });
+    if (!has_plan(log_n, ar)) return cudaErrorInvalidValue;
+    return dispatch(log_n, nf, ar, fuse_foam, [&](auto L) { return decltype(L)::launch(a, q, grid, st); });
 }
 
 }  // namespace ocean_b200

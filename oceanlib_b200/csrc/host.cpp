@@ -664,11 +664,11 @@ private:
         q.wait_ns = 1000000000ull;
         q.defer = defer_ ? 1 : 0;
         const int plan = kernel_plan(log_n_, form_, plan_, static_cast<int>(k));
-        const int grid = frame_grid(plan, foam);
+        const int wave = frame_wave(plan, foam);
+        const int grid = frame_grid(log_n_, nf_, form_, foam, plan, static_cast<int>(k), wave, sms_);
         // A share below 1 leaves SMs to batches of other sizes running
         // concurrently (the ensemble's schedule).
-        const int shared = std::max(1, static_cast<int>(std::lround(grid * grid_share_)));
-        const int launch_grid = static_cast<int>(std::min<uint64_t>(shared, uint64_t(k) * n_));
+        const int launch_grid = std::min(grid, std::max(1, static_cast<int>(std::lround(wave * grid_share_))));
         timed(3, st, [&] {
             check(launch_frame(log_n_, nf_, form_, foam, a, q, launch_grid, st, plan),
                   "frame kernel");
@@ -688,15 +688,14 @@ private:
     static constexpr double kInvTwoPi = 0.159154943091895335769;
 
     // One wave of resident CTAs of a kernel plan (computed once).
-    int frame_grid(int plan, bool foam)
+    int frame_wave(int plan, bool foam)
     {
-        int& grid = frame_grid_[plan][foam ? 1 : 0];
+        int& grid = frame_wave_[plan][foam ? 1 : 0];
         if (grid == 0) {
-            int sms = 0;
-            check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "SM count");
+            check(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "SM count");
             const int per_sm = frame_blocks_per_sm(log_n_, nf_, form_, foam, plan);
             if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "frame occupancy");
-            grid = per_sm * sms;
+            grid = per_sm * sms_;
         }
         return grid;
     }
@@ -843,7 +842,7 @@ public:
     // Settles the launch shapes, so a capture issues launches only.
     void prime_shapes()
     {
-        if (persistent_) (void)frame_grid(kernel_plan(log_n_, form_, plan_, static_cast<int>(count_)), false);
+        if (persistent_) (void)frame_wave(kernel_plan(log_n_, form_, plan_, static_cast<int>(count_)), false);
     }
 
 private:
@@ -975,7 +974,8 @@ private:
     int slots_ = 1;      // intermediate ring slots the persistent kernel uses
     int max_slots_ = 1;  // slots the ring buffer holds
     bool defer_ = false; // QueueArgs::defer of the persistent kernel
-    int frame_grid_[kMaxFramePlans][2] = {};  // [plan][foam]: CTAs of one wave
+    int frame_wave_[kMaxFramePlans][2] = {};  // [kernel plan][foam]: CTAs of one wave
+    int sms_ = 0;
     int plan_ = 0;  // the persistent kernel's task plan (frame_plan_count)
     double grid_share_ = 1.0;
     FrameQueue queue_;

@@ -493,22 +493,24 @@ __device__ __forceinline__ void fft_pair(ulonglong2* seq, const float2* tw, int 
 // Sequence pairs that stay in registers: the transform of a pair over G = N / E
 // lanes, lane c holding the E indices c + j G in slots j (real parts f32x2 in
 // re, imaginary parts in im). The blocks' butterflies are PairBlock's; between
-// two blocks the values pass through `buf`, which the lanes of one CTA share
-// (CTA barriers: every thread of the CTA runs the same transforms, each pair
-// its own buf). WHOLE: 16 bytes an index, two barriers an exchange; else 8
-// bytes - the real parts, then the imaginary parts - and four. Afterwards slot
-// j holds index(j, c). One element of padding after every E keeps a block's
-// stores and loads free of bank conflicts when neighbouring threads are the
-// same lane of neighbouring pairs and the pairs' buffers lie STRIDE bytes apart.
+// two blocks the values pass through `buf`, 8 bytes an index - the real parts,
+// then the imaginary parts - which the lanes of one CTA share (CTA barriers:
+// every thread of the CTA runs the same transforms, each pair its own buf).
+// (16 bytes an index would halve the barriers but double the shared memory: at
+// 512^2 three CTAs of 74 KB left the L1 nothing and the frame took 743 us
+// instead of 672.) Afterwards slot j holds index(j, c). One f32x2 of padding
+// after every E keeps a block's stores and loads free of bank conflicts when
+// neighbouring threads are the same lane of neighbouring pairs and the pairs'
+// buffers lie seq_stride_bytes apart.
 // ---------------------------------------------------------------------------
-// Bytes from one pair's buffer to the next of `pairs` (a power of two up to 8):
-// the lanes of each pair that one wavefront serves fall into different banks.
-__host__ __device__ constexpr int seq_stride_bytes(int n, int e, int pairs, bool whole)
+// Bytes from one pair's buffer to the next of `pairs` (a power of two): the
+// lanes of each pair that one wavefront serves fall into different banks.
+__host__ __device__ constexpr int seq_stride_bytes(int n, int e, int pairs)
 {
-    return whole ? ((n + n / e + 7) / 8 * 8 + 8 / pairs) * 16 : ((n + n / e + 15) / 16 * 16 + 16 / pairs) * 8;
+    return ((n + n / e + 15) / 16 * 16 + (pairs >= 16 ? 1 : 16 / pairs)) * 8;
 }
 
-template <int LOG_N, int E, int AR, bool WHOLE>
+template <int LOG_N, int E, int AR>
 struct RegFft {
     static constexpr int N = 1 << LOG_N;
     static constexpr int G = N / E;
@@ -534,23 +536,8 @@ struct RegFft {
     template <class From, class To>
     __device__ __forceinline__ static void exchange(f32x2 (&re)[E], f32x2 (&im)[E], void* buf, int c)
     {
-        if constexpr (!WHOLE) {
-            exchange_part<From, To>(re, buf, c);
-            exchange_part<From, To>(im, buf, c);
-        } else {
-            ulonglong2* p = static_cast<ulonglong2*>(buf);
-            __syncthreads();
-#pragma unroll
-            for (int j = 0; j < E; ++j)
-                p[pad(From::index_after(j / From::RR, j % From::RR, c))] = make_ulonglong2(re[j], im[j]);
-            __syncthreads();
-#pragma unroll
-            for (int j = 0; j < E; ++j) {
-                const ulonglong2 v = p[pad(To::index_before(j / To::RR, j % To::RR, c))];
-                re[j] = v.x;
-                im[j] = v.y;
-            }
-        }
+        exchange_part<From, To>(re, buf, c);
+        exchange_part<From, To>(im, buf, c);
     }
     template <class From, class To>
     __device__ __forceinline__ static void exchange(float (&x)[E], float (&y)[E], void* buf, int c)

@@ -154,8 +154,12 @@ struct OceanKind {
     uint32_t n = 0;
     bool velocity = false;
     int log_n = 0, nf = 4;
-    int grid[kMaxFramePlans] = {};  // CTAs of one wave by kernel plan
+    int wave[kMaxFramePlans] = {};  // CTAs of one wave by kernel plan
     DevBuf<float2> tw, inter;
+    // A larger ring for batches of many sessions of one kind (pool allocation,
+    // counted as staging), and its oceans.
+    float2* deep = nullptr;
+    size_t deep_slots = 0;
     FrameQueue queue;
     size_t queue_cap = 0;
     size_t bytes = 0;
@@ -282,6 +286,8 @@ public:
         cudaStreamSynchronize(stream_);
         for (auto& kv : sessions_)
             if (kv.second->block) cudaFreeAsync(kv.second->block, stream_);
+        for (auto& k : ocean_kinds_)
+            if (k->deep) cudaFreeAsync(k->deep, stream_);
         for (auto& c : ctxs_) {
             if (c->dev) cudaFreeAsync(c->dev, stream_);
             if (c->start) cudaEventDestroy(c->start);
@@ -521,18 +527,12 @@ private:
         return field_kinds_.back().get();
     }
 
-    // Oceans that the frame kernels of a kind hold in its intermediate ring.
-    size_t ring_oceans(const ocean_desc& od) const
-    {
-        return static_cast<size_t>(std::max(3, frame_ring_slots(ilog2u(od.size), desc_.fft_form, 3, 64)));
-    }
-
     // Bytes a new ocean / field kind would add (shared tables).
     size_t ocean_kind_bytes(const ocean_desc& od) const
     {
         const size_t cells = static_cast<size_t>(od.size) * od.size;
         const int nf = od.compute_velocity ? 6 : 4;
-        return round_up((od.size - 1) * sizeof(float2), kAlign) + round_up(ring_oceans(od) * cells * nf * sizeof(float2), kAlign);
+        return round_up((od.size - 1) * sizeof(float2), kAlign) + round_up(3 * cells * nf * sizeof(float2), kAlign);
     }
 
     OceanKind* find_ocean_kind(const ocean_desc& od)
@@ -552,7 +552,7 @@ private:
         k->nf = k->velocity ? 6 : 4;
         const size_t cells = static_cast<size_t>(k->n) * k->n;
         k->tw = DevBuf<float2>(k->n - 1);
-        k->inter = DevBuf<float2>(ring_oceans(od) * cells * k->nf);
+        k->inter = DevBuf<float2>(3 * cells * k->nf);
         ensure_queue(k.get(), 1024);  // sessions updating in one batch before the words have to grow
         const std::vector<float2> tw = stage_twiddles(k->n);
         check(cudaMemcpyAsync(k->tw.p, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, stream_),
@@ -561,7 +561,7 @@ private:
         for (int plan : {kernel_plan(k->log_n, desc_.fft_form, 0, 1), kernel_plan(k->log_n, desc_.fft_form, 0, 64)}) {
             const int per_sm = frame_blocks_per_sm(k->log_n, k->nf, desc_.fft_form, false, plan);
             if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "frame occupancy");
-            k->grid[plan] = per_sm * sms_;
+            k->wave[plan] = per_sm * sms_;
         }
         k->bytes = ocean_kind_bytes(od);
         check(cudaStreamSynchronize(stream_), "twiddles");
@@ -798,6 +798,23 @@ private:
         }
     }
 
+    // The intermediate for a batch of `count` oceans that uses `slots` of them.
+    float2* ring_for(OceanKind* k, size_t slots)
+    {
+        if (slots <= 3) return k->inter.p;
+        if (slots > k->deep_slots) {
+            const size_t ocean = static_cast<size_t>(k->n) * k->n * k->nf * sizeof(float2);
+            const size_t grown = std::max(slots, 2 * k->deep_slots);
+            if (k->deep) check(cudaFreeAsync(k->deep, stream_), "free ring");
+            k->deep = nullptr;
+            check(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&k->deep), grown * ocean, pool_, stream_), "ring");
+            std::lock_guard<std::mutex> lk(mu_);
+            staging_bytes_ += (grown - k->deep_slots) * ocean;
+            k->deep_slots = grown;
+        }
+        return k->deep;
+    }
+
     void ensure_queue(OceanKind* k, size_t count)
     {
         if (count <= k->queue_cap) return;
@@ -960,7 +977,8 @@ private:
             q.wait_ns = 1000000000ull;
             q.defer = k->nf == 6 ? 1 : 0;
             const int plan = kernel_plan(k->log_n, desc_.fft_form, 0, count);
-            const int grid = static_cast<int>(std::min<uint64_t>(k->grid[plan], uint64_t(count) * k->n));
+            a.inter = ring_for(k, static_cast<size_t>(frame_ring_slots(k->log_n, desc_.fft_form, q.slots, count)));
+            const int grid = frame_grid(k->log_n, k->nf, desc_.fft_form, false, plan, count, k->wave[plan], sms_);
             check(launch_frame(k->log_n, k->nf, desc_.fft_form, false, a, q, grid, stream_, plan), "frame kernel");
             k->queue.launched(set);
             ++kernels;

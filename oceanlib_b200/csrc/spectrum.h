@@ -115,10 +115,16 @@ int kernel_plan(int log_n, int form, int plan, int count);
 // Ocean slots of `inter` that launches of up to `count` oceans with
 // q.slots <= slots use, whatever the plan.
 int frame_ring_slots(int log_n, int form, int slots, int count);
-// The register-resident persistent frame, as frame_blocks_per_sm and
-// launch_frame call it for kPairPlan.
-bool pair_frame_ok(int log_n, int count);
-int pair_frame_ring(int slots);
+// CTAs to launch a frame of `count` oceans with, of the `wave` that are resident
+// on `sms` SMs: no more per SM than it takes to hand every SM its even share of
+// the row tasks. (All CTAs of a wave draw their tickets at once, so with more of
+// them a few SMs would take several row tasks each while others spin.)
+int frame_grid(int log_n, int nf, int form, bool fuse_foam, int plan, int count, int wave, int sms);
+// The register-resident persistent frame, as frame_blocks_per_sm, frame_grid
+// and launch_frame call it for kPairPlan.
+bool pair_frame_ok(int log_n, int ar, int count);
+int pair_frame_ring(int log_n, int ar, int slots);
+int pair_frame_tasks(int log_n, int ar, bool fuse_foam);  // row tasks of an ocean
 int pair_frame_blocks_per_sm(int log_n, int nf, int ar, bool fuse_foam);
 cudaError_t launch_pair_frame(int log_n, int nf, int ar, bool fuse_foam, const FrameArgs& args, const QueueArgs& q,
                               int grid, cudaStream_t stream);
