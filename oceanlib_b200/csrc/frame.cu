@@ -1381,27 +1381,45 @@ cudaError_t launch_frame(int log_n, int nf, int form, bool fuse_foam, const Fram
 
 bool mixed_size_ok(int log_n) { return log_n >= kMixMinLog && log_n <= kMixMaxLog; }
 
-uint32_t mixed_tasks(int log_n, int count)
+bool mixed_pairs(int ar, const MixedArgs& m)
 {
-    unsigned rt = 0, ct = 0;
-    mix_tasks_per_ocean(log_n, rt, ct);
-    return static_cast<uint32_t>(count) * (rt + ct);
+    uint64_t rows = 0;
+    for (int g = 0; g < m.groups; ++g) {
+        if (!pair_mixed_ok(m.g[g].log_n, ar)) return false;
+        rows += uint64_t(m.g[g].count) * pair_mixed_tasks(m.g[g].log_n);
+    }
+    return rows >= 148;
 }
 
-int mixed_blocks_per_sm(int nf, int ar)
+int mixed_blocks_per_sm(int nf, int ar, const MixedArgs& m)
 {
+    if (mixed_pairs(ar, m)) return pair_mixed_blocks_per_sm(nf, ar);
     return with_arith(ar, [&](auto A) {
         constexpr int AR = decltype(A)::value;
         return nf == 4 ? MixedLaunch<4, AR>::blocks_per_sm() : MixedLaunch<6, AR>::blocks_per_sm();
     });
 }
 
-cudaError_t launch_mixed_frame(int nf, int ar, const MixedArgs& m, int grid, cudaStream_t st)
+cudaError_t launch_mixed_frame(int nf, int ar, const MixedArgs& args, int wave, cudaStream_t st)
 {
+    MixedArgs m = args;
     if (m.groups < 1 || m.groups > kMaxMixedGroups) return cudaErrorInvalidValue;
     for (int g = 0; g < m.groups; ++g)
-        if (!mixed_size_ok(m.g[g].log_n) || m.g[g].count < 1 || m.g[g].slots < 1)
+        if (!mixed_size_ok(m.g[g].log_n) || m.g[g].count < 1 || m.g[g].slots < 1 || m.g[g].ring < 1)
             return cudaErrorInvalidValue;
+    if (mixed_pairs(ar, m)) {
+        uint64_t rows = 0;
+        for (int g = 0; g < m.groups; ++g) rows += uint64_t(m.g[g].count) * pair_mixed_tasks(m.g[g].log_n);
+        return launch_pair_mixed(nf, ar, m, static_cast<int>(rows < static_cast<uint64_t>(wave) ? rows : wave), st);
+    }
+    m.total = 0;
+    for (int g = 0; g < m.groups; ++g) {
+        unsigned rt = 0, ct = 0;
+        mix_tasks_per_ocean(m.g[g].log_n, rt, ct);
+        m.g[g].first = m.total;
+        m.total += static_cast<uint32_t>(m.g[g].count) * (rt + ct);
+    }
+    const int grid = m.total < static_cast<uint32_t>(wave) ? static_cast<int>(m.total) : wave;
     return with_arith(ar, [&](auto A) {
         constexpr int AR = decltype(A)::value;
         return nf == 4 ? MixedLaunch<4, AR>::launch(m, grid, st) : MixedLaunch<6, AR>::launch(m, grid, st);

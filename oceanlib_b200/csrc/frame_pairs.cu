@@ -86,6 +86,14 @@ struct PairPlanOf {
 template <int LOG_N, int AR, bool FOAM>
 using PairPlan = typename PairPlanOf<LOG_N, AR, FOAM>::type;
 
+// A task's areas of shared memory: exchange buffers, the size's twiddles, the
+// threads' own values (16 bytes a cell in a column task).
+struct Shared {
+    unsigned char* exchange;
+    const float2* tw;
+    unsigned char* held;
+};
+
 // Adds this CTA's finished row task (pub[0]) or its own column task (pub[1]).
 __device__ __forceinline__ void publish(unsigned* counter, int tid)
 {
@@ -94,15 +102,14 @@ __device__ __forceinline__ void publish(unsigned* counter, int tid)
 
 template <class P, int NF, int AR>
 __device__ __forceinline__ void pair_row_task(const FrameArgs& a, int ocean, int task, float2* inter_slot,
-                                              unsigned char* smem, int tid, unsigned* const* pub)
+                                              const Shared& sh, int tid, unsigned* const* pub)
 {
     using Fft = RegFft<P::LOG_N, P::E, AR>;
     constexpr int N = P::N, G = P::G, E = P::E, ROWS = P::ROWS, T = P::T, Q = NF / 2;
     const int r = tid % ROWS, c = tid / ROWS;
-    void* buf = smem + r * P::SEQ;
-    const float2* tws = reinterpret_cast<const float2*>(smem + P::TW);
-    float2* held_h = reinterpret_cast<float2*>(smem + P::HELD) + tid;                         // (hr, hi) of cell j at [j * T]
-    float* held_k = reinterpret_cast<float*>(smem + P::HELD + sizeof(float2) * E * T) + tid;  // its 1/|k|
+    void* buf = sh.exchange + r * P::SEQ;
+    float2* held_h = reinterpret_cast<float2*>(sh.held) + tid;                         // (hr, hi) of cell j at [j * T]
+    float* held_k = reinterpret_cast<float*>(sh.held + sizeof(float2) * E * T) + tid;  // its 1/|k|
 
     // Rows and the rows with their mirrors are neighbouring tasks: the second
     // read of h0 finds it in the L2.
@@ -170,7 +177,7 @@ __device__ __forceinline__ void pair_row_task(const FrameArgs& a, int ocean, int
                 im[j] = px_pack(pa.y, pb.y);
             }
         }
-        Fft::run(re, im, buf, tws, c);
+        Fft::run(re, im, buf, sh.tw, c);
         if (k == 0) publish(pub[0], tid);  // the CTA's previous row task, whose stores have drained by now
 #pragma unroll
         for (int j = 0; j < E; ++j) {
@@ -182,15 +189,14 @@ __device__ __forceinline__ void pair_row_task(const FrameArgs& a, int ocean, int
 
 template <class P, int NF, int AR, bool FOAM>
 __device__ __forceinline__ void pair_col_task(const FrameArgs& a, int ocean, int strip, const float2* inter_slot,
-                                              unsigned char* smem, int tid, unsigned* const* pub)
+                                              const Shared& sh, int tid, unsigned* const* pub)
 {
     using Fft = RegFft<P::LOG_N, P::E, AR>;
     constexpr int N = P::N, E = P::E, ROWS = P::ROWS, T = P::T, Q = NF / 2;
     const int w = tid % ROWS, c = tid / ROWS;
-    void* buf = smem + w * P::SEQ;
-    const float2* tws = reinterpret_cast<const float2*>(smem + P::TW);
-    ulonglong2* held = reinterpret_cast<ulonglong2*>(smem + P::HELD) + tid;  // pair 0 of cell j at [j * T]
-    float* src = reinterpret_cast<float*>(held);                             // later its foam source, at [4 T j]
+    void* buf = sh.exchange + w * P::SEQ;
+    ulonglong2* held = reinterpret_cast<ulonglong2*>(sh.held) + tid;  // pair 0 of cell j at [j * T]
+    float* src = reinterpret_cast<float*>(held);                      // later its foam source, at [4 T j]
     const int x0 = strip * ROWS;
     const size_t base = static_cast<size_t>(ocean) * N * N;
 #pragma unroll 1
@@ -203,7 +209,7 @@ __device__ __forceinline__ void pair_col_task(const FrameArgs& a, int ocean, int
             re[j] = px_pack(v.x, v.y);
             im[j] = px_pack(v.z, v.w);
         }
-        Fft::run(re, im, buf, tws, c);
+        Fft::run(re, im, buf, sh.tw, c);
         if (q == 0) publish(pub[0], tid);
         // Every thread's values of the last pair were in registers before the
         // transform's first barrier: the slot is free.
@@ -266,6 +272,23 @@ __device__ __forceinline__ void pair_col_task(const FrameArgs& a, int ocean, int
     }
 }
 
+// Ticket -> (row?, ocean, task index) for the queue order above: `tasks` tickets
+// each of R(0 .. ahead - 1), then R(ahead + i) and C(i) in turn, then the last C's.
+__device__ __forceinline__ void decode(unsigned t, unsigned tasks, unsigned ahead, unsigned count, bool& row,
+                                       unsigned& ocean, unsigned& idx)
+{
+    idx = t % tasks;
+    unsigned b = t / tasks;
+    if (b < ahead) {
+        row = true, ocean = b;
+        return;
+    }
+    b -= ahead;
+    const unsigned pairs = count - ahead;
+    row = b < 2u * pairs && (b & 1u) == 0u;
+    ocean = b < 2u * pairs ? (b >> 1) + (row ? ahead : 0u) : b - pairs;
+}
+
 template <class P, int NF, int AR, bool FOAM>
 __global__ void __launch_bounds__(P::T, P::CTAS) pair_frame_kernel(FrameArgs a, QueueArgs q)
 {
@@ -285,25 +308,13 @@ __global__ void __launch_bounds__(P::T, P::CTAS) pair_frame_kernel(FrameArgs a, 
     clear_words(q.clear, q.clear_words, tid, P::T);
     float2* tws = reinterpret_cast<float2*>(smem + P::TW);
     for (int i = tid; i < N - 1; i += P::T) tws[i] = a.twiddles[i];
+    const Shared sh{smem, tws, smem + P::HELD};
 
     const unsigned count = static_cast<unsigned>(q.count);
     const unsigned slots = static_cast<unsigned>(q.slots);
     const unsigned ring = min(P::ring(slots), count);
     const unsigned ahead = min(P::ahead(slots), count);
     const unsigned total = 2u * count * TASKS;
-    // Ticket -> (row?, ocean, task index) for the queue order above.
-    auto decode = [&](unsigned t, bool& row, unsigned& ocean, unsigned& idx) {
-        idx = t % TASKS;
-        unsigned b = t / TASKS;  // R(0 .. ahead - 1), then R(ahead + i), C(i) in turn, then the last C's
-        if (b < ahead) {
-            row = true, ocean = b;
-            return;
-        }
-        b -= ahead;
-        const unsigned pairs = count - ahead;
-        row = b < 2u * pairs && (b & 1u) == 0u;
-        ocean = b < 2u * pairs ? (b >> 1) + (row ? ahead : 0u) : b - pairs;
-    };
     if (tid == 0) {
         s_publish = nullptr;
         r_next = atomicAdd(q.ticket, 1u);
@@ -328,7 +339,7 @@ __global__ void __launch_bounds__(P::T, P::CTAS) pair_frame_kernel(FrameArgs a, 
                 }
                 bool row;
                 unsigned ocean, idx;
-                decode(t, row, ocean, idx);
+                decode(t, TASKS, ahead, count, row, ocean, idx);
                 if (row) {
                     if (ocean >= ring) dep = q.cols_done + (ocean - ring);
                     pub = q.rows_done + ocean;
@@ -353,15 +364,186 @@ __global__ void __launch_bounds__(P::T, P::CTAS) pair_frame_kernel(FrameArgs a, 
         if (t >= total || !s_ok) break;
         bool row;
         unsigned ocean, idx;
-        decode(t, row, ocean, idx);
+        decode(t, TASKS, ahead, count, row, ocean, idx);
         float2* inter = a.inter + static_cast<size_t>(ocean % ring) * N * N * NF;
         const int abs_ocean = a.ocean_base + static_cast<int>(ocean);
         if (row) {
-            pair_row_task<P, NF, AR>(a, abs_ocean, static_cast<int>(idx), inter, smem, tid, s_pub);
+            pair_row_task<P, NF, AR>(a, abs_ocean, static_cast<int>(idx), inter, sh, tid, s_pub);
         } else {
-            pair_col_task<P, NF, AR, FOAM>(a, abs_ocean, static_cast<int>(idx), inter, smem, tid, s_pub);
+            pair_col_task<P, NF, AR, FOAM>(a, abs_ocean, static_cast<int>(idx), inter, sh, tid, s_pub);
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// Several sizes in one launch (N = 64 to 1024, one field count, FP32 forms): the
+// tickets of group after group, each in the order above with its own counters,
+// ring and rows ahead. Every size's tasks take 256 threads, which 1024^2 needs
+// (the sizes below are 5 to 30 % faster alone with 128). Each size's twiddles
+// stay in shared memory. 64 oceans of 64^2 to 1024^2: 826 -> 531 us a frame, with
+// velocity 1209 -> 760; 5 oceans 110 -> 91. With fewer row tasks than SMs
+// (3 oceans up to 256^2 with velocity: 33 us there, 57 here) frame.cu's launch
+// takes them.
+// ---------------------------------------------------------------------------
+constexpr int kMixMin = 6, kMixMax = 10;
+constexpr int kMixThreads = 256;
+template <int LOG_N>
+using MixPlan = RegPlan<LOG_N, 8, kMixThreads * 8 / (1 << LOG_N)>;
+
+template <int LOG_N = kMixMin>
+constexpr size_t mix_exchange()
+{
+    constexpr size_t here = MixPlan<LOG_N>::TW;
+    if constexpr (LOG_N == kMixMax) {
+        return here;
+    } else {
+        constexpr size_t rest = mix_exchange<LOG_N + 1>();
+        return here > rest ? here : rest;
+    }
+}
+// The exchange area, then the twiddle tables (that of 2^l from float2 2^l - 64
+// on), then the threads' own values.
+constexpr size_t kMixTw = mix_exchange();
+constexpr size_t kMixHeld = kMixTw + sizeof(float2) * ((2 << kMixMax) - (1 << kMixMin));
+constexpr size_t kMixSmem = kMixHeld + sizeof(float4) * 8 * kMixThreads;
+static_assert(3 * (kMixSmem + 2048) <= 228 * 1024 && kMixHeld % 16 == 0, "three mixed CTAs fit on an SM");
+
+// A size's tasks. (As functions of their own, not inlined, they spilled around
+// the calls: 570 us against 531 for 64 oceans of 64^2 to 1024^2.)
+template <int LOG_N, int NF, int AR>
+__device__ __forceinline__ void mix_run(const MixedGroup& g, bool row, int ocean, int idx, unsigned char* smem, int tid,
+                                     unsigned* const* pub)
+{
+    using P = MixPlan<LOG_N>;
+    const Shared sh{smem, reinterpret_cast<const float2*>(smem + kMixTw) + (P::N - (1 << kMixMin)), smem + kMixHeld};
+    float2* inter = g.a.inter + static_cast<size_t>(ocean % g.ring) * P::N * P::N * NF;
+    if (row) {
+        pair_row_task<P, NF, AR>(g.a, ocean, idx, inter, sh, tid, pub);
+    } else {
+        pair_col_task<P, NF, AR, false>(g.a, ocean, idx, inter, sh, tid, pub);
+    }
+}
+
+__host__ __device__ constexpr unsigned mix_tasks(int log_n) { return (1u << (2 * log_n)) / (8u * kMixThreads); }
+static_assert(mix_tasks(6) == MixPlan<6>::TASKS && mix_tasks(10) == MixPlan<10>::TASKS, "tasks of a size");
+
+template <int NF, int AR>
+__global__ void __launch_bounds__(kMixThreads, 3) pair_mixed_kernel(const __grid_constant__ MixedArgs m)
+{
+    extern __shared__ float4 smem4[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(smem4);
+    __shared__ unsigned s_ticket;
+    __shared__ int s_ok, s_group, s_row, s_ocean, s_idx;
+    __shared__ unsigned* s_publish;
+    __shared__ unsigned* s_pub[2];
+    __shared__ MixedGroup s_groups[kMaxMixedGroups];  // tasks index it by a runtime group
+    unsigned r_next = 0;
+    int r_have_next = 0;
+    const int tid = threadIdx.x;
+    for (int i = tid; i < static_cast<int>(m.groups * sizeof(MixedGroup) / sizeof(unsigned)); i += kMixThreads)
+        reinterpret_cast<unsigned*>(s_groups)[i] = reinterpret_cast<const unsigned*>(m.g)[i];
+    if (blockIdx.x == 0 && tid == 0 && m.clear_ticket != nullptr) *m.clear_ticket = 0u;
+    for (int gi = 0; gi < m.groups; ++gi) {
+        const MixedGroup& g = m.g[gi];
+        clear_words(g.clear, g.clear_words, tid, kMixThreads);
+        const int n = 1 << g.log_n;
+        float2* tw = reinterpret_cast<float2*>(smem + kMixTw) + (n - (1 << kMixMin));
+        for (int i = tid; i < n - 1; i += kMixThreads) tw[i] = g.a.twiddles[i];
+    }
+    if (tid == 0) {
+        s_publish = nullptr;
+        r_next = atomicAdd(m.ticket, 1u);
+        r_have_next = 1;
+    }
+    while (true) {
+        __syncthreads();
+        if (tid == 0) {
+            unsigned* prev = s_publish;
+            const unsigned t = r_have_next ? r_next : atomicAdd(m.ticket, 1u);
+            r_have_next = 0;
+            int ok = 1;
+            unsigned* pub = nullptr;
+            unsigned* self = nullptr;
+            const unsigned* dep = nullptr;
+            unsigned need = 0;
+            if (t < m.total) {
+                if (t + 2u * gridDim.x < m.total) {
+                    r_next = atomicAdd(m.ticket, 1u);
+                    r_have_next = 1;
+                }
+                int gi = m.groups - 1;
+                while (gi > 0 && t < m.g[gi].first) --gi;
+                const MixedGroup& g = m.g[gi];
+                need = mix_tasks(g.log_n);
+                bool row;
+                unsigned ocean, idx;
+                decode(t - g.first, need, static_cast<unsigned>(g.ahead), static_cast<unsigned>(g.count), row, ocean, idx);
+                if (row) {
+                    if (ocean >= static_cast<unsigned>(g.ring)) dep = g.cols_done + (ocean - g.ring);
+                    pub = g.rows_done + ocean;
+                } else {
+                    dep = g.rows_done + ocean;
+                    self = g.cols_done + ocean;
+                }
+                s_group = gi;
+                s_row = row ? 1 : 0;
+                s_ocean = static_cast<int>(ocean);
+                s_idx = static_cast<int>(idx);
+            }
+            if (t >= m.total || !m.defer || (dep != nullptr && ld_acquire(dep) < need)) {
+                if (prev != nullptr) red_release_add(prev, 1u);
+                prev = nullptr;
+                if (dep != nullptr) ok = wait_at_least(dep, need, m.error, m.wait_ns);
+            }
+            s_pub[0] = prev;
+            s_pub[1] = self;
+            s_publish = pub;
+            s_ticket = t;
+            s_ok = ok;
+        }
+        __syncthreads();
+        if (s_ticket >= m.total || !s_ok) break;
+        const MixedGroup& g = s_groups[s_group];
+        const bool row = s_row != 0;
+        switch (g.log_n) {
+            case 6: mix_run<6, NF, AR>(g, row, s_ocean, s_idx, smem, tid, s_pub); break;
+            case 7: mix_run<7, NF, AR>(g, row, s_ocean, s_idx, smem, tid, s_pub); break;
+            case 8: mix_run<8, NF, AR>(g, row, s_ocean, s_idx, smem, tid, s_pub); break;
+            case 9: mix_run<9, NF, AR>(g, row, s_ocean, s_idx, smem, tid, s_pub); break;
+            default: mix_run<10, NF, AR>(g, row, s_ocean, s_idx, smem, tid, s_pub); break;
+        }
+    }
+}
+
+template <int NF, int AR>
+struct PairMixed {
+    static cudaError_t prepare()
+    {
+        return cudaFuncSetAttribute(pair_mixed_kernel<NF, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(kMixSmem));
+    }
+    static int blocks_per_sm()
+    {
+        int n = 0;
+        if (prepare() != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pair_mixed_kernel<NF, AR>, kMixThreads, kMixSmem) !=
+            cudaSuccess)
+            return 0;
+        return n;
+    }
+    static cudaError_t launch(const MixedArgs& m, int grid, cudaStream_t st)
+    {
+        cudaError_t e = prepare();
+        if (e != cudaSuccess) return e;
+        pair_mixed_kernel<NF, AR><<<grid, kMixThreads, kMixSmem, st>>>(m);
+        return cudaGetLastError();
+    }
+};
+template <typename Fn>
+auto mixed_variant(int nf, int ar, Fn&& fn)
+{
+    if (ar == kArFast) return nf == 4 ? fn(PairMixed<4, kArFast>{}) : fn(PairMixed<6, kArFast>{});
+    return nf == 4 ? fn(PairMixed<4, kArExact>{}) : fn(PairMixed<6, kArExact>{});
 }
 
 template <int LOG_N, int NF, int AR, bool FOAM>
@@ -430,6 +612,31 @@ bool has_plan(int log_n, int ar)
 }
 
 }  // namespace
+
+bool pair_mixed_ok(int log_n, int ar) { return ar != kArPrecise && log_n >= kMixMin && log_n <= kMixMax; }
+
+uint32_t pair_mixed_tasks(int log_n) { return mix_tasks(log_n); }
+
+int pair_mixed_blocks_per_sm(int nf, int ar)
+{
+    return mixed_variant(nf, ar, [](auto L) { return decltype(L)::blocks_per_sm(); });
+}
+
+cudaError_t launch_pair_mixed(int nf, int ar, MixedArgs m, int grid, cudaStream_t st)
+{
+    m.total = 0;
+    for (int i = 0; i < m.groups; ++i) {
+        MixedGroup& g = m.g[i];
+        const int tasks = static_cast<int>(mix_tasks(g.log_n));
+        const int wave = (148 * 3 + tasks - 1) / tasks;
+        const int ahead = wave > 2 ? wave : 2;
+        g.ahead = ahead < g.count ? ahead : g.count;
+        if (g.ring < g.count && g.ring <= g.ahead) return cudaErrorInvalidValue;  // the queue would wait on later tickets
+        g.first = m.total;
+        m.total += 2u * static_cast<uint32_t>(g.count) * static_cast<uint32_t>(tasks);
+    }
+    return mixed_variant(nf, ar, [&](auto L) { return decltype(L)::launch(m, grid, st); });
+}
 
 // A task takes its pairs one after the other, so a frame of few oceans, whose
 // tasks do not fill the GPU, is a longer chain here than with a task's pairs side

@@ -250,10 +250,10 @@ public:
         slots_ = static_cast<int>(std::min<uint32_t>(count_, 3));
         max_slots_ = slots_;
         defer_ = nf_ == 6;
-        // The persistent kernels' ring needs `ring` oceans; the row/column
+        // The persistent kernels' ring needs `ring_` oceans; the row/column
         // passes one per chunk ocean (all a batch above N = 1024 ever uses).
-        const uint32_t ring = static_cast<uint32_t>(frame_ring_slots(log_n_, form_, slots_, static_cast<int>(count_)));
-        const uint32_t inter_oceans = large() ? chunk_ : std::max(chunk_, ring);
+        ring_ = frame_ring_slots(log_n_, form_, slots_, static_cast<int>(count_));
+        const uint32_t inter_oceans = large() ? chunk_ : std::max(chunk_, static_cast<uint32_t>(ring_));
         inter_ = DevBuf<float2>(cells_ * nf_ * inter_oceans);
         queue_ = FrameQueue(count_, stream_);
         error_ = DevBuf<unsigned>(1);
@@ -833,6 +833,7 @@ public:
         g.clear_words = mixed_set_.words;
         g.count = static_cast<int32_t>(count_);
         g.slots = slots_;
+        g.ring = ring_;
         g.log_n = log_n_;
         return g;
     }
@@ -972,7 +973,8 @@ private:
     double prof_ms_[4] = {0.0, 0.0, 0.0, 0.0};
     bool persistent_ = true;
     int slots_ = 1;      // intermediate ring slots the persistent kernel uses
-    int max_slots_ = 1;  // slots the ring buffer holds
+    int max_slots_ = 1;  // the most of them
+    int ring_ = 1;       // oceans that the kernels' rings use at most
     bool defer_ = false; // QueueArgs::defer of the persistent kernel
     int frame_wave_[kMaxFramePlans][2] = {};  // [kernel plan][foam]: CTAs of one wave
     int sms_ = 0;
@@ -1383,8 +1385,13 @@ public:
             int sms = 0, dev = 0;
             check(cudaGetDevice(&dev), "cudaGetDevice");
             check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-            const int per_sm =
-                mixed_blocks_per_sm(batches_[0]->nf(), arith_of_form(batches_[0]->form()));
+            MixedArgs shape{};
+            shape.groups = static_cast<int32_t>(batches_.size());
+            for (size_t g = 0; g < batches_.size(); ++g) {
+                shape.g[g].log_n = ilog2u(batches_[g]->size());
+                shape.g[g].count = static_cast<int32_t>(batches_[g]->count());
+            }
+            const int per_sm = mixed_blocks_per_sm(batches_[0]->nf(), arith_of_form(batches_[0]->form()), shape);
             if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "mixed frame occupancy");
             mix_grid_ = per_sm * sms;
         }
@@ -1536,22 +1543,14 @@ private:
     {
         MixedArgs m{};
         m.groups = static_cast<int32_t>(mix_order_.size());
-        uint32_t first = 0;
-        for (size_t k = 0; k < mix_order_.size(); ++k) {
-            const size_t g = mix_order_[k];
-            m.g[k] = batches_[g]->mixed_group(t_over_2pi, st);
-            m.g[k].first = first;
-            first += mixed_tasks(m.g[k].log_n, m.g[k].count);
-        }
-        m.total = first;
+        for (size_t k = 0; k < mix_order_.size(); ++k) m.g[k] = batches_[mix_order_[k]]->mixed_group(t_over_2pi, st);
         const FrameQueue::Set ticket = mix_ticket_.take(st);
         m.ticket = ticket.ticket;
         m.clear_ticket = ticket.clear;
         m.error = mix_error_.p;
         m.wait_ns = 1000000000ull;
         m.defer = mix_defer_ ? 1 : 0;
-        const int grid = static_cast<int>(std::min<uint64_t>(static_cast<uint64_t>(mix_grid_), first));
-        check(launch_mixed_frame(batches_[0]->nf(), arith_of_form(batches_[0]->form()), m, grid, st),
+        check(launch_mixed_frame(batches_[0]->nf(), arith_of_form(batches_[0]->form()), m, mix_grid_, st),
               "mixed frame kernel");
         mix_ticket_.launched(ticket);
         for (size_t g : mix_order_) batches_[g]->mixed_launched();
@@ -1723,7 +1722,7 @@ private:
     bool mixed_ = false;
     bool mixed_shallow_ = false;  // the one launch timed fastest with the shallowest rings
     bool mix_defer_ = false;      // MixedArgs::defer (default: with velocity)
-    int mix_grid_ = 0;
+    int mix_grid_ = 0;            // CTAs of one wave
     std::vector<size_t> mix_order_;
     FrameQueue mix_ticket_;
     DevBuf<unsigned> mix_error_;

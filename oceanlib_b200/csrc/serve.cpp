@@ -962,6 +962,8 @@ private:
                 g.clear_words = set.words;
                 g.count = count;
                 g.slots = std::min(count, 3);
+                g.ring = frame_ring_slots(k->log_n, desc_.fft_form, g.slots, count);
+                g.a.inter = ring_for(k, static_cast<size_t>(g.ring));
                 g.log_n = k->log_n;
                 continue;
             }
@@ -986,12 +988,6 @@ private:
         if (one_launch) {
             // Largest sizes first, so the short tasks fill the wave's tail.
             std::sort(m.g, m.g + m.groups, [](const MixedGroup& x, const MixedGroup& y) { return x.log_n > y.log_n; });
-            uint32_t first = 0;
-            for (int i = 0; i < m.groups; ++i) {
-                m.g[i].first = first;
-                first += mixed_tasks(m.g[i].log_n, m.g[i].count);
-            }
-            m.total = first;
             const FrameQueue::Set ticket = mix_ticket_.take(stream_);
             m.ticket = ticket.ticket;
             m.clear_ticket = ticket.clear;
@@ -1000,14 +996,13 @@ private:
             const int nf = oparts[0].k->nf;
             m.defer = nf == 6 ? 1 : 0;
             const int ar = arith_of_form(desc_.fft_form);
-            int& grid = mix_grid_[nf == 6 ? 1 : 0];
-            if (grid == 0) {
-                const int per_sm = mixed_blocks_per_sm(nf, ar);
+            int& wave = mix_wave_[mixed_pairs(ar, m) ? 1 : 0][nf == 6 ? 1 : 0];
+            if (wave == 0) {
+                const int per_sm = mixed_blocks_per_sm(nf, ar, m);
                 if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "mixed frame occupancy");
-                grid = per_sm * sms_;
+                wave = per_sm * sms_;
             }
-            check(launch_mixed_frame(nf, ar, m, static_cast<int>(std::min<uint64_t>(grid, first)), stream_),
-                  "mixed frame kernel");
+            check(launch_mixed_frame(nf, ar, m, wave, stream_), "mixed frame kernel");
             mix_ticket_.launched(ticket);
             for (size_t i = 0; i < oparts.size(); ++i) oparts[i].k->queue.launched(sets[i]);
             ++kernels;
@@ -1247,7 +1242,7 @@ private:
     cudaMemPool_t pool_ = nullptr;
     DevBuf<unsigned> error_;
     FrameQueue mix_ticket_;  // the one-launch frame's ticket
-    int mix_grid_[2] = {0, 0};     // its resident grid, by field count (4, 6)
+    int mix_wave_[2][2] = {};      // its CTAs of one wave, by kernel and field count (4, 6)
     std::vector<std::unique_ptr<BatchCtx>> ctxs_;
     std::deque<BatchCtx*> free_ctx_, inflight_;
     std::vector<std::unique_ptr<OceanKind>> ocean_kinds_;

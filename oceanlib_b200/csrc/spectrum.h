@@ -147,9 +147,11 @@ struct MixedGroup {
     FrameArgs a;          // the group's arrays, or its pointer table (ocean_base 0)
     unsigned* rows_done;  // [count]
     unsigned* cols_done;  // [count]
-    uint32_t first;       // first ticket of the group
+    uint32_t first;       // first ticket of the group (set by the launch)
     int32_t count;        // oceans
-    int32_t slots;        // intermediate ring slots (a.inter holds them)
+    int32_t slots;        // intermediate ring slots of the plain mixed launch
+    int32_t ring;         // slots that a.inter holds (min(count, frame_ring_slots))
+    int32_t ahead;        // set by the launch
     int32_t log_n;
     unsigned* clear;      // next launch's words of this group
     uint32_t clear_words;
@@ -157,7 +159,7 @@ struct MixedGroup {
 struct MixedArgs {
     MixedGroup g[kMaxMixedGroups];
     int32_t groups;
-    uint32_t total;       // tickets of all groups
+    uint32_t total;       // tickets of all groups (set by the launch)
     unsigned* ticket;
     unsigned* clear_ticket;  // may be null
     unsigned* error;      // sticky: set when a bounded wait gives up
@@ -165,9 +167,17 @@ struct MixedArgs {
     int32_t defer;        // as QueueArgs::defer, for every group
 };
 bool mixed_size_ok(int log_n);
-uint32_t mixed_tasks(int log_n, int count);
-int mixed_blocks_per_sm(int nf, int ar);
-cudaError_t launch_mixed_frame(int nf, int ar, const MixedArgs& m, int grid, cudaStream_t stream);
+// Whether these groups (log_n, count) run in this arithmetic as register-resident
+// tasks (frame_pairs.cu: sizes from 64 on, FP32 forms, enough row tasks to give
+// every SM one) or as frame.cu's; the launch's
+// resident CTAs per SM; and the launch, with the CTAs of one wave.
+bool mixed_pairs(int ar, const MixedArgs& m);
+int mixed_blocks_per_sm(int nf, int ar, const MixedArgs& m);
+cudaError_t launch_mixed_frame(int nf, int ar, const MixedArgs& m, int wave, cudaStream_t stream);
+bool pair_mixed_ok(int log_n, int ar);
+uint32_t pair_mixed_tasks(int log_n);  // row tasks of an ocean
+int pair_mixed_blocks_per_sm(int nf, int ar);
+cudaError_t launch_pair_mixed(int nf, int ar, MixedArgs m, int grid, cudaStream_t stream);
 
 // Row pass (evolve + row FFTs) and column pass (column FFTs + finalize, with
 // an optional fused foam substep) for `args.chunk` oceans starting at
