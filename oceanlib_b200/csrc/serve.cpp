@@ -37,6 +37,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <condition_variable>
@@ -217,7 +218,6 @@ struct BatchCtx {
     float gpu_ms = 0.0f;
     bool complete = false;
     bool failed = false;
-    void* server = nullptr;
 };
 
 struct Layout {
@@ -266,7 +266,6 @@ public:
             c = std::make_unique<BatchCtx>();
             check(cudaEventCreate(&c->start), "event");
             check(cudaEventCreate(&c->done), "event");
-            c->server = this;
             ensure_host(c.get(), in_reserve, out_reserve);
             free_ctx_.push_back(c.get());
         }
@@ -281,7 +280,7 @@ public:
             std::lock_guard<std::mutex> lk(mu_);
             stop_ = true;
         }
-        cv_.notify_all();
+        wake();
         if (thread_.joinable()) thread_.join();
         cudaStreamSynchronize(stream_);
         for (auto& kv : sessions_)
@@ -342,7 +341,7 @@ public:
         Session* raw = s.get();
         sessions_[raw->id] = std::move(s);
         waiting_.push_back(raw);
-        cv_.notify_all();
+        wake();
         return raw->id;
     }
 
@@ -373,7 +372,7 @@ public:
             ready_.push_back(s);
         }
         ++submitted_;
-        cv_.notify_all();
+        wake();
         return raw->ticket;
     }
 
@@ -1048,20 +1047,8 @@ private:
             if (s->block) check(cudaFreeAsync(s->block, stream_), "free session");
             s->block = nullptr;
         }
-        check(cudaLaunchHostFunc(stream_, &Server::on_done, c), "host callback");
         c->points = plan.points;
         c->kernels = kernels;
-    }
-
-    static void CUDART_CB on_done(void* p)
-    {
-        BatchCtx* c = static_cast<BatchCtx*>(p);
-        Server* s = static_cast<Server*>(c->server);
-        {
-            std::lock_guard<std::mutex> lk(s->mu_);
-            c->complete = true;
-        }
-        s->cv_.notify_all();
     }
 
     // Outside the lock: results to the callers' buffers.
@@ -1122,6 +1109,35 @@ private:
     }
 
     // ---- the dispatcher -------------------------------------------------------
+    // After a change to what the dispatcher looks at, under the lock or not.
+    void wake()
+    {
+        poked_.store(true, std::memory_order_release);
+        cv_.notify_all();
+    }
+
+    // While a batch is in flight: watches for its end, or for new work. A host
+    // callback in the stream instead held the next batch back until it had run
+    // (it takes the server's lock) and woke this thread through the scheduler,
+    // twice per batch; 32 sessions' update and query a tick 1.6 -> 0.88 ms.
+    void poll_front(std::unique_lock<std::mutex>& lk)
+    {
+        BatchCtx* c = inflight_.front();
+        poked_.store(false, std::memory_order_relaxed);  // under the lock: what came before has been looked at
+        lk.unlock();
+        cudaError_t e = cudaErrorNotReady;
+        while (!poked_.load(std::memory_order_acquire)) {
+            e = cudaEventQuery(c->done);
+            if (e != cudaErrorNotReady) break;
+            std::this_thread::yield();
+        }
+        lk.lock();
+        if (e != cudaErrorNotReady) {
+            c->complete = true;
+            if (e != cudaSuccess) c->failed = true;
+        }
+    }
+
     void run()
     {
         cudaSetDevice(device_);  // the dispatcher issues every launch on the server's device
@@ -1203,8 +1219,11 @@ private:
             if (stop_ && inflight_.empty() && ready_.empty()) {
                 if (!can_admit_locked()) break;  // nothing left to free for those waiting
             }
+            if (!inflight_.empty()) {
+                poll_front(lk);
+                continue;
+            }
             cv_.wait_for(lk, std::chrono::milliseconds(50), [&] {
-                if (!inflight_.empty() && inflight_.front()->complete) return true;
                 if (!free_ctx_.empty() && !ready_.empty()) return true;
                 if (can_admit_locked()) return true;
                 return stop_;
@@ -1250,6 +1269,7 @@ private:
 
     std::mutex mu_;
     std::condition_variable cv_, done_cv_;
+    std::atomic<bool> poked_{false};
     std::thread thread_;
     bool stop_ = false;
     std::unordered_map<uint64_t, std::unique_ptr<Session>> sessions_;
