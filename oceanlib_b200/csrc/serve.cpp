@@ -245,6 +245,9 @@ public:
         check(cudaGetDevice(&device_), "cudaGetDevice");
         check(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "SM count");
         check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
+        check(cudaStreamCreateWithFlags(&field_stream_, cudaStreamNonBlocking), "cudaStreamCreate");
+        check(cudaEventCreateWithFlags(&uploaded_, cudaEventDisableTiming), "event");
+        check(cudaEventCreateWithFlags(&fields_done_, cudaEventDisableTiming), "event");
         cudaMemPoolProps props;
         std::memset(&props, 0, sizeof(props));
         props.allocType = cudaMemAllocationTypePinned;
@@ -282,6 +285,7 @@ public:
         }
         wake();
         if (thread_.joinable()) thread_.join();
+        cudaStreamSynchronize(field_stream_);
         cudaStreamSynchronize(stream_);
         for (auto& kv : sessions_)
             if (kv.second->block) cudaFreeAsync(kv.second->block, stream_);
@@ -296,6 +300,9 @@ public:
         ocean_kinds_.clear();
         field_kinds_.clear();
         if (pool_) cudaMemPoolDestroy(pool_);
+        cudaEventDestroy(uploaded_);
+        cudaEventDestroy(fields_done_);
+        cudaStreamDestroy(field_stream_);
         cudaStreamDestroy(stream_);
     }
 
@@ -931,6 +938,7 @@ private:
         uint32_t kernels = 0;
         check(cudaEventRecord(c->start, stream_), "event");
         if (in_bytes > 0) check(cudaMemcpyAsync(d, h, in_bytes, cudaMemcpyHostToDevice, stream_), "batch upload");
+        check(cudaEventRecord(uploaded_, stream_), "event");
         // The batch's oceans: one launch for every size when the sizes allow
         // it (mixed_frame_kernel: N up to 1024, one field count, an FP32
         // form), else one persistent launch per size.
@@ -1006,9 +1014,14 @@ private:
             for (size_t i = 0; i < oparts.size(); ++i) oparts[i].k->queue.launched(sets[i]);
             ++kernels;
         }
+        // The fields beside the oceans: neither needs the other before the
+        // queries, and a batch of a few sessions fills the GPU with neither
+        // (32 sessions' update and query a tick 0.88 -> 0.81 ms).
+        const cudaStream_t fst = !plan.fields.empty() && !plan.frames.empty() ? field_stream_ : stream_;
+        if (fst != stream_) check(cudaStreamWaitEvent(fst, uploaded_, 0), "fork");
         const IWaveSource* dev_src = reinterpret_cast<const IWaveSource*>(d + src_off);
         if (!plan.sources.empty()) {
-            check(launch_source_mean(const_cast<IWaveSource*>(dev_src), static_cast<int>(plan.sources.size()), stream_),
+            check(launch_source_mean(const_cast<IWaveSource*>(dev_src), static_cast<int>(plan.sources.size()), fst),
                   "source mean");
             ++kernels;
         }
@@ -1018,17 +1031,21 @@ private:
                 const IWaveField* fl = reinterpret_cast<const IWaveField*>(d + sp.fields);
                 if (sp.any_sources) {
                     check(launch_source_apply(fl, reinterpret_cast<const int2*>(d + sp.ranges), int2{}, dev_src,
-                                              static_cast<int>(sp.count), static_cast<int>(g.n), stream_),
+                                              static_cast<int>(sp.count), static_cast<int>(g.n), fst),
                           "sources");
                     ++kernels;
                 }
                 check(launch_iwave_step(static_cast<int>(g.p), fl, static_cast<int>(sp.count), static_cast<int>(g.n),
-                                        g.taps, stream_), "iwave step");
+                                        g.taps, fst), "iwave step");
                 ++kernels;
             }
             check(launch_iwave_finalize(reinterpret_cast<const IWaveField*>(d + fp.fin), static_cast<int>(fp.fin_count),
-                                        static_cast<int>(g.n), stream_), "finalize");
+                                        static_cast<int>(g.n), fst), "finalize");
             ++kernels;
+        }
+        if (fst != stream_) {
+            check(cudaEventRecord(fields_done_, fst), "join");
+            check(cudaStreamWaitEvent(stream_, fields_done_, 0), "join");
         }
         if (!plan.queries.empty()) {
             check(launch_serve_queries(reinterpret_cast<const QueryJob*>(d + jobs_off),
@@ -1209,6 +1226,11 @@ private:
                         batched_requests_ += c->requests.size();
                         inflight_.push_back(c);
                     } else {
+                        // Whatever of it was queued may still use its staging.
+                        lk.unlock();
+                        cudaStreamSynchronize(field_stream_);
+                        cudaStreamSynchronize(stream_);
+                        lk.lock();
                         fail_locked(c);
                         free_ctx_.push_back(c);
                         done_cv_.notify_all();
@@ -1257,7 +1279,8 @@ private:
 
     ocean_server_desc desc_;
     int device_ = 0, sms_ = 0;
-    cudaStream_t stream_ = nullptr;
+    cudaStream_t stream_ = nullptr, field_stream_ = nullptr;
+    cudaEvent_t uploaded_ = nullptr, fields_done_ = nullptr;  // a batch's fork and join
     cudaMemPool_t pool_ = nullptr;
     DevBuf<unsigned> error_;
     FrameQueue mix_ticket_;  // the one-launch frame's ticket
