@@ -70,7 +70,7 @@ struct Shape {
 //   from L2: the mirror row's task is the neighbouring ticket) for half the
 //   threads. Column tasks of the persistent kernels cover PW = ROWS columns,
 //   so both task kinds have the same thread count, ROWS * NF * G.
-template <int LOG_N_, int G_, bool TC_, bool SINGLE_ROWS>
+template <int LOG_N_, int G_, bool TC_, bool SINGLE_ROWS, int MAX_PAIRS = 32>
 struct Plan {
     static constexpr int LOG_N = LOG_N_;
     static constexpr int N = 1 << LOG_N;
@@ -78,7 +78,7 @@ struct Plan {
     static constexpr bool TC = TC_;
     static constexpr int SEQ = padded_len(N) + kPad;                  // sequence stride (float2)
     static constexpr int SEQ4 = padded_len4(N) + kPad4;               // pair stride (float4)
-    static constexpr int RP = cmin(N / 2, 32 / G > 1 ? 32 / G : 1);  // row pairs / task
+    static constexpr int RP = cmin(MAX_PAIRS, cmin(N / 2, 32 / G > 1 ? 32 / G : 1));  // row pairs / task
     static constexpr int LANE_LOG = ilog2c(N / G);
     static_assert(LANE_LOG >= 2, "a lane keeps at least four values");
     static constexpr bool PAIRED =
@@ -102,8 +102,19 @@ struct Plan {
 // measured at N = 512 (64 oceans, velocity and persistent foam): 1.336 ms per
 // frame against 1.117 ms with row pairs - the second h0 read and twice the
 // tasks cost more than the smaller CTAs recover.
-template <int LOG_N, bool TC>
-using FramePlan = Plan<LOG_N, lanes_for(LOG_N), TC, false>;
+// At N = 64 to 256 this kernel runs frames of a few oceans (pair_frame_ok), whose
+// tasks do not fill the GPU: a task is one row pair (two at 64), so that the SMs
+// share them evenly. 3 x 256^2 with velocity, frames of several cascades at once:
+// 13.0 -> 12.2 us, 2 x 128^2 6.1 -> 4.5, one 64^2 ocean 12.6 -> 9.8, against eight
+// to two pairs a task. (With foam 256^2 keeps two: two columns' foam is 8 bytes a
+// row, 22.4 us for three oceans against 20.9.)
+template <int LOG_N>
+__host__ __device__ constexpr int frame_max_pairs(bool tc, bool foam)
+{
+    return tc || LOG_N < 6 || LOG_N > 8 ? 32 : (LOG_N == 6 || (LOG_N == 8 && foam) ? 2 : 1);
+}
+template <int LOG_N, bool TC, bool FOAM = false>
+using FramePlan = Plan<LOG_N, lanes_for(LOG_N), TC, false, frame_max_pairs<LOG_N>(TC, FOAM)>;
 // The per-chunk kernels' plan.
 template <int LOG_N>
 using ChunkPlan = Plan<LOG_N, lanes_for(LOG_N), false, false>;
@@ -119,16 +130,16 @@ __host__ __device__ constexpr int frame_plan_count(bool tc)
 {
     return (!tc && LOG_N >= 8 && LOG_N <= 10) ? 2 : 1;
 }
-template <int LOG_N, int V, bool TC>
+template <int LOG_N, int V, bool TC, bool FOAM>
 struct PlanOfT {
-    using type = FramePlan<LOG_N, TC>;
+    using type = FramePlan<LOG_N, TC, FOAM>;
 };
-template <int LOG_N>
-struct PlanOfT<LOG_N, 1, false> {
+template <int LOG_N, bool FOAM>
+struct PlanOfT<LOG_N, 1, false, FOAM> {
     using type = Plan<LOG_N, (LOG_N >= 10 ? 64 : lanes_for(LOG_N)), false, true>;
 };
-template <int LOG_N, int V, bool TC>
-using PlanOf = typename PlanOfT<LOG_N, V, TC>::type;
+template <int LOG_N, int V, bool TC, bool FOAM>
+using PlanOf = typename PlanOfT<LOG_N, V, TC, FOAM>::type;
 
 // Column tasks over 2 columns shift their sequence pairs (pair s = field
 // pair * W + column) by a few float4 so that the intermediate's stores (lanes
@@ -1202,7 +1213,7 @@ constexpr size_t frame_smem_bytes()
 
 template <int LOG_N, int NF, int AR, bool FOAM, bool TC = false, int V = 0>
 struct FrameLaunch {
-    using P = PlanOf<LOG_N, V, TC>;
+    using P = PlanOf<LOG_N, V, TC, FOAM>;
     using Eng = TcEngineOf<LOG_N, NF>;
     static constexpr int threads() { return P::template threads<NF>(); }
     static constexpr size_t smem() { return frame_smem_bytes<P, NF>(); }
