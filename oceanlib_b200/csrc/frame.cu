@@ -27,6 +27,7 @@
 #include "tc_dft.cuh"
 #include "tc_dft_small.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace ocean_b200 {
@@ -94,7 +95,9 @@ struct Plan {
     template <int NF>
     __host__ __device__ static constexpr int threads()
     {
-        return ROWS * NF * G;
+        // The 512-point tensor engine takes a velocity task's 12 sequences in
+        // two calls of 6, so that the accumulators of two CTAs fit an SM.
+        return TC && LOG_N == 9 && NF == 6 ? ROWS * 3 * G : ROWS * NF * G;
     }
 };
 
@@ -179,11 +182,11 @@ __host__ __device__ constexpr int foam_window_f2()
     return (1 << LOG_N) * foam_window<W>() / 2;
 }
 
-// The tensor-core engine of a task's sequences, one engine call per
-// transform: at N = 512 the 2 NF sequences of a row pair or two columns (8
-// without velocity, 12 with); at N = 64, 128 and 256 the ROWS x NF of the
-// plan's rows or columns (16 x threads values in all). Sizes without a
-// tensor-core form name the 512-point engine, which their kernels never use.
+// The tensor-core engine of a task's sequences: at N = 512 one call of 8 for
+// the fields of a row pair or two columns without velocity, two of 6 with it;
+// at N = 64, 128 and 256 one call for the ROWS x NF of the plan's rows or
+// columns (16 x threads values in all). Sizes without a tensor-core form name
+// the 512-point engine, which their kernels never use.
 template <int LOG_N>
 __host__ __device__ constexpr bool has_tc_form()
 {
@@ -191,7 +194,7 @@ __host__ __device__ constexpr bool has_tc_form()
 }
 template <int LOG_N, int NF>
 struct TcEngineOfT {
-    using type = tc::Engine<2 * NF>;
+    using type = tc::Engine<NF == 6 ? 6 : 8>;
 };
 template <int LOG_N, int NF>
     requires(LOG_N >= 6 && LOG_N <= 8)
@@ -212,16 +215,18 @@ __device__ __forceinline__ void load_twiddles(float2* tws, const float2* __restr
 // The inverse DFT of the COUNT sequences of a task: the radix-2 Stockham FFT
 // on single sequences (one lane group of G per sequence) or on sequence pairs
 // (one lane group of G2 per pair, named barrier 1 + pair where a pair spans
-// two warps), or with TC the tensor-core four-step DFT, 8 sequences per
-// engine call (N = 512; its twiddles live in the engine).
+// two warps), or with TC the tensor-core four-step DFT (its twiddles live in the
+// engine).
 template <class P, int AR, int COUNT, int COLW = 0, class Eng = tc::Engine<8>>
 __device__ __forceinline__ void transform_all(float2* data, const float2* tws, int tid, Eng* eng,
                                               unsigned* error)
 {
     if constexpr (P::TC && P::LOG_N == 9) {
         static_assert(P::SEQ * 2 >= 16 * tc::kZStride, "a sequence's space must hold its staged stage-3 rows");
-        static_assert(COUNT == Eng::Lay::kThreads / 32, "one engine call holds the task's sequences");
-        eng->dft512(data, P::SEQ, COUNT, tid, error);
+        constexpr int S = Eng::Lay::kThreads / 32;
+        static_assert(COUNT % S == 0, "whole engine calls");
+#pragma unroll 1
+        for (int s = 0; s < COUNT; s += S) eng->dft512(data + s * P::SEQ, P::SEQ, S, tid, error);
     } else if constexpr (P::TC) {
         static_assert(has_tc_form<P::LOG_N>(), "the tensor-core form covers N = 64 to 512");
         static_assert(P::SEQ * 2 >= Eng::Lay::N1 * Eng::Lay::kZStride,
@@ -333,7 +338,7 @@ __device__ __forceinline__ void row_task(const FrameArgs& a, int ocean, int grou
     using D = P;
     constexpr int LOG_N = P::LOG_N;
     constexpr int N = P::N, G = P::G, SEQ = P::SEQ, SEQ4 = P::SEQ4, ROWS = P::ROWS;
-    constexpr int NT = ROWS * NF * G;
+    constexpr int NT = P::template threads<NF>();
     constexpr int Q = NF / 2;
     constexpr bool PAIRED = P::PAIRED;
 
@@ -500,7 +505,7 @@ __device__ __forceinline__ void col_task(const FrameArgs& a, int ocean, int stri
                                          unsigned* error = nullptr, unsigned* const* pub = nullptr)
 {
     constexpr int N = P::N, G = P::G, SEQ = P::SEQ, SEQ4 = P::SEQ4;
-    constexpr int NT = NF * W * G;
+    constexpr int NT = W == P::PW ? P::template threads<NF>() : NF * W * G;
     constexpr int Q = NF / 2;
     constexpr bool PAIRED = P::PAIRED;
     float2* data = smem;                             // TC: sequence f*W + w
@@ -703,7 +708,7 @@ template <class P, int NF>
 constexpr int frame_min_blocks()
 {
     constexpr int nt = P::template threads<NF>();
-    if (P::TC) return 1;
+    if (P::TC) return P::LOG_N == 9 ? 2 : 1;  // two: 256 of the SM's 512 columns of tensor memory each
     if (P::LANE_LOG >= 5) return 1;  // 32 values a lane: the registers allow one CTA
     return 768 / nt < 1 ? 1 : (768 / nt > 16 ? 16 : 768 / nt);
 }
@@ -1228,26 +1233,39 @@ struct FrameLaunch {
     static int blocks_per_sm()
     {
         if (prepare() != cudaSuccess) return 0;
+        if (TC) return tensor_blocks_per_sm();
         int n = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, frame_kernel<P, NF, AR, FOAM>, threads(), smem()) !=
             cudaSuccess)
             return 0;
-        // The tensor-core engine's tensor memory bounds its residency.
-        if (TC && n * Eng::Lay::kTmemCols > 512) n = 512 / Eng::Lay::kTmemCols;
         return n;
+    }
+
+    // The tensor-core kernels' CTAs per SM, from their columns of tensor
+    // memory, shared memory and registers: the runtime's own figure is one
+    // for every kernel that allocates tensor memory. At 512 two share an SM
+    // (64 x 512^2 without velocity: 1755 us a frame with one, 1124 with two).
+    // A CTA that had to wait for its columns would hold no ticket, so a grid
+    // beyond what fits costs time only.
+    static int tensor_blocks_per_sm()
+    {
+        int dev = 0, sm_smem = 0, cta_smem = 0, sm_regs = 0;
+        cudaFuncAttributes at{};
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&cta_smem, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sm_regs, cudaDevAttrMaxRegistersPerMultiprocessor, dev) != cudaSuccess ||
+            cudaFuncGetAttributes(&at, frame_kernel<P, NF, AR, FOAM>) != cudaSuccess)
+            return 0;
+        const int by_smem = sm_smem / (static_cast<int>(smem() + at.sharedSizeBytes + 127) / 128 * 128 + cta_smem);
+        const int by_regs = sm_regs / ((at.numRegs + 7) / 8 * 8 * threads());
+        return std::min({512 / Eng::Lay::kTmemCols, by_smem, by_regs});
     }
 
     static cudaError_t launch(const FrameArgs& a, const QueueArgs& q, int grid, cudaStream_t st)
     {
         cudaError_t e = prepare();
         if (e != cudaSuccess) return e;
-        if (TC) {
-            // Every resident CTA must obtain its tensor memory without waiting.
-            int n = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, frame_kernel<P, NF, AR, FOAM>, threads(), smem());
-            if (e != cudaSuccess) return e;
-            if (n * Eng::Lay::kTmemCols > 512) return cudaErrorInvalidConfiguration;
-        }
         frame_kernel<P, NF, AR, FOAM><<<grid, threads(), smem(), st>>>(a, q);
         return cudaGetLastError();
     }

@@ -9,11 +9,11 @@
 //   X[k1 + 16 k2] = sum_n2 W32^(n2 k2) Z[n2, k1]           stage 3 (GEMM)
 //
 // Each stage is one real GEMM D = A B^T on the tensor cores
-// (tcgen05.mma kind::f16: FP16 operands in shared memory, FP32 accumulators
-// in tensor memory): the complex DFT matrix becomes the real block matrix
-// [[C, -S], [S, C]] and a row of A holds one short sequence as (re..., im...).
-// Stage 1 has 8 x 32 = 256 rows (two M = 128 tiles), K = 32, N = 32; stage 3
-// has 8 x 16 = 128 rows, K = 64, N = 64.
+// (tcgen05.mma kind::i8: signed 8-bit operands in shared memory, 32-bit
+// integer accumulators in tensor memory): the complex DFT matrix becomes the
+// real block matrix [[C, -S], [S, C]] and a row of A holds one short sequence
+// as (re..., im...). Stage 1 has 8 x 32 = 256 rows (two M = 128 tiles), K =
+// 32, N = 32; stage 3 has 8 x 16 = 128 rows, K = 64, N = 64.
 //
 // Precision: a plain FP16 split (hi + lo) still rounds every accumulation in
 // FP32 against the dominant spectral terms of a row, which costs 2-3x the
@@ -21,15 +21,23 @@
 // scaled by a power of two so its largest magnitude lies in [2^29, 2^30),
 // rounded to an integer (30 significant bits relative to the row maximum),
 // and cut into four signed 8-bit digits a_i (weights 2^24, 2^16, 2^8, 1);
-// the DFT matrices likewise at 2^30. FP16 holds the digits exactly, every
-// product a_i b_j is an exact integer below 2^14, and a level
-// D_L = sum over i + j = L of A_i B_j^T (at most 4 pairs x 64 terms) stays
-// below 2^22 - so the FP32 accumulators hold every level EXACTLY, whatever
-// order the tensor cores add in. Levels 0..3 (10 products per K step) are
-// kept; the dropped ones weigh 2^-32 of the leading term. The four exact
-// levels are then combined in FP32 (three roundings). The GEMMs are thus
-// as good as FP64 ones; the remaining error is the FP32 twiddle step and the
-// FP32 values between the stages - below the radix-2 FP32 FFT's own.
+// the DFT matrices likewise at 2^30. A level D_L = sum over i + j = L of
+// A_i B_j^T (at most 4 pairs x 64 terms) stays below 2^22, exact in the
+// integer accumulators. Levels 0..3 (10 products per K step) are kept; the
+// dropped ones weigh 2^-32 of the leading term. The levels combine in pairs,
+// still exactly, and the two pairs in FP32 (two roundings). The GEMMs are
+// thus as good as FP64 ones; the remaining error is the FP32 twiddle step and
+// the FP32 values between the stages - below the radix-2 FP32 FFT's own.
+//
+// What bounds it: the work around the MMAs (digits, tensor-memory reads,
+// staging) and the waits between its phases, at 12-16 warps an SM; the tensor
+// pipe is 6-9 % active. The digits as bytes of one integer (a conversion, an
+// add, a flip and two byte permutes a value) took 18 FP32 and conversion
+// instructions a value as FP16 operands, whose planes were also twice as
+// large and took twice the MMAs: 16 x 512^2 with velocity 735 -> 551 us a
+// frame. Operands and accumulators then fit two CTAs on an SM, so that one
+// works while the other waits: 551 -> 459 (and without velocity, where the
+// frame is one engine call a task, 503 -> 295).
 //
 // One elected thread issues the MMAs and commits them to an mbarrier; every
 // wait on it is bounded (the error word is set and the engine gives up
@@ -56,37 +64,37 @@ constexpr int kFixExp = 29;      // row max scaled into [2^29, 2^30)
 constexpr int kBExp = 30;        // DFT matrices scaled by 2^30
 constexpr unsigned long long kWaitNs = 1000000000ull;  // 1 s
 
-// An engine call transforms SEQS sequences (8, or 12: a frame task's 2 rows
-// x 6 fields) with SEQS x 32 threads. Stage 1 has SEQS x 32 rows (SEQS / 4
-// tiles of M = 128); stage 3 has SEQS x 16 rows, one tile or two, the second
-// holding rows 128..191 (its MMA also reads the 64 rows behind them, which
-// lie inside the engine's shared memory and land in tensor-memory lanes that
-// are never read). Accumulators (FP32 columns), one per level: stage 1 tile
-// t, level L at 128 t + 32 L; stage 3 tile t, level L at 256 t + 64 L.
+// An engine call transforms SEQS sequences (8, or 6: half of a frame task's 2
+// rows x 6 fields) with SEQS x 32 threads. Stage 1 has SEQS x 32 rows, two
+// tiles of M = 128; stage 3 SEQS x 16 rows, one tile. With 6 sequences the
+// tiles also read 64 and 32 rows past the operand: they lie inside the
+// engine's shared memory and land in tensor-memory lanes that are never
+// read. Accumulators (32-bit integer columns), one per level: stage 1 tile t,
+// level L at 128 t + 32 L; stage 3, level L at 64 L: 256 columns, so two CTAs
+// share an SM's 512.
 // Shared-memory layout in bytes, all offsets 128-byte aligned.
 template <int SEQS>
 struct Layout {
-    static_assert(SEQS == 8 || SEQS == 12, "8 or 12 sequences per engine call");
+    static_assert(SEQS == 6 || SEQS == 8, "6 or 8 sequences per engine call");
     static constexpr int kRows1 = SEQS * 32;
-    static constexpr int kTiles1 = kRows1 / 128;
+    static constexpr int kTiles1 = (kRows1 + 127) / 128;
     static constexpr int kRows3 = SEQS * 16;
-    static constexpr int kTiles3 = (kRows3 + 127) / 128;
     static constexpr int kThreads = SEQS * 32;
-    static constexpr int kTmemCols = kTiles3 > 1 ? 512 : 256;
-    static constexpr int kAHalves = kRows1 * kK1;  // halves per digit plane (== kRows3 * kK3)
+    static constexpr int kTmemCols = 256;
+    static constexpr int kABytes = kRows1 * kK1;  // bytes per digit plane (== kRows3 * kK3)
     static_assert(kRows1 * kK1 == kRows3 * kK3, "stage operands share one buffer");
-    static constexpr int kOffA = 0;                                 // [digit][kAHalves]
-    static constexpr int kOffB1 = kOffA + kDigits * kAHalves * 2;    // [digit][32*32]
-    static constexpr int kOffB3 = kOffB1 + kDigits * kN1 * kK1 * 2;  // [digit][64*64]
-    static constexpr int kOffE3 = kOffB3 + kDigits * kN3 * kK3 * 2;  // int[kRows3]
+    static constexpr int kOffA = 0;                              // [digit][kABytes]
+    static constexpr int kOffB1 = kOffA + kDigits * kABytes;      // [digit][32*32]
+    static constexpr int kOffB3 = kOffB1 + kDigits * kN1 * kK1;   // [digit][64*64]
+    static constexpr int kOffE3 = kOffB3 + kDigits * kN3 * kK3;   // int[kRows3]
     static constexpr int kOffTw3 = kOffE3 + kRows3 * 4;              // float2[16][32]: W^(n2 k1)
     static constexpr int kOffBar = kOffTw3 + 16 * 32 * 8;            // uint64 mbarrier
     static constexpr int kOffTmem = kOffBar + 8;                     // uint32 tmem base
     static constexpr int kSmemBytes = kOffTmem + 8;
-    // The second stage-3 tile's MMA reads rows 128..255 of each digit plane;
-    // for the last plane those end inside B1.
-    static_assert(kTiles3 == 1 || kOffA + (kDigits - 1) * kAHalves * 2 + 256 * kK3 * 2 <= kOffB3,
-                  "stage-3 tile reads stay inside the engine's shared memory");
+    // With 6 sequences stage 1's second tile and stage 3's only one end past
+    // the operand; for the last plane those rows lie inside B1.
+    static_assert(kTiles1 == 2 && kOffA + (kDigits - 1) * kABytes + 256 * kK1 <= kOffB3 && 256 * kK1 == 128 * kK3,
+                  "tile reads stay inside the engine's shared memory");
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p)
@@ -102,6 +110,12 @@ __device__ __forceinline__ int kmajor(int row, int k, int K)
     return (row >> 3) * (K * 8) + (k >> 3) * 64 + (row & 7) * 8 + (k & 7);
 }
 
+// The same for 8-bit operands (16 of them a core-matrix row). Offset in bytes.
+__device__ __forceinline__ int kmajor8(int row, int k, int K)
+{
+    return (row >> 3) * (K * 8) + (k >> 4) * 128 + (row & 7) * 16 + (k & 15);
+}
+
 // Shared-memory matrix descriptor: start, LBO, SBO (all >> 4), version 1,
 // base offset 0, no swizzle.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo)
@@ -115,6 +129,24 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 __host__ __device__ constexpr uint32_t instr_desc(int m, int n)
 {
     return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
+}
+
+// Signed 8-bit A and B (K-major), 32-bit integer accumulator, M x N.
+__host__ __device__ constexpr uint32_t instr_desc_i8(int m, int n)
+{
+    return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
+           (static_cast<uint32_t>(m >> 4) << 24);
+}
+
+__device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n"
+        :
+        : "r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
 }
 
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
@@ -251,6 +283,60 @@ __device__ __forceinline__ void digits4f(float x, float (&t)[4])
     t[3] = nearest_half_up(x3, 1.0f);
 }
 
+// The digits of x 2^e, rounded to the nearest integer (halves up), |x 2^e| <
+// 2^30, as the four signed bytes of one word (byte 3 the leading digit d0):
+// adding 0x80 to each lower byte carries a digit above 127 into the next one,
+// and flipping the same bits leaves each byte's two's complement.
+__device__ __forceinline__ uint32_t digit_bytes(int v)
+{
+    return (static_cast<uint32_t>(v) + 0x00808080u) ^ 0x00808080u;
+}
+__device__ __forceinline__ uint32_t digit_bytes(float x, float scale)
+{
+    return digit_bytes(__float2int_rd(__fmaf_rd(x, scale, 0.5f)));
+}
+
+// Four values' digit words as one word per digit plane: p[g] holds digit g
+// of the four values, in their order.
+__device__ __forceinline__ void digit_planes(const uint32_t (&w)[4], uint32_t (&p)[4])
+{
+    const uint32_t l0 = __byte_perm(w[0], w[1], 0x5140), l1 = __byte_perm(w[2], w[3], 0x5140);
+    const uint32_t h0 = __byte_perm(w[0], w[1], 0x7362), h1 = __byte_perm(w[2], w[3], 0x7362);
+    p[3] = __byte_perm(l0, l1, 0x5410);
+    p[2] = __byte_perm(l0, l1, 0x7632);
+    p[1] = __byte_perm(h0, h1, 0x5410);
+    p[0] = __byte_perm(h0, h1, 0x7632);
+}
+
+// max(a, |x|), NaN when either is one.
+__device__ __forceinline__ float max_abs_nan(float a, float x)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(fabsf(x)));
+    return r;
+}
+
+// The exponent of a row whose magnitudes' max_abs_nan is `m`. A row that
+// holds an infinity or a NaN has no fixed-point form: its weights are NaN,
+// so that all it contributes to is NaN, as in a floating-point transform.
+constexpr int kBadRow = -1000;
+__device__ __forceinline__ int row_exp_or_bad(float m) { return m < __int_as_float(0x7f800000) ? row_exp(m) : kBadRow; }
+__device__ __forceinline__ float level_weight(int shift, int e)
+{
+    return e == kBadRow ? __int_as_float(0x7fc00000) : pow2f(shift - e);
+}
+
+// Levels L and L + 1 of a row as one integer D_L 2^8 + D_(L+1), below 2^31
+// (level L holds at most (L + 1) 64 products up to 2^14, and the leading
+// digits are at most 2^6: |D_0| <= 2^18, |D_2| < 2^21).
+__device__ __forceinline__ int level_pair(uint32_t a, uint32_t b) { return static_cast<int>((a << 8) + b); }
+// The row's value from its two pairs: hi 2^(10 - e) + lo 2^(-6 - e), two
+// roundings (hi to FP32, and the sum).
+__device__ __forceinline__ float pair_value(int hi, int lo, float whi, float wlo)
+{
+    return __fmaf_rn(__int2float_rn(lo), wlo, __fmul_rn(__int2float_rn(hi), whi));
+}
+
 // a b - c d with about one rounding (Kahan: the rounding error of c d is
 // recovered exactly by a fused multiply-add and added back). The twiddle
 // step Z = Y W uses it: rounding each product and the sum separately (three
@@ -292,10 +378,7 @@ struct Engine {
     unsigned char* smem;  // Lay::kSmemBytes, 128-byte aligned
     uint32_t tmem;        // tensor-memory base (lane 0, column 0)
 
-    __device__ uint16_t* a(int digit) const
-    {
-        return reinterpret_cast<uint16_t*>(smem + Lay::kOffA) + digit * Lay::kAHalves;
-    }
+    __device__ unsigned char* a(int digit) const { return smem + Lay::kOffA + digit * Lay::kABytes; }
     __device__ int* e3() const { return reinterpret_cast<int*>(smem + Lay::kOffE3); }
     __device__ uint32_t bar() const { return smem_u32(smem + Lay::kOffBar); }
 
@@ -315,8 +398,8 @@ struct Engine {
             if (e & 256) w = make_float2(-w.x, -w.y);
             t3[i] = w;
         }
-        uint16_t* b1 = reinterpret_cast<uint16_t*>(smem + Lay::kOffB1);
-        uint16_t* b3 = reinterpret_cast<uint16_t*>(smem + Lay::kOffB3);
+        unsigned char* b1 = smem + Lay::kOffB1;
+        unsigned char* b3 = smem + Lay::kOffB3;
         const double scale = static_cast<double>(1ll << kBExp);
         // B1[j][k]: j = (q, k1) output, k = (p, n1) input, angle 2 pi n1 k1 / 16
         for (int i = tid; i < kN1 * kK1; i += nthreads) {
@@ -325,9 +408,9 @@ struct Engine {
             double s, c;
             sincospi(static_cast<double>((n1 * k1) & 15) / 8.0, &s, &c);
             const double v = (q == p) ? c : (q == 0 ? -s : s);
-            uint16_t d[4];
-            digits4(static_cast<int>(rint(v * scale)), d);
-            for (int g = 0; g < kDigits; ++g) b1[g * kN1 * kK1 + kmajor(j, k, kK1)] = d[g];
+            const uint32_t w = digit_bytes(static_cast<int>(rint(v * scale)));
+            for (int g = 0; g < kDigits; ++g)
+                b1[g * kN1 * kK1 + kmajor8(j, k, kK1)] = static_cast<unsigned char>(w >> (24 - 8 * g));
         }
         // B3[j][k]: j = (q, k2), k = (p, n2), angle 2 pi n2 k2 / 32
         for (int i = tid; i < kN3 * kK3; i += nthreads) {
@@ -336,9 +419,9 @@ struct Engine {
             double s, c;
             sincospi(static_cast<double>((n2 * k2) & 31) / 16.0, &s, &c);
             const double v = (q == p) ? c : (q == 0 ? -s : s);
-            uint16_t d[4];
-            digits4(static_cast<int>(rint(v * scale)), d);
-            for (int g = 0; g < kDigits; ++g) b3[g * kN3 * kK3 + kmajor(j, k, kK3)] = d[g];
+            const uint32_t w = digit_bytes(static_cast<int>(rint(v * scale)));
+            for (int g = 0; g < kDigits; ++g)
+                b3[g * kN3 * kK3 + kmajor8(j, k, kK3)] = static_cast<unsigned char>(w >> (24 - 8 * g));
         }
         if (tid == 0) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar()) : "memory");
@@ -371,6 +454,7 @@ struct Engine {
 
     // The 10 digit-pair MMAs of one K step into the level accumulators at
     // `d` + 32 L (stage 1) or + 64 L (stage 3). `first` starts each level.
+    template <bool I8>
     __device__ static void issue_levels(uint32_t d, int level_stride, uint32_t a0, uint32_t b0, uint32_t a_digit,
                                         uint32_t b_digit, uint32_t kofs, uint32_t tile, uint32_t sbo_a,
                                         uint32_t sbo_b, uint32_t idesc, bool first)
@@ -384,10 +468,32 @@ struct Engine {
                 if (i >= kDigits || j >= kDigits) continue;
                 const uint64_t da = smem_desc(a0 + i * a_digit + tile + kofs, 128, sbo_a);
                 const uint64_t db = smem_desc(b0 + j * b_digit + kofs, 128, sbo_b);
-                mma_f16(d + L * level_stride, da, db, idesc, started ? 1u : 0u);
+                if constexpr (I8)
+                    mma_i8(d + L * level_stride, da, db, idesc, started ? 1u : 0u);
+                else
+                    mma_f16(d + L * level_stride, da, db, idesc, started ? 1u : 0u);
                 started = true;
             }
         }
+    }
+
+    // Sixteen values of an operand row, scaled by `sc`, as 16 bytes in each
+    // digit plane at `off` (one core-matrix row).
+    __device__ void put_digits(int off, const float* v, float sc) const
+    {
+        uint32_t p[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t w[4] = {digit_bytes(v[4 * q], sc), digit_bytes(v[4 * q + 1], sc),
+                                   digit_bytes(v[4 * q + 2], sc), digit_bytes(v[4 * q + 3], sc)};
+            uint32_t d[4];
+            digit_planes(w, d);
+#pragma unroll
+            for (int g = 0; g < kDigits; ++g) p[g][q] = d[g];
+        }
+#pragma unroll
+        for (int g = 0; g < kDigits; ++g)
+            *reinterpret_cast<uint4*>(a(g) + off) = make_uint4(p[g][0], p[g][1], p[g][2], p[g][3]);
     }
 
     // In-place inverse DFT of sequences s < count (<= SEQS) of length 512 at
@@ -398,11 +504,10 @@ struct Engine {
     {
         const int warp = tid >> 5, lane = tid & 31;
         const bool worker = tid < Lay::kThreads;
-        uint16_t* a0p = a(0);
-        // Stage-1 tile t holds sequences 4t..4t+3, stage-3 tile t sequences
-        // 8t..8t+7: tiles without sequences are skipped.
+        unsigned char* a0p = a(0);
+        // Stage-1 tile t holds sequences 4t..4t+3 (a tile without sequences is
+        // skipped), stage 3's tile all of them.
         const int tiles1 = (count + 3) / 4;
-        const int tiles3 = (count + 7) / 8;
 
         // ---- stage 1 operand: row r = (s, n2), 16 complex x[32 n1 + n2] ----
         int e1 = 0;
@@ -417,43 +522,32 @@ struct Engine {
                     const float2 x = seq[pad_idx(32 * n1 + n2)];
                     v[n1] = x.x;
                     v[16 + n1] = x.y;
-                    m = fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y)));
+                    m = max_abs_nan(max_abs_nan(m, x.x), x.y);
                 }
             } else {
 #pragma unroll
                 for (int k = 0; k < 32; ++k) v[k] = 0.0f;
             }
-            e1 = row_exp(m);
+            e1 = row_exp_or_bad(m);
             const float sc = pow2f(e1);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float d[8][4];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) digits4f(v[8 * c + q] * sc, d[q]);
-                const int off = kmajor(tid, 8 * c, kK1);
-#pragma unroll
-                for (int g = 0; g < kDigits; ++g)
-                    *reinterpret_cast<uint4*>(a0p + g * Lay::kAHalves + off) =
-                        make_uint4(half2_bits(d[0][g], d[1][g]), half2_bits(d[2][g], d[3][g]),
-                                   half2_bits(d[4][g], d[5][g]), half2_bits(d[6][g], d[7][g]));
-            }
+            for (int c = 0; c < 2; ++c) put_digits(kmajor8(tid, 16 * c, kK1), v + 16 * c, sc);
         }
         fence_proxy_async();
         fence_before_sync();
         __syncthreads();
         fence_after_sync();
 
-        // ---- stage 1 MMAs: tiles1 tiles x 2 K steps x 10 digit pairs ----
+        // ---- stage 1 MMAs: tiles1 tiles x 1 K step x 10 digit pairs ----
         if (tid == 0) {
             const uint32_t abase = smem_u32(a0p), bbase = smem_u32(smem + Lay::kOffB1);
-            constexpr uint32_t sbo = kK1 * 16;
-            constexpr uint32_t idesc = instr_desc(128, kN1);
+            constexpr uint32_t sbo = kK1 * 8;
+            constexpr uint32_t idesc = instr_desc_i8(128, kN1);
+            static_assert(kK1 == 32, "one K step");
 #pragma unroll 1
             for (int t = 0; t < tiles1; ++t)
-#pragma unroll 1
-                for (int ks = 0; ks < kK1 / 16; ++ks)
-                    issue_levels(tmem + t * 128, kN1, abase, bbase, Lay::kAHalves * 2, kN1 * kK1 * 2, ks * 256,
-                                 t * 16 * sbo, sbo, sbo, idesc, ks == 0);
+                issue_levels<true>(tmem + t * 128, kN1, abase, bbase, Lay::kABytes, kN1 * kK1, 0, t * 16 * sbo, sbo,
+                                   sbo, idesc, true);
             mma_commit(bar());
         }
         bar_wait(bar(), 0u, error);
@@ -464,15 +558,16 @@ struct Engine {
         if (worker && (warp >> 2) < tiles1) {
             const int t = warp >> 2;
             const uint32_t col = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + t * 128;
+            const float whi = level_weight(10, e1), wlo = level_weight(-6, e1);
             float y[32];
+            int hi[32];
             {
                 uint32_t r0[32], r1[32];
                 OCEAN_TMEM_LD32(col, r0);
                 OCEAN_TMEM_LD32(col + 32, r1);
                 tmem_wait_ld();
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    y[j] = level_sum(r0[j], r1[j], e1);
+                for (int j = 0; j < 32; ++j) hi[j] = level_pair(r0[j], r1[j]);
             }
             {
                 uint32_t r2[32], r3[32];
@@ -480,8 +575,7 @@ struct Engine {
                 OCEAN_TMEM_LD32(col + 96, r3);
                 tmem_wait_ld();
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    y[j] = level_add(y[j], r2[j], r3[j], e1);
+                for (int j = 0; j < 32; ++j) y[j] = pair_value(hi[j], level_pair(r2[j], r3[j]), whi, wlo);
             }
             // Z staged as FP32, stage-3 row (s, k1) at zbuf + (s * 16 + k1) *
             // kZStride, K = (p, n2), in the sequences' own buffer: every
@@ -518,27 +612,17 @@ struct Engine {
                     v[4 * q + 1] = f.y;
                     v[4 * q + 2] = f.z;
                     v[4 * q + 3] = f.w;
-                    m = fmaxf(m, fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))));
+                    m = max_abs_nan(max_abs_nan(max_abs_nan(max_abs_nan(m, f.x), f.y), f.z), f.w);
                 }
             } else {
 #pragma unroll
                 for (int k = 0; k < 32; ++k) v[k] = 0.0f;
             }
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-            const int ex3 = row_exp(m);
+            m = max_abs_nan(m, __shfl_xor_sync(0xffffffffu, m, 8));
+            const int ex3 = row_exp_or_bad(m);
             const float sc = pow2f(ex3);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float d[8][4];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) digits4f(v[8 * c + q] * sc, d[q]);
-                const int off = kmajor(row, half_k * 32 + 8 * c, kK3);
-#pragma unroll
-                for (int g = 0; g < kDigits; ++g)
-                    *reinterpret_cast<uint4*>(a0p + g * Lay::kAHalves + off) =
-                        make_uint4(half2_bits(d[0][g], d[1][g]), half2_bits(d[2][g], d[3][g]),
-                                   half2_bits(d[4][g], d[5][g]), half2_bits(d[6][g], d[7][g]));
-            }
+            for (int c = 0; c < 2; ++c) put_digits(kmajor8(row, half_k * 32 + 16 * c, kK3), v + 16 * c, sc);
             if (half_k == 0) e3()[row] = ex3;
         }
         fence_proxy_async();
@@ -546,41 +630,40 @@ struct Engine {
         __syncthreads();
         fence_after_sync();
 
-        // ---- stage 3 MMAs: tiles3 tiles x 4 K steps x 10 digit pairs ----
+        // ---- stage 3 MMAs: 2 K steps x 10 digit pairs ----
         if (tid == 0) {
             const uint32_t abase = smem_u32(a0p), bbase = smem_u32(smem + Lay::kOffB3);
-            constexpr uint32_t sbo = kK3 * 16;
-            constexpr uint32_t idesc = instr_desc(128, kN3);
+            constexpr uint32_t sbo = kK3 * 8;
+            constexpr uint32_t idesc = instr_desc_i8(128, kN3);
 #pragma unroll 1
-            for (int t = 0; t < tiles3; ++t)
-#pragma unroll 1
-                for (int ks = 0; ks < kK3 / 16; ++ks)
-                    issue_levels(tmem + t * 256, kN3, abase, bbase, Lay::kAHalves * 2, kN3 * kK3 * 2, ks * 256,
-                                 t * 16 * sbo, sbo, sbo, idesc, ks == 0);
+            for (int ks = 0; ks < kK3 / 32; ++ks)
+                issue_levels<true>(tmem, kN3, abase, bbase, Lay::kABytes, kN3 * kK3, ks * 256, 0, sbo, sbo, idesc,
+                                   ks == 0);
             mma_commit(bar());
         }
         bar_wait(bar(), 1u, error);
         fence_after_sync();
 
-        // ---- read X: row (s, k1) of stage-3 tile t in lane quadrant (row &
-        // 127) / 32, where warp w may read quadrant w & 3. Tile 0: warps 0-3
-        // take k2 < 16 and warps 4-7 k2 >= 16; tile 1 (rows 128..191, lanes
-        // 0..63): warps 8 and 9, both halves. Each reads both parts (level
-        // L's real parts in columns 256 t + 64 L + k2, imaginary ones 32
-        // further), so every output is one float2 store and a half warp
-        // writes 128 contiguous bytes ----
+        // ---- read X: row (s, k1) in lane quadrant row / 32, where warp w may
+        // read quadrant w & 3. Warps 0-3 take k2 < 16 and warps 4-7 k2 >= 16;
+        // with 6 sequences (rows in quadrants 0-2, warps 0-5) warp 2 takes
+        // both halves of its quadrant. Each reads both parts (level L's real
+        // parts in columns 64 L + k2, imaginary ones 32 further), so every
+        // output is one float2 store and a half warp writes 128 contiguous
+        // bytes ----
         if (worker) {
-            const bool second = warp >= 8;
-            const int t = second ? 1 : 0;
-            if (!second || (t < tiles3 && warp < 10)) {
-                const int row = 128 * t + 32 * (warp & 3) + lane;  // (s, k1)
+            const bool both = SEQS == 6 && warp == 2;
+            if (SEQS == 8 || warp != 3) {
+                const int row = 32 * (warp & 3) + lane;  // (s, k1)
                 const int e = e3()[row];
                 const int s = row >> 4, k1 = row & 15;
+                const float whi = level_weight(10, e), wlo = level_weight(-6, e);
                 float2* seq = data + s * seq_stride;
-                const int h0 = second ? 0 : (warp >> 2), h1 = second ? 2 : h0 + 1;
+                const int h0 = warp >> 2, h1 = both ? 2 : h0 + 1;
 #pragma unroll 1
                 for (int half = h0; half < h1; ++half) {
-                    const uint32_t col = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + 256 * t + half * 16;
+                    const uint32_t col = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + half * 16;
+                    int hr[16], hi[16];
                     float xr[16], xi[16];
                     {
                         uint32_t r0[16], i0[16], r1[16], i1[16];
@@ -591,8 +674,8 @@ struct Engine {
                         tmem_wait_ld();
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
-                            xr[j] = level_sum(r0[j], r1[j], e);
-                            xi[j] = level_sum(i0[j], i1[j], e);
+                            hr[j] = level_pair(r0[j], r1[j]);
+                            hi[j] = level_pair(i0[j], i1[j]);
                         }
                     }
                     {
@@ -604,8 +687,8 @@ struct Engine {
                         tmem_wait_ld();
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
-                            xr[j] = level_add(xr[j], r2[j], r3[j], e);
-                            xi[j] = level_add(xi[j], i2[j], i3[j], e);
+                            xr[j] = pair_value(hr[j], level_pair(r2[j], r3[j]), whi, wlo);
+                            xi[j] = pair_value(hi[j], level_pair(i2[j], i3[j]), whi, wlo);
                         }
                     }
                     if (s < count) {

@@ -187,7 +187,7 @@ struct SmallEngine {
         for (int t = 0; t < tiles; ++t)
 #pragma unroll 1
             for (int ks = 0; ks < K / 16; ++ks)
-                Engine<8>::issue_levels(tmem + t * kLevels * NO, NO, abase, bbase, Lay::kAHalves * 2, NO * K * 2,
+                Engine<8>::issue_levels<false>(tmem + t * kLevels * NO, NO, abase, bbase, Lay::kAHalves * 2, NO * K * 2,
                                         ks * 256, t * 16 * sbo, sbo, sbo, idesc, ks == 0);
         mma_commit(bar());
     }
