@@ -368,7 +368,7 @@ def bench_large_sizes(torch, frames: int = 10):
         alg = 56 * n * n  # h0 in; displacement, normal and velocity out
         res[str(n)] = {"workload": f"{count} x {n}^2, L = {0.8 * n:.0f} m, U = 15 m/s, velocity on",
                        "updates_per_s": count * 1000.0 / ms, "ms_per_frame": ms,
-                       "gpu_launches_per_frame": 3, "alg_bytes_per_update": alg,
+                       "gpu_launches_per_frame": 2, "alg_bytes_per_update": alg,
                        "achieved_gbs": alg * count / (ms / 1000.0) / 1e9}
         b.close()
     return res
@@ -931,7 +931,7 @@ def main():
     tc = None
     if args.form != "tensor":
         tc = other_form(abi.OCEAN_FFT_TENSOR,
-                        "frame_kernel, tensor form (tcgen05 four-step DFT, exact FP16 digit-slice GEMMs)")
+                        "frame_kernel, tensor form (tcgen05 four-step DFT, exact 8-bit digit-slice GEMMs)")
     precise = None
     if args.form != "precise":
         precise = other_form(abi.OCEAN_FFT_PRECISE,
@@ -947,7 +947,7 @@ def main():
             oceans_per_launch = B * args.steps / prof["frame_launches"]
             alg = ALG_BYTES_PER_CELL * CELLS * oceans_per_launch
             achieved = alg / (launch_ms / 1000.0) / 1e9
-            roof = {"bound": "hbm", "kernel": "frame_kernel (persistent: evolve + row FFT, "
+            roof = {"bound": "hbm", "kernel": "pair_frame_kernel (persistent: evolve + row FFT, "
                                               "column FFT + finalize + foam)",
                     "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "peak_kind": peak_kind, "alg_bytes_per_launch": alg, "avg_launch_ms": launch_ms,

@@ -464,7 +464,7 @@ typedef struct ocean_ensemble ocean_ensemble;
 
 /* Groups the oceans by size. Schedules of a frame: the sizes in sequence,
  * each size's persistent kernel on its own stream concurrently with SM shares
- * (by estimated or by measured cost; the three-pass schedule at N = 2048 and
+ * (by estimated or by measured cost; the two-pass schedule at N = 2048 and
  * 4096), or - when every size is 32..1024, all with the same velocity flag,
  * in an FP32 form - one persistent launch whose work queue holds every
  * size's tasks. With autotune != 0 the schedule is chosen by timing each
@@ -495,10 +495,12 @@ OCEAN_API ocean_status ocean_ensemble_synchronize(ocean_ensemble* ensemble);
 OCEAN_API ocean_status ocean_ensemble_set_schedule(ocean_ensemble* ensemble, int32_t schedule);
 /* The schedule in use: 0, 1 or 2 as above (-1 for NULL). */
 OCEAN_API int32_t ocean_ensemble_schedule(const ocean_ensemble* ensemble);
-/* With enable != 0 (the default) each update replays one CUDA graph of the
- * whole frame - the time upload, the fork onto one stream per size, every
- * size's persistent launch and the join - captured at the first update under
- * the schedule the autotuner chose; with 0, each update issues the calls. */
+/* With enable != 0 (the default) each update under the sequential or a
+ * concurrent schedule replays one CUDA graph of the whole frame - the time
+ * upload, the fork onto one stream per size, every size's persistent launch
+ * and the join - captured at the first update under the schedule in use; with
+ * 0, each update issues the calls. The one-launch schedule is one call either
+ * way. */
 OCEAN_API ocean_status ocean_ensemble_set_graph(ocean_ensemble* ensemble, int32_t enable);
 OCEAN_API ocean_status ocean_ensemble_device_buffers(const ocean_ensemble* ensemble, uint32_t index,
                                                      ocean_device_buffers* out);
@@ -739,14 +741,17 @@ OCEAN_API ocean_status ocean_batch_set_profiling(ocean_batch* batch, int32_t ena
 OCEAN_API ocean_status ocean_batch_read_profile(ocean_batch* batch, ocean_pass_profile* out);
 
 /* Task plans of the batch's persistent kernel (no reference counterpart):
- * plan 0 is the default; N = 256 and 512 also have single-row tasks (plan
+ * plan 0 is the default (with enough oceans, the register-resident frames);
+ * N = 256 and 512 also have single-row tasks (plan
  * 1), N = 1024 sequences over 64 lanes with single-row tasks (plan 1). Every
  * plan gives the same bits. plan_count is 1 or 2; set_plan returns
  * OCEAN_ERROR_INVALID_ARG for a plan the batch does not have. The ring
  * slots are how many oceans' row-pass results may be in flight: 2 or 3 (1
  * for a batch of one ocean; at most the ocean count); fewer keep a large
  * size's ring in L2, more overlap an ocean's rows with the previous ones'
- * columns; same bits. Other values return OCEAN_ERROR_INVALID_ARG.
+ * columns; same bits. (The register-resident frames run their rows a wave's
+ * worth of oceans ahead of the columns with 3, half as far with 2.) Other
+ * values return OCEAN_ERROR_INVALID_ARG.
  * The deferred publish (1) lets a CTA of the persistent kernel announce a
  * finished row task only once its next task has staged its inputs, so the
  * release does not stall it; 0 announces it before the next task. Same

@@ -19,7 +19,7 @@ bool copy_desc(const ocean_desc* src, ocean_desc& dst);
 // (src/ocean.cpp:28-59): N a power of two in [16, 4096], and so on.
 void validate(const ocean_desc& d);
 // Largest N of the persistent frame kernel (frame.cu); 2048 and 4096 run
-// the three-pass schedule of frame_large.cu.
+// the two-pass schedule of frame_large.cu.
 constexpr uint32_t kMaxPersistentSize = 1024;
 int ilog2u(uint32_t v);
 // Per-stage inverse twiddles, N - 1 entries (src/core/fft.cpp:24-33).

@@ -31,7 +31,7 @@
 //
 // What bounds it: the work around the MMAs (digits, tensor-memory reads,
 // staging) and the waits between its phases, at 12-16 warps an SM; the tensor
-// pipe is 6-9 % active. The digits as bytes of one integer (a conversion, an
+// pipe is 12 % active. The digits as bytes of one integer (a conversion, an
 // add, a flip and two byte permutes a value) took 18 FP32 and conversion
 // instructions a value as FP16 operands, whose planes were also twice as
 // large and took twice the MMAs: 16 x 512^2 with velocity 735 -> 551 us a
