@@ -1054,7 +1054,7 @@ public:
     void refresh()
     {
         cudaStream_t st = batch_.stream();
-        check(cudaMemcpyAsync(mirror_.p, batch_.disp(0), mirror_.n * sizeof(float), cudaMemcpyDeviceToHost, st), "copy");
+        check(launch_mirror(batch_.disp(0), mirror_.n / 4, reinterpret_cast<float4*>(mirror_.p), st), "mirror");
         check(cudaStreamSynchronize(st), "refresh");
     }
 

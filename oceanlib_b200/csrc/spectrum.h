@@ -236,6 +236,8 @@ cudaError_t launch_cascade_sample(const CascadeLevels& levels, const float2* xz,
                                   SurfaceEx* out, int iters, float tol, cudaStream_t stream);
 
 // RGBA32F -> RGBA16F, alpha optionally from a separate plane (pack.cu).
+// n texels to pinned host memory.
+cudaError_t launch_mirror(const float4* src, size_t n, float4* pinned, cudaStream_t st);
 cudaError_t launch_pack_rgba16(const float4* src, const float* alpha, uint64_t cells, ushort4* dst,
                                cudaStream_t st);
 
