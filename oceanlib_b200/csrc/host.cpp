@@ -1018,8 +1018,6 @@ public:
         // Displacement, normal and velocity one after the other, as the batch
         // holds them: the mirror is one copy.
         mirror_ = HostBuf<float>(cells * 4 * (batch_.velocity() ? 3 : 2));
-        q_in_ = DevBuf<float2>(1);
-        q_out_ = DevBuf<SurfaceEx>(1);
         q_host_in_ = HostBuf<float2>(1);
         q_host_out_ = HostBuf<SurfaceEx>(1);
         // The reference constructor leaves the ocean evaluated at t = 0
@@ -1063,11 +1061,10 @@ public:
         std::lock_guard<std::mutex> lock(query_mutex_);
         cudaStream_t st = batch_.stream();
         q_host_in_.p[0] = make_float2(x, z);
-        check(cudaMemcpyAsync(q_in_.p, q_host_in_.p, sizeof(float2), cudaMemcpyHostToDevice, st), "query");
+        // The kernel reads the point from pinned memory and writes the record
+        // there, without a copy on either side.
         check(launch_sample(static_cast<int>(desc_.size), inv_cell(), batch_.disp(0), batch_.normal(0),
-                            batch_.velocity_ptr(0), q_in_.p, 1, q_out_.p, st), "query kernel");
-        check(cudaMemcpyAsync(q_host_out_.p, q_out_.p, sizeof(SurfaceEx), cudaMemcpyDeviceToHost, st),
-              "query");
+                            batch_.velocity_ptr(0), q_host_in_.p, 1, q_host_out_.p, st), "query kernel");
         check(cudaStreamSynchronize(st), "query");
         *out = q_host_out_.p[0];
     }
@@ -1147,8 +1144,8 @@ private:
     double time_ = 0.0;
     HostBuf<float> mirror_;
     mutable std::mutex query_mutex_;
-    mutable DevBuf<float2> q_in_, many_in_;
-    mutable DevBuf<SurfaceEx> q_out_, many_out_;
+    mutable DevBuf<float2> many_in_;
+    mutable DevBuf<SurfaceEx> many_out_;
     mutable HostBuf<float2> q_host_in_;
     mutable HostBuf<SurfaceEx> q_host_out_;
     ocean_status last_error_ = OCEAN_OK;
