@@ -129,7 +129,7 @@ OCEAN_API double ocean_get_time(const ocean_sim* sim);
 
 /* include/ocean/ocean.h:205. The reference's 4-step fixed-point inversion,
  * run by the GPU query kernel on the device outputs (one query is a launch
- * plus a copy; use ocean_sample_many for many). */
+ * and a wait; use ocean_sample_many for many). */
 OCEAN_API float ocean_height_at(const ocean_sim* sim, float world_x, float world_z);
 
 /* include/ocean/ocean.h:215 (frozen: returned by value). */
