@@ -1370,6 +1370,17 @@ int frame_ring_slots(int log_n, int form, int slots, int count)
     return ring < count ? ring : count;
 }
 
+FrameChoice frame_choice(int log_n, int form, int count, int have)
+{
+    const int slots = std::min(count, 3);
+    const int plan = kernel_plan(log_n, form, 0, count);
+    for (int s = slots; s >= std::min(count, 2); --s) {
+        const int ring = frame_ring_slots(log_n, form, s, count);
+        if (ring <= have) return {plan, s, ring};
+    }
+    return {0, slots, slots};
+}
+
 int frame_grid(int log_n, int nf, int form, bool fuse_foam, int plan, int count, int wave, int sms)
 {
     long tasks;  // row tasks of the frame, and as many column tasks
@@ -1414,7 +1425,7 @@ bool mixed_pairs(int ar, const MixedArgs& m)
 {
     uint64_t rows = 0;
     for (int g = 0; g < m.groups; ++g) {
-        if (!pair_mixed_ok(m.g[g].log_n, ar)) return false;
+        if (!pair_mixed_ok(m.g[g].log_n, ar, m.g[g].count, m.g[g].ring)) return false;
         rows += uint64_t(m.g[g].count) * pair_mixed_tasks(m.g[g].log_n);
     }
     return rows >= 148;

@@ -426,6 +426,13 @@ __device__ __forceinline__ void mix_run(const MixedGroup& g, bool row, int ocean
 
 __host__ __device__ constexpr unsigned mix_tasks(int log_n) { return (1u << (2 * log_n)) / (8u * kMixThreads); }
 static_assert(mix_tasks(6) == MixPlan<6>::TASKS && mix_tasks(10) == MixPlan<10>::TASKS, "tasks of a size");
+// Oceans that a size's rows run ahead of its columns in the one launch.
+constexpr int mix_ahead(int log_n)
+{
+    const int tasks = static_cast<int>(mix_tasks(log_n));
+    const int wave = (148 * 3 + tasks - 1) / tasks;
+    return wave > 2 ? wave : 2;
+}
 
 template <int NF, int AR>
 __global__ void __launch_bounds__(kMixThreads, 3) pair_mixed_kernel(const __grid_constant__ MixedArgs m)
@@ -613,7 +620,12 @@ bool has_plan(int log_n, int ar)
 
 }  // namespace
 
-bool pair_mixed_ok(int log_n, int ar) { return ar != kArPrecise && log_n >= kMixMin && log_n <= kMixMax; }
+// A ring no deeper than the rows ahead would have row tasks wait for later
+// tickets.
+bool pair_mixed_ok(int log_n, int ar, int count, int ring)
+{
+    return ar != kArPrecise && log_n >= kMixMin && log_n <= kMixMax && (ring >= count || ring > mix_ahead(log_n));
+}
 
 uint32_t pair_mixed_tasks(int log_n) { return mix_tasks(log_n); }
 
@@ -627,13 +639,11 @@ cudaError_t launch_pair_mixed(int nf, int ar, MixedArgs m, int grid, cudaStream_
     m.total = 0;
     for (int i = 0; i < m.groups; ++i) {
         MixedGroup& g = m.g[i];
-        const int tasks = static_cast<int>(mix_tasks(g.log_n));
-        const int wave = (148 * 3 + tasks - 1) / tasks;
-        const int ahead = wave > 2 ? wave : 2;
+        if (!pair_mixed_ok(g.log_n, ar, g.count, g.ring)) return cudaErrorInvalidValue;
+        const int ahead = mix_ahead(g.log_n);
         g.ahead = ahead < g.count ? ahead : g.count;
-        if (g.ring < g.count && g.ring <= g.ahead) return cudaErrorInvalidValue;  // the queue would wait on later tickets
         g.first = m.total;
-        m.total += 2u * static_cast<uint32_t>(g.count) * static_cast<uint32_t>(tasks);
+        m.total += 2u * static_cast<uint32_t>(g.count) * mix_tasks(g.log_n);
     }
     return mixed_variant(nf, ar, [&](auto L) { return decltype(L)::launch(m, grid, st); });
 }

@@ -722,6 +722,7 @@ public:
     // oceans would make R(b + 1) wait for C(b), whose tickets come after it
     // in the queue: the queue is only deadlock-free from two slots up.
     int ring_slots() const { return slots_; }
+    int ring() const { return ring_; }
     int min_ring_slots() const { return std::min(max_slots_, 2); }
     void set_ring_slots(int slots)
     {
@@ -1387,6 +1388,7 @@ public:
             for (size_t g = 0; g < batches_.size(); ++g) {
                 shape.g[g].log_n = ilog2u(batches_[g]->size());
                 shape.g[g].count = static_cast<int32_t>(batches_[g]->count());
+                shape.g[g].ring = batches_[g]->ring();
             }
             const int per_sm = mixed_blocks_per_sm(batches_[0]->nf(), arith_of_form(batches_[0]->form()), shape);
             if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "mixed frame occupancy");

@@ -32,6 +32,7 @@
 #include "iwave_host.h"
 #include "ocean_host.h"
 #include "serve.h"
+#include "serve_block.h"
 #include "spectrum.h"
 
 #include <cuda_runtime.h>
@@ -39,8 +40,10 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <condition_variable>
+#include <cstdint>
 #include <cstring>
 #include <deque>
 #include <map>
@@ -149,6 +152,21 @@ struct Request {
     size_t out_offset = 0;  // float index into the batch's height block
 };
 
+// The server's stream-ordered memory pool.
+struct StreamPool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
+
+    void* alloc(size_t bytes)
+    {
+        void* p = nullptr;
+        if (cudaMallocFromPoolAsync(&p, bytes, pool, stream) == cudaSuccess) return p;
+        cudaGetLastError();  // answered here: the next launch's check must not find it
+        return nullptr;
+    }
+    void free(void* p) { cudaFreeAsync(p, stream); }
+};
+
 // Ocean sessions of one (N, velocity) share the frame kernel's twiddles,
 // intermediate ring and work-queue counters.
 struct OceanKind {
@@ -157,10 +175,10 @@ struct OceanKind {
     int log_n = 0, nf = 4;
     int wave[kMaxFramePlans] = {};  // CTAs of one wave by kernel plan
     DevBuf<float2> tw, inter;
-    // A larger ring for batches of many sessions of one kind (pool allocation,
-    // counted as staging), and its oceans.
-    float2* deep = nullptr;
-    size_t deep_slots = 0;
+    // A larger ring for batches of many sessions of one kind (counted as
+    // staging), and the fewest oceans of a ring that memory was short of.
+    PoolBlock<StreamPool> deep;
+    size_t short_of = SIZE_MAX;
     FrameQueue queue;
     size_t queue_cap = 0;
     size_t bytes = 0;
@@ -256,6 +274,7 @@ public:
         check(cudaMemPoolCreate(&pool_, &props), "cudaMemPoolCreate");
         uint64_t keep = UINT64_MAX;  // keep freed memory cached in the pool
         check(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep), "pool attribute");
+        blocks_ = {pool_, stream_};
         error_ = DevBuf<unsigned>(1);
         mix_ticket_ = FrameQueue(0, stream_);
         check(cudaMemsetAsync(error_.p, 0, sizeof(unsigned), stream_), "memset");
@@ -290,7 +309,7 @@ public:
         for (auto& kv : sessions_)
             if (kv.second->block) cudaFreeAsync(kv.second->block, stream_);
         for (auto& k : ocean_kinds_)
-            if (k->deep) cudaFreeAsync(k->deep, stream_);
+            k->deep.release(blocks_);
         for (auto& c : ctxs_) {
             if (c->dev) cudaFreeAsync(c->dev, stream_);
             if (c->start) cudaEventDestroy(c->start);
@@ -804,21 +823,28 @@ private:
         }
     }
 
-    // The intermediate for a batch of `count` oceans that uses `slots` of them.
-    float2* ring_for(OceanKind* k, size_t slots)
+    // The intermediate for a batch that would use `slots` oceans of it, and the
+    // oceans it holds: the kind's three where memory is short of a larger ring
+    // (the frame then takes the kernel of three slots).
+    struct Ring {
+        float2* inter;
+        int slots;
+    };
+    Ring ring_for(OceanKind* k, size_t slots)
     {
-        if (slots <= 3) return k->inter.p;
-        if (slots > k->deep_slots) {
-            const size_t ocean = static_cast<size_t>(k->n) * k->n * k->nf * sizeof(float2);
-            const size_t grown = std::max(slots, 2 * k->deep_slots);
-            if (k->deep) check(cudaFreeAsync(k->deep, stream_), "free ring");
-            k->deep = nullptr;
-            check(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&k->deep), grown * ocean, pool_, stream_), "ring");
+        if (slots <= 3) return {k->inter.p, 3};
+        const size_t ocean = static_cast<size_t>(k->n) * k->n * k->nf * sizeof(float2);
+        const size_t had = k->deep.bytes();
+        // Memory that was short is not asked for again until a session closes (launch()).
+        if (slots * ocean > had && slots < k->short_of) {
+            const size_t most = static_cast<size_t>(frame_ring_slots(k->log_n, desc_.fft_form, 3, INT_MAX));
+            const size_t grown = std::min(most * ocean, std::max(slots * ocean, 2 * had));
+            if (!k->deep.reserve(blocks_, slots * ocean, grown)) k->short_of = slots;
             std::lock_guard<std::mutex> lk(mu_);
-            staging_bytes_ += (grown - k->deep_slots) * ocean;
-            k->deep_slots = grown;
+            staging_bytes_ += k->deep.bytes() - had;
         }
-        return k->deep;
+        if (k->deep.get() == nullptr) return {k->inter.p, 3};
+        return {static_cast<float2*>(k->deep.get()), static_cast<int>(k->deep.bytes() / ocean)};
     }
 
     void ensure_queue(OceanKind* k, size_t count)
@@ -969,8 +995,10 @@ private:
                 g.clear_words = set.words;
                 g.count = count;
                 g.slots = std::min(count, 3);
-                g.ring = frame_ring_slots(k->log_n, desc_.fft_form, g.slots, count);
-                g.a.inter = ring_for(k, static_cast<size_t>(g.ring));
+                const int want = frame_ring_slots(k->log_n, desc_.fft_form, g.slots, count);
+                const Ring ring = ring_for(k, static_cast<size_t>(want));
+                g.ring = std::min(want, ring.slots);
+                g.a.inter = ring.inter;
                 g.log_n = k->log_n;
                 continue;
             }
@@ -982,13 +1010,17 @@ private:
             q.clear_words = set.words;
             q.error = error_.p;
             q.count = count;
-            q.slots = std::min(count, 3);
             q.wait_ns = 1000000000ull;
             q.defer = k->nf == 6 ? 1 : 0;
-            const int plan = kernel_plan(k->log_n, desc_.fft_form, 0, count);
-            a.inter = ring_for(k, static_cast<size_t>(frame_ring_slots(k->log_n, desc_.fft_form, q.slots, count)));
-            const int grid = frame_grid(k->log_n, k->nf, desc_.fft_form, false, plan, count, k->wave[plan], sms_);
-            check(launch_frame(k->log_n, k->nf, desc_.fft_form, false, a, q, grid, stream_, plan), "frame kernel");
+            const int want = frame_ring_slots(k->log_n, desc_.fft_form, std::min(count, 3), count);
+            const Ring ring = ring_for(k, static_cast<size_t>(want));
+            const FrameChoice choice = frame_choice(k->log_n, desc_.fft_form, count, ring.slots);
+            q.slots = choice.slots;
+            a.inter = ring.inter;
+            const int grid = frame_grid(k->log_n, k->nf, desc_.fft_form, false, choice.plan, count,
+                                        k->wave[choice.plan], sms_);
+            check(launch_frame(k->log_n, k->nf, desc_.fft_form, false, a, q, grid, stream_, choice.plan),
+                  "frame kernel");
             k->queue.launched(set);
             ++kernels;
         }
@@ -1064,6 +1096,8 @@ private:
             if (s->block) check(cudaFreeAsync(s->block, stream_), "free session");
             s->block = nullptr;
         }
+        if (!c->closes.empty())
+            for (auto& k : ocean_kinds_) k->short_of = SIZE_MAX;
         c->points = plan.points;
         c->kernels = kernels;
     }
@@ -1282,6 +1316,7 @@ private:
     cudaStream_t stream_ = nullptr, field_stream_ = nullptr;
     cudaEvent_t uploaded_ = nullptr, fields_done_ = nullptr;  // a batch's fork and join
     cudaMemPool_t pool_ = nullptr;
+    StreamPool blocks_;  // pool_ on stream_
     DevBuf<unsigned> error_;
     FrameQueue mix_ticket_;  // the one-launch frame's ticket
     int mix_wave_[2][2] = {};      // its CTAs of one wave, by kernel and field count (4, 6)

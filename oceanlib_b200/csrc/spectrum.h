@@ -115,6 +115,14 @@ int kernel_plan(int log_n, int form, int plan, int count);
 // Ocean slots of `inter` that launches of up to `count` oceans with
 // q.slots <= slots use, whatever the plan.
 int frame_ring_slots(int log_n, int form, int slots, int count);
+// How to launch `count` oceans (plan 0) where `inter` holds `have` of them, at
+// least min(count, 3): the kernel plan, QueueArgs::slots, and the oceans of
+// `inter` it uses. A ring too short for all its rows ahead runs half of them
+// if that fits, else the kernel of three slots.
+struct FrameChoice {
+    int plan, slots, ring;
+};
+FrameChoice frame_choice(int log_n, int form, int count, int have);
 // CTAs to launch a frame of `count` oceans with, of the `wave` that are resident
 // on `sms` SMs: no more per SM than it takes to hand every SM its even share of
 // the row tasks. (All CTAs of a wave draw their tickets at once, so with more of
@@ -167,14 +175,14 @@ struct MixedArgs {
     int32_t defer;        // as QueueArgs::defer, for every group
 };
 bool mixed_size_ok(int log_n);
-// Whether these groups (log_n, count) run in this arithmetic as register-resident
-// tasks (frame_pairs.cu: sizes from 64 on, FP32 forms, enough row tasks to give
-// every SM one) or as frame.cu's; the launch's
-// resident CTAs per SM; and the launch, with the CTAs of one wave.
+// Whether these groups (log_n, count, ring) run in this arithmetic as register-
+// resident tasks (frame_pairs.cu: sizes from 64 on, FP32 forms, rings that hold
+// the rows ahead, enough row tasks to give every SM one) or as frame.cu's; the
+// launch's resident CTAs per SM; and the launch, with the CTAs of one wave.
 bool mixed_pairs(int ar, const MixedArgs& m);
 int mixed_blocks_per_sm(int nf, int ar, const MixedArgs& m);
 cudaError_t launch_mixed_frame(int nf, int ar, const MixedArgs& m, int wave, cudaStream_t stream);
-bool pair_mixed_ok(int log_n, int ar);
+bool pair_mixed_ok(int log_n, int ar, int count, int ring);
 uint32_t pair_mixed_tasks(int log_n);  // row tasks of an ocean
 int pair_mixed_blocks_per_sm(int nf, int ar);
 cudaError_t launch_pair_mixed(int nf, int ar, MixedArgs m, int grid, cudaStream_t stream);
