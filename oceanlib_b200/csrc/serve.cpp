@@ -224,8 +224,7 @@ struct Session {
 struct BatchCtx {
     HostBuf<unsigned char> host_in;
     size_t host_in_cap = 0;
-    unsigned char* dev = nullptr;  // pool allocation: inputs, then heights
-    size_t dev_cap = 0;
+    PoolBlock<StreamPool> dev;     // inputs, then heights
     HostBuf<float> host_out;       // heights + the error word
     size_t host_out_cap = 0;       // floats
     cudaEvent_t start = nullptr, done = nullptr;
@@ -311,7 +310,7 @@ public:
         for (auto& k : ocean_kinds_)
             k->deep.release(blocks_);
         for (auto& c : ctxs_) {
-            if (c->dev) cudaFreeAsync(c->dev, stream_);
+            c->dev.release(blocks_);
             if (c->start) cudaEventDestroy(c->start);
             if (c->done) cudaEventDestroy(c->done);
         }
@@ -812,14 +811,14 @@ private:
             ++staging_growths_;
         }
         const size_t dev_bytes = in_bytes + round_up(out_floats * sizeof(float), 16);
-        if (dev_bytes > c->dev_cap) {
-            const size_t cap = std::max(dev_bytes, c->dev_cap * 2);
-            if (c->dev) check(cudaFreeAsync(c->dev, stream_), "free staging");
-            c->dev = nullptr;
-            check(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&c->dev), cap, pool_, stream_), "staging");
-            std::lock_guard<std::mutex> lk(mu_);
-            staging_bytes_ += cap - c->dev_cap;  // reported, not part of the session budget
-            c->dev_cap = cap;
+        const size_t had = c->dev.bytes();
+        if (dev_bytes > had) {
+            const bool ok = c->dev.reserve(blocks_, dev_bytes, 2 * had);
+            {
+                std::lock_guard<std::mutex> lk(mu_);
+                staging_bytes_ += c->dev.bytes() - had;  // reported, not part of the session budget
+            }
+            if (!ok) throw DeviceError(cudaErrorMemoryAllocation, "staging");
         }
     }
 
@@ -896,7 +895,7 @@ private:
         for (auto& p : oparts) ensure_queue(p.k, p.count);
 
         unsigned char* h = c->host_in.p;
-        unsigned char* d = c->dev;
+        unsigned char* d = static_cast<unsigned char*>(c->dev.get());
         float* dev_heights = reinterpret_cast<float*>(d + in_bytes);
 
         // Fill the block.
