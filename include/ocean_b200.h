@@ -626,7 +626,7 @@ typedef struct ocean_server_stats {
     uint64_t sessions_active;
     uint64_t sessions_waiting;
     uint64_t sessions_closed;
-    uint64_t bytes_in_use;        /* admitted sessions plus shared tables and staging */
+    uint64_t bytes_in_use;        /* admitted sessions plus shared tables */
     uint64_t hbm_budget;
     uint64_t requests_submitted;
     uint64_t requests_completed;
@@ -636,7 +636,8 @@ typedef struct ocean_server_stats {
     uint64_t query_points_completed;
     uint64_t batches;             /* batches launched */
     uint64_t kernel_launches;     /* kernels those batches launched */
-    uint64_t bytes_staging;       /* per-batch device staging (outside the budget) */
+    uint64_t bytes_staging;       /* per-batch device staging (outside the budget) and larger
+                                     intermediate rings (only where sessions leave room in it) */
     double   mean_batch_requests;
     double   latency_p50_ms;      /* submit -> result ready (host clock), all requests */
     double   latency_p99_ms;
@@ -648,7 +649,7 @@ typedef struct ocean_server_stats {
     double   gpu_busy_ms;         /* summed device time of the batches (CUDA events) */
     double   wall_ms;             /* since creation or the last reset */
     double   dispatch_max_ms;     /* longest single host step of the dispatcher */
-    uint64_t staging_growths;     /* staging buffers grown past their reserve */
+    uint64_t staging_growths;     /* pinned staging buffers grown past their reserve */
 } ocean_server_stats;
 
 OCEAN_API void ocean_server_desc_init(ocean_server_desc* desc);

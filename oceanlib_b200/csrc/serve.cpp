@@ -24,7 +24,9 @@
 // kernels, same per-cell order), so a result is the same alone and in any
 // mix. Session memory comes from a stream-ordered pool: a session is
 // admitted when its bytes fit in the budget (FIFO), and a closed session's
-// memory is released behind the last batch that used it.
+// memory is released behind the last batch that used it. What the sessions
+// leave of the budget may hold larger intermediate rings, which make frames of
+// many sessions faster; they make way for sessions.
 
 #include "../../include/ocean_b200.h"
 #include "host_util.h"
@@ -175,8 +177,9 @@ struct OceanKind {
     int log_n = 0, nf = 4;
     int wave[kMaxFramePlans] = {};  // CTAs of one wave by kernel plan
     DevBuf<float2> tw, inter;
-    // A larger ring for batches of many sessions of one kind (counted as
-    // staging), and the fewest oceans of a ring that memory was short of.
+    // A larger ring for batches of many sessions of one kind, as far as the
+    // budget has room beside the sessions (ring_bytes_), and the fewest oceans
+    // of a ring that memory was short of.
     PoolBlock<StreamPool> deep;
     size_t short_of = SIZE_MAX;
     FrameQueue queue;
@@ -484,7 +487,7 @@ public:
             o->query_points_completed = points_done_;
             o->batches = batches_;
             o->kernel_launches = kernels_;
-            o->bytes_staging = staging_bytes_;
+            o->bytes_staging = staging_bytes_ + ring_bytes_;
             o->mean_batch_requests = batches_ ? static_cast<double>(batched_requests_) / batches_ : 0.0;
             o->gpu_busy_ms = gpu_ms_;
             o->wall_ms = ms_between(stats_t0_, Clock::now());
@@ -641,6 +644,24 @@ private:
         if (s->fk && !s->fk->reserved)
             cost += 2 * round_up(static_cast<size_t>(s->fd.size) * s->fd.size * sizeof(float), kAlign);
         return cost;
+    }
+
+    // Dispatcher thread, under the lock: the larger rings make way for the
+    // sessions just picked (their freed blocks go back to the pool that the
+    // sessions come from, behind the last batch that used them).
+    void trim_rings_locked()
+    {
+        for (auto& k : ocean_kinds_) {
+            if (in_use_ + ring_bytes_ <= desc_.hbm_budget) return;
+            ring_bytes_ -= k->deep.bytes();
+            k->deep.release(blocks_);
+        }
+    }
+
+    // Memory came back: a ring that was too large may fit now.
+    void forget_short_rings()
+    {
+        for (auto& k : ocean_kinds_) k->short_of = SIZE_MAX;
     }
 
     // Outside the lock: allocate and build each admitted session.
@@ -834,13 +855,16 @@ private:
         if (slots <= 3) return {k->inter.p, 3};
         const size_t ocean = static_cast<size_t>(k->n) * k->n * k->nf * sizeof(float2);
         const size_t had = k->deep.bytes();
-        // Memory that was short is not asked for again until a session closes (launch()).
-        if (slots * ocean > had && slots < k->short_of) {
-            const size_t most = static_cast<size_t>(frame_ring_slots(k->log_n, desc_.fft_form, 3, INT_MAX));
-            const size_t grown = std::min(most * ocean, std::max(slots * ocean, 2 * had));
-            if (!k->deep.reserve(blocks_, slots * ocean, grown)) k->short_of = slots;
+        const size_t want = slots * ocean;
+        // Memory that was short is not asked for again until a session closes.
+        if (want > had && slots < k->short_of) {
             std::lock_guard<std::mutex> lk(mu_);
-            staging_bytes_ += k->deep.bytes() - had;
+            const size_t others = in_use_ + ring_bytes_ - had;
+            const size_t room = desc_.hbm_budget > others ? desc_.hbm_budget - others : 0;
+            const size_t most = ocean * static_cast<size_t>(frame_ring_slots(k->log_n, desc_.fft_form, 3, INT_MAX));
+            if (want > room || !k->deep.reserve(blocks_, want, std::min({most, room, std::max(want, 2 * had)})))
+                k->short_of = slots;
+            ring_bytes_ += k->deep.bytes() - had;
         }
         if (k->deep.get() == nullptr) return {k->inter.p, 3};
         return {static_cast<float2*>(k->deep.get()), static_cast<int>(k->deep.bytes() / ocean)};
@@ -994,10 +1018,7 @@ private:
                 g.clear_words = set.words;
                 g.count = count;
                 g.slots = std::min(count, 3);
-                const int want = frame_ring_slots(k->log_n, desc_.fft_form, g.slots, count);
-                const Ring ring = ring_for(k, static_cast<size_t>(want));
-                g.ring = std::min(want, ring.slots);
-                g.a.inter = ring.inter;
+                g.ring = frame_ring_slots(k->log_n, desc_.fft_form, g.slots, count);
                 g.log_n = k->log_n;
                 continue;
             }
@@ -1024,6 +1045,15 @@ private:
             ++kernels;
         }
         if (one_launch) {
+            // The larger rings where the register-resident tasks would use them.
+            const int ar = arith_of_form(desc_.fft_form);
+            if (mixed_pairs(ar, m)) {
+                for (int i = 0; i < m.groups; ++i) {
+                    const Ring ring = ring_for(oparts[i].k, static_cast<size_t>(m.g[i].ring));
+                    m.g[i].ring = std::min(m.g[i].ring, ring.slots);
+                    m.g[i].a.inter = ring.inter;
+                }
+            }
             // Largest sizes first, so the short tasks fill the wave's tail.
             std::sort(m.g, m.g + m.groups, [](const MixedGroup& x, const MixedGroup& y) { return x.log_n > y.log_n; });
             const FrameQueue::Set ticket = mix_ticket_.take(stream_);
@@ -1033,7 +1063,6 @@ private:
             m.wait_ns = 1000000000ull;
             const int nf = oparts[0].k->nf;
             m.defer = nf == 6 ? 1 : 0;
-            const int ar = arith_of_form(desc_.fft_form);
             int& wave = mix_wave_[mixed_pairs(ar, m) ? 1 : 0][nf == 6 ? 1 : 0];
             if (wave == 0) {
                 const int per_sm = mixed_blocks_per_sm(nf, ar, m);
@@ -1095,8 +1124,6 @@ private:
             if (s->block) check(cudaFreeAsync(s->block, stream_), "free session");
             s->block = nullptr;
         }
-        if (!c->closes.empty())
-            for (auto& k : ocean_kinds_) k->short_of = SIZE_MAX;
         c->points = plan.points;
         c->kernels = kernels;
     }
@@ -1145,6 +1172,7 @@ private:
             s->state = OCEAN_SESSION_CLOSED;
             in_use_ -= s->bytes;
         }
+        if (!c->closes.empty()) forget_short_rings();
         c->requests.clear();
         c->closes.clear();
         c->complete = false;
@@ -1210,6 +1238,7 @@ private:
             // 2. Admissions.
             std::vector<Session*> admits = pick_admissions_locked();
             if (!admits.empty()) {
+                trim_rings_locked();
                 lk.unlock();
                 std::vector<bool> ok(admits.size(), true);
                 for (size_t i = 0; i < admits.size(); ++i) {
@@ -1224,6 +1253,7 @@ private:
                     Session* s = admits[i];
                     if (!ok[i]) {
                         in_use_ -= s->bytes;
+                        forget_short_rings();
                         s->state = OCEAN_SESSION_CLOSED;
                         fail_queue_locked(s);
                         continue;
@@ -1337,6 +1367,7 @@ private:
     uint64_t next_session_ = 1, next_ticket_ = 1;
     size_t in_use_ = 0;        // sessions and their shared tables (the budgeted bytes)
     size_t staging_bytes_ = 0; // per-batch device staging
+    size_t ring_bytes_ = 0;    // the kinds' larger rings
     uint64_t staging_growths_ = 0;
     double dispatch_max_ms_ = 0.0;  // longest host step of the dispatcher (launch or finish)
     // statistics
