@@ -35,6 +35,7 @@
 #include "ocean_host.h"
 #include "serve.h"
 #include "serve_block.h"
+#include "serve_poll.h"
 #include "spectrum.h"
 
 #include <cuda_runtime.h>
@@ -1201,16 +1202,8 @@ private:
     void poll_front(std::unique_lock<std::mutex>& lk)
     {
         BatchCtx* c = inflight_.front();
-        poked_.store(false, std::memory_order_relaxed);  // under the lock: what came before has been looked at
-        lk.unlock();
         cudaError_t e = cudaErrorNotReady;
-        while (!poked_.load(std::memory_order_acquire)) {
-            e = cudaEventQuery(c->done);
-            if (e != cudaErrorNotReady) break;
-            std::this_thread::yield();
-        }
-        lk.lock();
-        if (e != cudaErrorNotReady) {
+        if (watch_batch(lk, poked_, [&] { return (e = cudaEventQuery(c->done)) != cudaErrorNotReady; })) {
             c->complete = true;
             if (e != cudaSuccess) c->failed = true;
         }
