@@ -40,6 +40,8 @@
 
 #include <cuda_runtime.h>
 
+#include <sys/prctl.h>
+
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -1195,7 +1197,8 @@ private:
         cv_.notify_all();
     }
 
-    // While a batch is in flight: watches for its end, or for new work. A host
+    // While a batch is in flight: watches for its end, or for new work, closely
+    // (a core at work) unless the batch is a long one (serve_poll.h). A host
     // callback in the stream instead held the next batch back until it had run
     // (it takes the server's lock) and woke this thread through the scheduler,
     // twice per batch; 32 sessions' update and query a tick 1.6 -> 0.88 ms.
@@ -1203,7 +1206,7 @@ private:
     {
         BatchCtx* c = inflight_.front();
         cudaError_t e = cudaErrorNotReady;
-        if (watch_batch(lk, poked_, [&] { return (e = cudaEventQuery(c->done)) != cudaErrorNotReady; })) {
+        if (watch_batch(lk, cv_, poked_, front_since_, [&] { return (e = cudaEventQuery(c->done)) != cudaErrorNotReady; })) {
             c->complete = true;
             if (e != cudaSuccess) c->failed = true;
         }
@@ -1212,12 +1215,14 @@ private:
     void run()
     {
         cudaSetDevice(device_);  // the dispatcher issues every launch on the server's device
+        prctl(PR_SET_TIMERSLACK, 1000ul);  // (this thread's) pauses of some 30 us end on time, not 50 us late
         std::unique_lock<std::mutex> lk(mu_);
         while (true) {
             // 1. Completed batches, in launch order.
             while (!inflight_.empty() && inflight_.front()->complete) {
                 BatchCtx* c = inflight_.front();
                 inflight_.pop_front();
+                front_since_ = Clock::now();
                 lk.unlock();
                 const auto t_finish = Clock::now();
                 finish(c);
@@ -1280,6 +1285,7 @@ private:
                         ++batches_;
                         kernels_ += c->kernels;
                         batched_requests_ += c->requests.size();
+                        if (inflight_.empty()) front_since_ = t_launch;
                         inflight_.push_back(c);
                     } else {
                         // Whatever of it was queued may still use its staging.
@@ -1344,6 +1350,7 @@ private:
     int mix_wave_[2][2] = {};      // its CTAs of one wave, by kernel and field count (4, 6)
     std::vector<std::unique_ptr<BatchCtx>> ctxs_;
     std::deque<BatchCtx*> free_ctx_, inflight_;
+    Clock::time_point front_since_;  // inflight_.front() was launched, or the one before it ended
     std::vector<std::unique_ptr<OceanKind>> ocean_kinds_;
     std::vector<std::unique_ptr<FieldKind>> field_kinds_;
 
