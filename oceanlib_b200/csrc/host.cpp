@@ -1390,6 +1390,7 @@ public:
                 shape.g[g].count = static_cast<int32_t>(batches_[g]->count());
                 shape.g[g].ring = batches_[g]->ring();
             }
+            mix_pairs_ = mixed_pairs(arith_of_form(batches_[0]->form()), shape);
             const int per_sm = mixed_blocks_per_sm(batches_[0]->nf(), arith_of_form(batches_[0]->form()), shape);
             if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "mixed frame occupancy");
             mix_grid_ = per_sm * sms;
@@ -1542,7 +1543,11 @@ private:
     {
         MixedArgs m{};
         m.groups = static_cast<int32_t>(mix_order_.size());
-        for (size_t k = 0; k < mix_order_.size(); ++k) m.g[k] = batches_[mix_order_[k]]->mixed_group(t_over_2pi, st);
+        for (size_t k = 0; k < mix_order_.size(); ++k) {
+            Batch& b = *batches_[mix_order_[k]];
+            m.g[k] = b.mixed_group(t_over_2pi, st);
+            if (mixed_shallow_) m.g[k].slots = b.min_ring_slots();
+        }
         const FrameQueue::Set ticket = mix_ticket_.take(st);
         m.ticket = ticket.ticket;
         m.clear_ticket = ticket.clear;
@@ -1638,26 +1643,21 @@ private:
         apply_shares(alone);
         const double t_meas = time_frames(frames, [&](double t) { update(t, stream_); });
         double t_mixed = -1.0;
-        std::vector<int> kept;  // each size's ring depth from its own tuning
         if (mixed_ok_) {
             mixed_ = true;
             t_mixed = time_frames(frames, [&](double t) { update(t, stream_); });
             // The one launch again with every group at its shallowest ring:
-            // all sizes' intermediates share L2 in this schedule.
+            // all sizes' intermediates share L2 in this schedule. (Register-
+            // resident tasks have the one depth of the launch.)
             bool shallower = false;
-            for (auto& b : batches_) {
-                kept.push_back(b->ring_slots());
-                shallower = shallower || b->ring_slots() > b->min_ring_slots();
-            }
-            if (shallower) {
-                for (auto& b : batches_) b->set_ring_slots(b->min_ring_slots());
+            for (auto& b : batches_) shallower = shallower || b->ring_slots() > b->min_ring_slots();
+            if (shallower && !mix_pairs_) {
+                mixed_shallow_ = true;
                 const double t2 = time_frames(frames, [&](double t) { update(t, stream_); });
-                if (t2 < t_mixed) {
+                if (t2 < t_mixed)
                     t_mixed = t2;
-                    mixed_shallow_ = true;
-                } else {
-                    for (size_t g = 0; g < batches_.size(); ++g) batches_[g]->set_ring_slots(kept[g]);
-                }
+                else
+                    mixed_shallow_ = false;
             }
             // And with the other publish timing.
             mix_defer_ = !mix_defer_;
@@ -1677,11 +1677,6 @@ private:
         // more than 3 % faster.
         const double other = std::min(t_seq, std::min(t_work, t_meas));
         const bool mixed_wins = t_mixed >= 0.0 && t_mixed <= 1.03 * other;
-        if (!mixed_wins && mixed_shallow_) {
-            // The shallow rings were for the one launch only.
-            for (size_t g = 0; g < batches_.size(); ++g) batches_[g]->set_ring_slots(kept[g]);
-            mixed_shallow_ = false;
-        }
         if (mixed_wins) {
             mixed_ = true;
             concurrent_ = false;
@@ -1719,6 +1714,7 @@ private:
     // the mixed-size launch
     bool mixed_ok_ = false;
     bool mixed_ = false;
+    bool mix_pairs_ = false;      // the one launch runs register-resident tasks
     bool mixed_shallow_ = false;  // the one launch timed fastest with the shallowest rings
     bool mix_defer_ = false;      // MixedArgs::defer (default: with velocity)
     int mix_grid_ = 0;            // CTAs of one wave
