@@ -1285,12 +1285,17 @@ auto with_arith(int ar, Fn&& fn)
 template <int LOG_N, int V, typename Fn>
 auto frame_variant_plan(int nf, int ar, bool foam, Fn&& fn)
 {
-    return with_arith(ar, [&](auto A) {
+    const auto in_arith = [&](auto A) {
         constexpr int AR = decltype(A)::value;
         if (nf == 4) return fn(FrameLaunch<LOG_N, 4, AR, false, false, V>{});
         if (foam) return fn(FrameLaunch<LOG_N, 6, AR, true, false, V>{});
         return fn(FrameLaunch<LOG_N, 6, AR, false, false, V>{});
-    });
+    };
+    if constexpr (LOG_N == 10 && V == 0) {
+        return in_arith(std::integral_constant<int, kArPrecise>{});  // (frame_kernel_ok)
+    } else {
+        return with_arith(ar, in_arith);
+    }
 }
 
 template <int LOG_N, typename Fn>
@@ -1355,6 +1360,14 @@ int frame_plan_count(int log_n, int form)
     return (form != 2 && log_n >= 8) ? 2 : 1;
 }
 
+// Whether frame_kernel has this task plan. The FP32 forms run 1024^2 under plan
+// 0 as the register-resident frame at every count (pair_frame_ok).
+static bool frame_kernel_ok(int log_n, int form, int plan)
+{
+    if (log_n == 10 && plan == 0 && arith_of_form(form) != kArPrecise) return false;
+    return plan >= 0 && plan < frame_plan_count(log_n, form);
+}
+
 int kernel_plan(int log_n, int form, int plan, int count)
 {
     return plan == 0 && form != 2 && pair_frame_ok(log_n, arith_of_form(form), count) ? kPairPlan : plan;
@@ -1387,7 +1400,7 @@ int frame_grid(int log_n, int nf, int form, bool fuse_foam, int plan, int count,
     if (plan == kPairPlan) {
         tasks = static_cast<long>(count) * pair_frame_tasks(log_n, arith_of_form(form), fuse_foam);
     } else {
-        if (plan < 0 || plan >= frame_plan_count(log_n, form)) return 0;
+        if (!frame_kernel_ok(log_n, form, plan)) return 0;
         tasks = static_cast<long>(count) *
                 frame_dispatch(log_n, nf, form, fuse_foam, plan, [](auto L) { return decltype(L)::P::RT; });
     }
@@ -1400,7 +1413,7 @@ int frame_blocks_per_sm(int log_n, int nf, int form, bool fuse_foam, int plan)
     if (log_n < 4 || log_n > 10) return 0;
     if (form == 2 && (log_n < 6 || log_n > 9)) return 0;
     if (plan == kPairPlan) return form == 2 ? 0 : pair_frame_blocks_per_sm(log_n, nf, arith_of_form(form), fuse_foam);
-    if (plan < 0 || plan >= frame_plan_count(log_n, form)) return 0;
+    if (!frame_kernel_ok(log_n, form, plan)) return 0;
     return frame_dispatch(log_n, nf, form, fuse_foam, plan, [](auto L) { return decltype(L)::blocks_per_sm(); });
 }
 
@@ -1413,7 +1426,7 @@ cudaError_t launch_frame(int log_n, int nf, int form, bool fuse_foam, const Fram
         if (form == 2) return cudaErrorInvalidValue;
         return launch_pair_frame(log_n, nf, arith_of_form(form), fuse_foam, a, q, grid, st);
     }
-    if (plan < 0 || plan >= frame_plan_count(log_n, form)) return cudaErrorInvalidValue;
+    if (!frame_kernel_ok(log_n, form, plan)) return cudaErrorInvalidValue;
     return frame_dispatch(log_n, nf, form, fuse_foam, plan,
                           [&](auto L) { return decltype(L)::launch(a, q, grid, st); });
 }

@@ -672,6 +672,9 @@ bool pair_frame_ok(int log_n, int ar, int count)
     return count >= (log_n >= 10 ? 1 : log_n == 9 ? 2 : 4);
 }
 
+// 1024^2 in the FP32 forms has no other kernel for a ring of three.
+static_assert(PairPlan<10, kArExact, false>::ring(2) <= 3 && PairPlan<10, kArExact, true>::ring(2) <= 3);
+
 int pair_frame_ring(int log_n, int ar, int slots)
 {
     if (!has_plan(log_n, ar)) return 0;
