@@ -1287,15 +1287,15 @@ auto frame_variant_plan(int nf, int ar, bool foam, Fn&& fn)
 {
     const auto in_arith = [&](auto A) {
         constexpr int AR = decltype(A)::value;
-        if (nf == 4) return fn(FrameLaunch<LOG_N, 4, AR, false, false, V>{});
-        if (foam) return fn(FrameLaunch<LOG_N, 6, AR, true, false, V>{});
-        return fn(FrameLaunch<LOG_N, 6, AR, false, false, V>{});
+        if constexpr (LOG_N == 10 && V == 0 && AR != kArPrecise) {
+            return fn(FrameLaunch<LOG_N, 6, AR, true, false, V>{});  // with foam only (frame_kernel_ok)
+        } else {
+            if (nf == 4) return fn(FrameLaunch<LOG_N, 4, AR, false, false, V>{});
+            if (foam) return fn(FrameLaunch<LOG_N, 6, AR, true, false, V>{});
+            return fn(FrameLaunch<LOG_N, 6, AR, false, false, V>{});
+        }
     };
-    if constexpr (LOG_N == 10 && V == 0) {
-        return in_arith(std::integral_constant<int, kArPrecise>{});  // (frame_kernel_ok)
-    } else {
-        return with_arith(ar, in_arith);
-    }
+    return with_arith(ar, in_arith);
 }
 
 template <int LOG_N, typename Fn>
@@ -1360,36 +1360,38 @@ int frame_plan_count(int log_n, int form)
     return (form != 2 && log_n >= 8) ? 2 : 1;
 }
 
-// Whether frame_kernel has this task plan. The FP32 forms run 1024^2 under plan
-// 0 as the register-resident frame at every count (pair_frame_ok).
-static bool frame_kernel_ok(int log_n, int form, int plan)
+// Whether frame_kernel has this task plan. Without foam the FP32 forms run
+// 1024^2 under plan 0 as the register-resident frame at every count.
+static bool frame_kernel_ok(int log_n, int form, bool foam, int plan)
 {
-    if (log_n == 10 && plan == 0 && arith_of_form(form) != kArPrecise) return false;
+    if (log_n == 10 && plan == 0 && !foam && arith_of_form(form) != kArPrecise) return false;
     return plan >= 0 && plan < frame_plan_count(log_n, form);
 }
 
-int kernel_plan(int log_n, int form, int plan, int count)
+int kernel_plan(int log_n, int nf, int form, bool fuse_foam, int plan, int count)
 {
-    return plan == 0 && form != 2 && pair_frame_ok(log_n, arith_of_form(form), count) ? kPairPlan : plan;
+    return plan == 0 && form != 2 && pair_frame_ok(log_n, arith_of_form(form), nf, fuse_foam, count) ? kPairPlan : plan;
 }
 
-int frame_ring_slots(int log_n, int form, int slots, int count)
+int frame_ring_slots(int log_n, int nf, int form, int slots, int count)
 {
+    const int ar = arith_of_form(form);
     int ring = slots;
-    if (kernel_plan(log_n, form, 0, count) == kPairPlan) {
-        const int r = pair_frame_ring(log_n, arith_of_form(form), slots);
-        ring = ring > r ? ring : r;
-    }
-    return ring < count ? ring : count;
+    // A mixed launch (FP32) may run fewer oceans of a size as register-resident
+    // tasks than a launch of their own.
+    if (form != 2 && (ar != kArPrecise || pair_frame_ok(log_n, ar, nf, false, count)))
+        ring = std::max(ring, pair_frame_ring(log_n, ar, slots));
+    return std::min(ring, count);
 }
 
-FrameChoice frame_choice(int log_n, int form, int count, int have)
+FrameChoice frame_choice(int log_n, int nf, int form, int count, int have)
 {
     const int slots = std::min(count, 3);
-    const int plan = kernel_plan(log_n, form, 0, count);
-    for (int s = slots; s >= std::min(count, 2); --s) {
-        const int ring = frame_ring_slots(log_n, form, s, count);
-        if (ring <= have) return {plan, s, ring};
+    if (kernel_plan(log_n, nf, form, false, 0, count) == kPairPlan) {
+        for (int s = slots; s >= std::min(count, 2); --s) {
+            const int ring = frame_ring_slots(log_n, nf, form, s, count);
+            if (ring <= have) return {kPairPlan, s, ring};
+        }
     }
     return {0, slots, slots};
 }
@@ -1400,7 +1402,7 @@ int frame_grid(int log_n, int nf, int form, bool fuse_foam, int plan, int count,
     if (plan == kPairPlan) {
         tasks = static_cast<long>(count) * pair_frame_tasks(log_n, arith_of_form(form), fuse_foam);
     } else {
-        if (!frame_kernel_ok(log_n, form, plan)) return 0;
+        if (!frame_kernel_ok(log_n, form, fuse_foam, plan)) return 0;
         tasks = static_cast<long>(count) *
                 frame_dispatch(log_n, nf, form, fuse_foam, plan, [](auto L) { return decltype(L)::P::RT; });
     }
@@ -1413,7 +1415,7 @@ int frame_blocks_per_sm(int log_n, int nf, int form, bool fuse_foam, int plan)
     if (log_n < 4 || log_n > 10) return 0;
     if (form == 2 && (log_n < 6 || log_n > 9)) return 0;
     if (plan == kPairPlan) return form == 2 ? 0 : pair_frame_blocks_per_sm(log_n, nf, arith_of_form(form), fuse_foam);
-    if (!frame_kernel_ok(log_n, form, plan)) return 0;
+    if (!frame_kernel_ok(log_n, form, fuse_foam, plan)) return 0;
     return frame_dispatch(log_n, nf, form, fuse_foam, plan, [](auto L) { return decltype(L)::blocks_per_sm(); });
 }
 
@@ -1426,7 +1428,7 @@ cudaError_t launch_frame(int log_n, int nf, int form, bool fuse_foam, const Fram
         if (form == 2) return cudaErrorInvalidValue;
         return launch_pair_frame(log_n, nf, arith_of_form(form), fuse_foam, a, q, grid, st);
     }
-    if (!frame_kernel_ok(log_n, form, plan)) return cudaErrorInvalidValue;
+    if (!frame_kernel_ok(log_n, form, fuse_foam, plan)) return cudaErrorInvalidValue;
     return frame_dispatch(log_n, nf, form, fuse_foam, plan,
                           [&](auto L) { return decltype(L)::launch(a, q, grid, st); });
 }

@@ -652,27 +652,45 @@ cudaError_t launch_pair_mixed(int nf, int ar, MixedArgs m, int grid, cudaStream_
 // tasks do not fill the GPU, is a longer chain here than with a task's pairs side
 // by side (frame_kernel). From the fourth ocean on that kernel waits for the three
 // slots of its ring; at 512^2 and above a frame fills the GPU sooner. us a frame
-// there / here, with velocity unless "-":
-//   N = 16   4 oceans 14.4 / 12.4, 64- 112 / 12, 4096- 6843 / 50
-//   N = 32   2 14.4 / 15.8, 4- 19.5 / 13.4, 2048- 5119 / 82
-//   N = 64   2 13.4 / 16.2, 3- 11.3 / 13.4, 4 21.3 / 16.5, 1024- 2625 / 143
-//   N = 128  3- 12.8 / 14.4, 4 24.6 / 18.5, 256- 1019 / 140
-//   N = 256  2 14.4 / 18.5, 3 20.5 / 20.8, 4 30.9 / 20.8, 64 414 / 165
-//   N = 512  1 22.6 / 22.6, 2 36.2 / 32.8, 64 854 / 651
-//   N = 1024 1- 61 / 57, 2- 111 / 78, 16 1137 / 793
+// there / here on either side of each line, without velocity, with it, and with
+// velocity and foam (where the lines differ, the first that holds for both):
+//   FP32   16    3  9.3/10.4    9.3/12.8   10.3/13.4    4  14.4/10.3   14.5/12.4   15.1/13.5
+//          32    3 12.4/13.4   15.4/15.7   15.4/17.0    4  19.6/13.4   23.7/15.9   23.9/17.2
+//          64    3 10.3/13.4                            4  15.2/13.4
+//                6             16.4/16.9   16.9/18.1    7              20.8/16.5   22.5/17.9
+//         128    3 12.4/14.4   12.4/18.1   13.2/18.6    4  17.9/14.5   19.6/18.5   20.6/18.7
+//         256    2 12.9/14.5                            3  18.5/16.5
+//                3             20.6/21.9   20.9/22.8    4              32.8/21.8   32.9/22.8
+//         512    1 18.2/18.1   22.7/22.6   24.7/26.0    2  28.3/24.7   36.5/32.9   40.1/35.7
+//        1024    1 60.7/56.6   81.6/81.9   90.2/94.5    2 110.8/78.5  148.1/113.6 161.6/133.6
 // The precise form's blocks of 16 indices (N = 128 and 256) leave four CTAs of 128
 // threads on an SM, and its chain is longest:
-//   N = 128  4 28.7 / 45, 8 40.2 / 47.0, 64 335 / 104
-//   N = 256  6 55.5 / 62.2, 10- 68.2 / 57.6, 21 168 / 141
-bool pair_frame_ok(int log_n, int ar, int count)
+//          32    3 14.5/17.8   17.5/22.0   17.5/22.7    4  21.9/18.2   27.5/22.2   27.7/22.7
+//          64    6 18.5/19.1   19.3/24.7   19.6/25.6    7  23.3/19.3   24.7/24.7   25.8/25.3
+//         128    9 30.9/31.4   37.5/47.2   39.4/48.0   10  40.8/31.3   48.7/47.2   50.9/48.0
+//         256    6 37.0/43.1   53.5/61.9   59.7/64.3    7  48.8/43.1   62.7/61.7   64.9/64.5
+//         512    1 24.6/26.8                            2  44.0/39.1
+//               12             259/264     272/269     16              341/341     359/352
+bool pair_frame_ok(int log_n, int ar, int nf, bool foam, int count)
 {
     if (!has_plan(log_n, ar)) return false;
-    if (ar == kArPrecise && log_n == 7) return count >= 12;
-    if (ar == kArPrecise && log_n == 8) return count >= 8;
-    return count >= (log_n >= 10 ? 1 : log_n == 9 ? 2 : 4);
+    const bool velocity = nf == 6;
+    int line;
+    if (ar == kArPrecise) {
+        line = log_n == 9 ? (velocity ? 16 : 2) : log_n == 8 ? 7 : log_n == 7 ? 10 : log_n == 6 ? 7 : 4;
+    } else {
+        switch (log_n) {
+            case 6: line = velocity ? 7 : 4; break;
+            case 8: line = velocity ? 4 : 3; break;
+            case 9: line = 2; break;
+            case 10: line = foam ? 2 : 1; break;
+            default: line = 4; break;
+        }
+    }
+    return count >= line;
 }
 
-// 1024^2 in the FP32 forms has no other kernel for a ring of three.
+// 1024^2 in the FP32 forms has no other kernel without foam for a ring of three.
 static_assert(PairPlan<10, kArExact, false>::ring(2) <= 3 && PairPlan<10, kArExact, true>::ring(2) <= 3);
 
 int pair_frame_ring(int log_n, int ar, int slots)

@@ -252,7 +252,7 @@ public:
         defer_ = nf_ == 6;
         // The persistent kernels' ring needs `ring_` oceans; the row/column
         // passes one per chunk ocean (all a batch above N = 1024 ever uses).
-        ring_ = frame_ring_slots(log_n_, form_, slots_, static_cast<int>(count_));
+        ring_ = frame_ring_slots(log_n_, nf_, form_, slots_, static_cast<int>(count_));
         const uint32_t inter_oceans = large() ? chunk_ : std::max(chunk_, static_cast<uint32_t>(ring_));
         inter_ = DevBuf<float2>(cells_ * nf_ * inter_oceans);
         queue_ = FrameQueue(count_, stream_);
@@ -663,7 +663,7 @@ private:
         q.slots = slots_;
         q.wait_ns = 1000000000ull;
         q.defer = defer_ ? 1 : 0;
-        const int plan = kernel_plan(log_n_, form_, plan_, static_cast<int>(k));
+        const int plan = kernel_plan(log_n_, nf_, form_, foam, plan_, static_cast<int>(k));
         const int wave = frame_wave(plan, foam);
         const int grid = frame_grid(log_n_, nf_, form_, foam, plan, static_cast<int>(k), wave, sms_);
         // A share below 1 leaves SMs to batches of other sizes running
@@ -844,7 +844,8 @@ public:
     // Settles the launch shapes, so a capture issues launches only.
     void prime_shapes()
     {
-        if (persistent_) (void)frame_wave(kernel_plan(log_n_, form_, plan_, static_cast<int>(count_)), false);
+        if (persistent_)
+            (void)frame_wave(kernel_plan(log_n_, nf_, form_, false, plan_, static_cast<int>(count_)), false);
     }
 
 private:

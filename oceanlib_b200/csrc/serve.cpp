@@ -588,7 +588,8 @@ private:
         check(cudaMemcpyAsync(k->tw.p, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, stream_),
               "twiddles");
         // The kernel plans of a few sessions and of many.
-        for (int plan : {kernel_plan(k->log_n, desc_.fft_form, 0, 1), kernel_plan(k->log_n, desc_.fft_form, 0, 64)}) {
+        for (int count : {1, 64}) {
+            const int plan = kernel_plan(k->log_n, k->nf, desc_.fft_form, false, 0, count);
             const int per_sm = frame_blocks_per_sm(k->log_n, k->nf, desc_.fft_form, false, plan);
             if (per_sm <= 0) throw DeviceError(cudaErrorInvalidConfiguration, "frame occupancy");
             k->wave[plan] = per_sm * sms_;
@@ -864,7 +865,7 @@ private:
             std::lock_guard<std::mutex> lk(mu_);
             const size_t others = in_use_ + ring_bytes_ - had;
             const size_t room = desc_.hbm_budget > others ? desc_.hbm_budget - others : 0;
-            const size_t most = ocean * static_cast<size_t>(frame_ring_slots(k->log_n, desc_.fft_form, 3, INT_MAX));
+            const size_t most = ocean * static_cast<size_t>(frame_ring_slots(k->log_n, k->nf, desc_.fft_form, 3, INT_MAX));
             if (want > room || !k->deep.reserve(blocks_, want, std::min({most, room, std::max(want, 2 * had)})))
                 k->short_of = slots;
             ring_bytes_ += k->deep.bytes() - had;
@@ -1021,7 +1022,7 @@ private:
                 g.clear_words = set.words;
                 g.count = count;
                 g.slots = std::min(count, 3);
-                g.ring = frame_ring_slots(k->log_n, desc_.fft_form, g.slots, count);
+                g.ring = frame_ring_slots(k->log_n, k->nf, desc_.fft_form, g.slots, count);
                 g.log_n = k->log_n;
                 continue;
             }
@@ -1035,9 +1036,9 @@ private:
             q.count = count;
             q.wait_ns = 1000000000ull;
             q.defer = k->nf == 6 ? 1 : 0;
-            const int want = frame_ring_slots(k->log_n, desc_.fft_form, std::min(count, 3), count);
-            const Ring ring = ring_for(k, static_cast<size_t>(want));
-            const FrameChoice choice = frame_choice(k->log_n, desc_.fft_form, count, ring.slots);
+            const FrameChoice roomy = frame_choice(k->log_n, k->nf, desc_.fft_form, count, INT_MAX);
+            const Ring ring = ring_for(k, static_cast<size_t>(roomy.ring));
+            const FrameChoice choice = frame_choice(k->log_n, k->nf, desc_.fft_form, count, ring.slots);
             q.slots = choice.slots;
             a.inter = ring.inter;
             const int grid = frame_grid(k->log_n, k->nf, desc_.fft_form, false, choice.plan, count,

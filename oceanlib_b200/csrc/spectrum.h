@@ -106,23 +106,23 @@ int frame_blocks_per_sm(int log_n, int nf, int form, bool fuse_foam, int plan);
 // Task plans a caller may choose for a size and form (1 or 2): 0 the default,
 // 1 the alternative of N = 256, 512 and 1024.
 int frame_plan_count(int log_n, int form);
-// The kernel plan of a launch of `count` oceans under task plan `plan`: the
-// plan itself, or kPairPlan, the register-resident frame (frame_pairs.cu), where
-// plan 0 takes that.
+// The kernel plan of a launch of `count` oceans (nf fields, with a fused foam
+// step) under task plan `plan`: the plan itself, or kPairPlan, the register-
+// resident frame (frame_pairs.cu), where plan 0 takes that.
 constexpr int kPairPlan = 2;
 constexpr int kMaxFramePlans = 3;  // kernel plans are below it
-int kernel_plan(int log_n, int form, int plan, int count);
+int kernel_plan(int log_n, int nf, int form, bool fuse_foam, int plan, int count);
 // Ocean slots of `inter` that launches of up to `count` oceans with
-// q.slots <= slots use, whatever the plan.
-int frame_ring_slots(int log_n, int form, int slots, int count);
-// How to launch `count` oceans (plan 0) where `inter` holds `have` of them, at
+// q.slots <= slots use, whatever the plan, alone or as a group of a mixed one.
+int frame_ring_slots(int log_n, int nf, int form, int slots, int count);
+// How to launch `count` oceans (plan 0, no foam) where `inter` holds `have` of them, at
 // least min(count, 3): the kernel plan, QueueArgs::slots, and the oceans of
 // `inter` it uses. A ring too short for all its rows ahead runs half of them
 // if that fits, else the kernel of three slots.
 struct FrameChoice {
     int plan, slots, ring;
 };
-FrameChoice frame_choice(int log_n, int form, int count, int have);
+FrameChoice frame_choice(int log_n, int nf, int form, int count, int have);
 // CTAs to launch a frame of `count` oceans with, of the `wave` that are resident
 // on `sms` SMs: no more per SM than it takes to hand every SM its even share of
 // the row tasks. (All CTAs of a wave draw their tickets at once, so with more of
@@ -130,7 +130,7 @@ FrameChoice frame_choice(int log_n, int form, int count, int have);
 int frame_grid(int log_n, int nf, int form, bool fuse_foam, int plan, int count, int wave, int sms);
 // The register-resident persistent frame, as frame_blocks_per_sm, frame_grid
 // and launch_frame call it for kPairPlan.
-bool pair_frame_ok(int log_n, int ar, int count);
+bool pair_frame_ok(int log_n, int ar, int nf, bool foam, int count);
 int pair_frame_ring(int log_n, int ar, int slots);
 int pair_frame_tasks(int log_n, int ar, bool fuse_foam);  // row tasks of an ocean
 int pair_frame_blocks_per_sm(int log_n, int nf, int ar, bool fuse_foam);

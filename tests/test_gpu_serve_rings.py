@@ -67,14 +67,16 @@ def _run(descs, budget, form, want_ring):
 
 SIZES = {
     "512": ([512] * 12, True),
+    "512_plain": ([512] * 12, False),
     "1024": ([1024] * 7, False),
     "64": ([64] * 40, True),
     "mixed_velocity": ([64] * 20 + [256] * 8 + [512] * 9, True),
     "mixed": ([128] * 12 + [512] * 6 + [1024] * 6, False),
 }
-# The precise form's 1024^2 and one launch of several sizes have three slots.
+# The precise form's 1024^2, its 512^2 with velocity below 16 oceans and its one
+# launch of several sizes have three slots.
 CASES = [(n, f) for n in SIZES for f in (abi.OCEAN_FFT_EXACT, abi.OCEAN_FFT_FAST)] + \
-    [("512", abi.OCEAN_FFT_PRECISE), ("64", abi.OCEAN_FFT_PRECISE)]
+    [("512_plain", abi.OCEAN_FFT_PRECISE), ("64", abi.OCEAN_FFT_PRECISE)]
 
 
 @pytest.mark.parametrize("name,form", CASES)
