@@ -715,12 +715,15 @@ public:
         plan_ = plan;
     }
 
-    // Intermediate ring slots of the persistent kernel: how many oceans'
-    // row-pass results may be in flight (2 or 3, as allocated; a batch of one
-    // ocean has 1). Fewer slots keep a large size's ring in L2; more let an
-    // ocean's rows overlap the previous oceans' columns. One slot with more
-    // oceans would make R(b + 1) wait for C(b), whose tickets come after it
-    // in the queue: the queue is only deadlock-free from two slots up.
+    // Intermediate ring slots of frame_kernel: how many oceans' row-pass
+    // results may be in flight (2 or 3, as allocated; a batch of one ocean has
+    // 1). Fewer slots keep a large size's ring in L2; more let an ocean's rows
+    // overlap the previous oceans' columns. One slot with more oceans would
+    // make R(b + 1) wait for C(b), whose tickets come after it in the queue:
+    // the queue is only deadlock-free from two slots up. The register-resident
+    // frame runs its rows ahead as far as a wave of CTAs holds with 3, half as
+    // far with 2 (its ring, ring(), is deeper); the one launch of an ensemble
+    // does not read the setting.
     int ring_slots() const { return slots_; }
     int ring() const { return ring_; }
     int min_ring_slots() const { return std::min(max_slots_, 2); }

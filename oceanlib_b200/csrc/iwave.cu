@@ -124,19 +124,21 @@ __device__ __forceinline__ float stamp_r2(const IWaveSource& s, int x, int z)
     return (px * px + pz * pz) * s.cell * s.cell;
 }
 
-// Mean of each source's clipped stamp, summed in double (deterministic tree
-// order) and rounded to float. The reference sums the same float terms
-// sequentially in double (src/interaction.cpp:357-366); the two orders' sums
-// differ by roundings near 1e-16 relative, far below the float mean's
-// 6e-8, so the float means agree (all 400 seeded random stamps of sizes up
-// to 257 x 257 cells compared equal).
+// Mean of each source's clipped stamp, summed in double (a fixed order) and
+// rounded to float. The reference sums the same float terms sequentially in
+// double (src/interaction.cpp:357-366); the two orders' sums differ by roundings
+// near 1e-16 of the terms, far below the float mean's 6e-8 of itself (the terms
+// cancel, but a stamp's box ends at 4 sigma, so not to nothing), and the float
+// means agree: 400 seeded random stamps of up to 257 x 257 cells, clipped ones
+// among them, summed in both orders on the CPU, were all equal.
 //
 // A stamp is a chain of double exponentials on few cells: what bounds it is
 // how many a thread evaluates one after the other, not the arithmetic rate.
 // So a source is a cluster of kMeanCtas CTAs, a warp a row of the stamp, and
 // CTA 0 adds the parts in order out of the others' shared memory: 21
-// exponentials a thread for a 193 x 193 stamp instead of 146 in one CTA of
-// 256 threads. 8 sources of up to 193 x 193 cells: 37.1 -> 8.1 us.
+// exponentials in most threads for a 193 x 193 stamp, 28 in the longest chain
+// (the warp with a fourth row), instead of 146 in one CTA of 256 threads. 8
+// sources of up to 193 x 193 cells: 37.1 -> 8.1 us.
 constexpr int kMeanCtas = 8;  // the portable cluster size
 constexpr int kMeanThreads = 256;
 

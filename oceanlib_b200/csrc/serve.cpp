@@ -9,8 +9,9 @@
 //   one H2D copy    every per-batch table (ocean pointer tables and times,
 //                   resolved sources, per-substep field lists, query jobs
 //                   and points) from one pinned block;
-//   ocean frames    one persistent frame kernel per ocean size over every
-//                   session updating in this batch (pointer-table form);
+//   ocean frames    one persistent launch over every session updating in this
+//                   batch (pointer-table form), or one per ocean size where
+//                   the sizes do not mix (see launch());
 //   interaction     one source-mean launch for all sources, then per field
 //                   kind and substep one batched source-stamp and one batched
 //                   stencil launch over every session stepping, one finalize;

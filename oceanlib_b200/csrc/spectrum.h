@@ -49,7 +49,7 @@ struct FrameArgs {
     const OceanConsts* consts; // [count]
     const double* t_over_2pi;  // [count], or null: every ocean at t_uniform
     double t_uniform;          // t / 2 pi of every ocean (t_over_2pi null)
-    float2* inter;             // [chunk][N][N][NF] row-pass output
+    float2* inter;             // row-pass output, NF N^2 an ocean of the chunk or ring (each kernel's own layout)
     float4* disp;              // [count][N*N]
     float4* normal;            // [count][N*N]
     float4* velocity;          // [count][N*N] or null
@@ -78,8 +78,11 @@ struct QueueArgs {
     unsigned* rows_done;
     unsigned* cols_done;
     unsigned* error;      // sticky: set to 1 when a bounded wait gives up
-    int32_t count;        // oceans in the frame (inter holds `slots` of them)
-    int32_t slots;        // intermediate ring slots
+    int32_t count;        // oceans in the frame
+    // Intermediate ring of frame_kernel, in oceans. The register-resident frame
+    // takes its rows ahead and its ring (up to hundreds of oceans) from the
+    // size: all of them with 3, half with 2. frame_ring_slots covers both.
+    int32_t slots;
     unsigned long long wait_ns;
     unsigned* clear;
     uint32_t clear_words;
@@ -146,10 +149,11 @@ cudaError_t launch_wait_probe(const unsigned* counter, unsigned target, unsigned
 // a batch with its own arrays, counters and intermediate ring) as one
 // persistent launch whose ticket queue holds group after group. Sizes N = 32
 // .. 1024 (log_n 5..10), one field count for all groups, FP32 forms, no
-// persistent foam. Group g's tickets are [first, first + tasks), tasks =
-// mixed_tasks(log_n, count); its rows_done / cols_done (count each) and the
-// ticket must be zero at launch, which clears the next launch's words, each
-// group's and `clear_ticket`, as QueueArgs says.
+// persistent foam. Group g's tickets follow those of the groups before it, from
+// `first` on, one for each row and column task of the kernel in use; its
+// rows_done / cols_done (count each) and the ticket must be zero at launch,
+// which clears the next launch's words, each group's and `clear_ticket`, as
+// QueueArgs says.
 constexpr int kMaxMixedGroups = 6;
 struct MixedGroup {
     FrameArgs a;          // the group's arrays, or its pointer table (ocean_base 0)
