@@ -21,9 +21,11 @@
 // Per session, requests keep their submission order: a batch takes at most
 // one update of a session and then only queries that follow it, so a query
 // sees exactly the updates submitted before it. Batches run in order on one
-// stream. Each session's arithmetic is the single-session arithmetic (same
+// stream; a batch's interaction fields run on a second one beside its oceans,
+// between its upload and its queries. Each session's arithmetic is the single-session arithmetic (same
 // kernels, same per-cell order), so a result is the same alone and in any
-// mix. Session memory comes from a stream-ordered pool: a session is
+// mix (but the precise form's 1024^2, whose stage blocks, and so roundings,
+// are others in a launch of several sizes). Session memory comes from a stream-ordered pool: a session is
 // admitted when its bytes fit in the budget (FIFO), and a closed session's
 // memory is released behind the last batch that used it. What the sessions
 // leave of the budget may hold larger intermediate rings, which make frames of

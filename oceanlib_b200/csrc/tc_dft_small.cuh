@@ -23,12 +23,13 @@
 // velocity (512 allocated, one CTA per SM), 256 without.
 //
 // The GEMMs are exact as the 512-point engine's: rows scaled to [2^29, 2^30),
-// four signed 8-bit digits, digit-pair levels 0..3. Here the digits are FP16
-// operands and the levels exact integers in FP32 (8-bit operands need K = 32,
-// twice stage 1's K at 64 and 128). The middle step is done in FP64 instead: the four levels of Y combine exactly
-// (an integer below 2^47 times a power of two), the twiddles W_N^(n2 k1) are
-// the exact ones (sincospi in double, not the FP32 table), and Z is rounded
-// to FP32 once. With the FP32 middle step (three roundings of Y, the FP32
+// four signed 8-bit digits, digit-pair levels 0..3. Here the digits are still
+// FP16 operands and the levels exact integers in FP32: 8-bit operands have not
+// been brought to these sizes (their K is 32: both stages' at 256, twice stage
+// 1's at 64 and 128). The middle step is done in FP64 instead: the four levels
+// of Y combine exactly (an integer below 2^47 times a power of two), the
+// twiddles W_N^(n2 k1) are the exact ones (sincospi in double, not the FP32
+// table), and Z is rounded to FP32 once. With the FP32 middle step (three roundings of Y, the FP32
 // twiddle, Kahan's difference of products) a 128^2 frame with velocity
 // reached 2.14e-6 of FP64 on normal.x.
 #pragma once
