@@ -865,12 +865,13 @@ private:
         const size_t want = slots * ocean;
         // Memory that was short is not asked for again until a session closes.
         if (want > had && slots < k->short_of) {
-            std::lock_guard<std::mutex> lk(mu_);
+            // (Only this thread changes the two sums; clients may submit meanwhile.)
             const size_t others = in_use_ + ring_bytes_ - had;
             const size_t room = desc_.hbm_budget > others ? desc_.hbm_budget - others : 0;
             const size_t most = ocean * static_cast<size_t>(frame_ring_slots(k->log_n, k->nf, desc_.fft_form, 3, INT_MAX));
             if (want > room || !k->deep.reserve(blocks_, want, std::min({most, room, std::max(want, 2 * had)})))
                 k->short_of = slots;
+            std::lock_guard<std::mutex> lk(mu_);
             ring_bytes_ += k->deep.bytes() - had;
         }
         if (k->deep.get() == nullptr) return {k->inter.p, 3};
