@@ -665,6 +665,23 @@ private:
         }
     }
 
+    // Dispatcher thread, outside the lock, where the device is short of memory
+    // that the budget still had: the larger rings give theirs back to the pool
+    // and to the device, once the batches that used it are over. Whether there
+    // was any to give.
+    bool drop_rings()
+    {
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (ring_bytes_ == 0) return false;
+            ring_bytes_ = 0;
+        }
+        for (auto& k : ocean_kinds_) k->deep.release(blocks_);
+        cudaStreamSynchronize(stream_);
+        cudaMemPoolTrimTo(pool_, 0);
+        return true;
+    }
+
     // Memory came back: a ring that was too large may fit now.
     void forget_short_rings()
     {
@@ -841,7 +858,8 @@ private:
         const size_t dev_bytes = in_bytes + round_up(out_floats * sizeof(float), 16);
         const size_t had = c->dev.bytes();
         if (dev_bytes > had) {
-            const bool ok = c->dev.reserve(blocks_, dev_bytes, 2 * had);
+            const bool ok = c->dev.reserve(blocks_, dev_bytes, 2 * had) ||
+                            (drop_rings() && c->dev.reserve(blocks_, dev_bytes, dev_bytes));
             {
                 std::lock_guard<std::mutex> lk(mu_);
                 staging_bytes_ += c->dev.bytes() - had;  // reported, not part of the session budget
@@ -1245,10 +1263,17 @@ private:
                 lk.unlock();
                 std::vector<bool> ok(admits.size(), true);
                 for (size_t i = 0; i < admits.size(); ++i) {
-                    try {
-                        admit(admits[i]);
-                    } catch (const std::exception&) {
-                        ok[i] = false;
+                    // Once more without the larger rings if memory ran out.
+                    for (bool again = true; again;) {
+                        again = false;
+                        try {
+                            admit(admits[i]);
+                        } catch (const DeviceError& e) {
+                            again = e.code == cudaErrorMemoryAllocation && admits[i]->block == nullptr && drop_rings();
+                            ok[i] = again;
+                        } catch (const std::exception&) {
+                            ok[i] = false;
+                        }
                     }
                 }
                 lk.lock();
