@@ -1384,16 +1384,15 @@ int frame_ring_slots(int log_n, int nf, int form, int slots, int count)
     return std::min(ring, count);
 }
 
-FrameChoice frame_choice(int log_n, int nf, int form, int count, int have)
+FrameChoice frame_choice(int log_n, int nf, int form, bool fuse_foam, int plan, int count, int slots, int have)
 {
-    const int slots = std::min(count, 3);
-    if (kernel_plan(log_n, nf, form, false, 0, count) == kPairPlan) {
-        for (int s = slots; s >= std::min(count, 2); --s) {
+    if (kernel_plan(log_n, nf, form, fuse_foam, plan, count) == kPairPlan) {
+        for (int s = slots; s >= std::min(slots, 2); --s) {
             const int ring = frame_ring_slots(log_n, nf, form, s, count);
             if (ring <= have) return {kPairPlan, s, ring};
         }
     }
-    return {0, slots, slots};
+    return {plan, slots, std::min(slots, count)};
 }
 
 int frame_grid(int log_n, int nf, int form, bool fuse_foam, int plan, int count, int wave, int sms)

@@ -253,8 +253,6 @@ public:
         // The persistent kernels' ring needs `ring_` oceans; the row/column
         // passes one per chunk ocean (all a batch above N = 1024 ever uses).
         ring_ = frame_ring_slots(log_n_, nf_, form_, slots_, static_cast<int>(count_));
-        const uint32_t inter_oceans = large() ? chunk_ : std::max(chunk_, static_cast<uint32_t>(ring_));
-        inter_ = DevBuf<float2>(cells_ * nf_ * inter_oceans);
         queue_ = FrameQueue(count_, stream_);
         error_ = DevBuf<unsigned>(1);
         check(cudaMemsetAsync(error_.p, 0, sizeof(unsigned), stream_), "memset");
@@ -269,6 +267,7 @@ public:
             check(cudaMemsetAsync(foam_a_.p, 0, cells_ * count_ * sizeof(float), stream_), "memset");
             check(cudaMemsetAsync(foam_b_.p, 0, cells_ * count_ * sizeof(float), stream_), "memset");
         }
+        alloc_ring();
         for (int s = 0; s < kTimeSlots; ++s) {
             check(cudaEventCreateWithFlags(&slot_done_[s], cudaEventDisableTiming), "event");
         }
@@ -660,10 +659,11 @@ private:
         q.clear_words = set.words;
         q.error = error_.p;
         q.count = static_cast<int32_t>(k);
-        q.slots = slots_;
+        const FrameChoice choice = frame_choice(log_n_, nf_, form_, foam, plan_, static_cast<int>(k), slots_, ring_);
+        q.slots = choice.slots;
         q.wait_ns = 1000000000ull;
         q.defer = defer_ ? 1 : 0;
-        const int plan = kernel_plan(log_n_, nf_, form_, foam, plan_, static_cast<int>(k));
+        const int plan = choice.plan;
         const int wave = frame_wave(plan, foam);
         const int grid = frame_grid(log_n_, nf_, form_, foam, plan, static_cast<int>(k), wave, sms_);
         // A share below 1 leaves SMs to batches of other sizes running
@@ -848,10 +848,27 @@ public:
     void prime_shapes()
     {
         if (persistent_)
-            (void)frame_wave(kernel_plan(log_n_, nf_, form_, false, plan_, static_cast<int>(count_)), false);
+            (void)frame_wave(
+                frame_choice(log_n_, nf_, form_, false, plan_, static_cast<int>(count_), slots_, ring_).plan, false);
     }
 
 private:
+    // The intermediate, after everything that a batch cannot do without: on a
+    // device with no room for the larger ring of the register-resident frames it
+    // holds the three slots that every batch can run on (frame_choice).
+    void alloc_ring()
+    {
+        const auto alloc = [&](uint32_t oceans) { inter_ = DevBuf<float2>(cells_ * nf_ * oceans); };
+        const uint32_t least = large() ? chunk_ : std::max(chunk_, static_cast<uint32_t>(slots_));
+        const uint32_t most = large() ? chunk_ : std::max(chunk_, static_cast<uint32_t>(ring_));
+        try {
+            alloc(most);
+        } catch (const DeviceError& e) {
+            if (e.code != cudaErrorMemoryAllocation || least == most) throw;
+            alloc(least);
+            ring_ = static_cast<int>(least);
+        }
+    }
 
     // The frame's arguments with t / 2 pi hoisted exactly as
     // src/core/evolve.cpp:33 does: one time for every ocean travels with the
@@ -979,7 +996,7 @@ private:
     bool persistent_ = true;
     int slots_ = 1;      // intermediate ring slots the persistent kernel uses
     int max_slots_ = 1;  // the most of them
-    int ring_ = 1;       // oceans that the kernels' rings use at most
+    int ring_ = 1;       // oceans of inter_ that the kernels' rings may use
     bool defer_ = false; // QueueArgs::defer of the persistent kernel
     int frame_wave_[kMaxFramePlans][2] = {};  // [kernel plan][foam]: CTAs of one wave
     int sms_ = 0;

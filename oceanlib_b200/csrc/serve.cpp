@@ -1058,9 +1058,11 @@ private:
             q.count = count;
             q.wait_ns = 1000000000ull;
             q.defer = k->nf == 6 ? 1 : 0;
-            const FrameChoice roomy = frame_choice(k->log_n, k->nf, desc_.fft_form, count, INT_MAX);
-            const Ring ring = ring_for(k, static_cast<size_t>(roomy.ring));
-            const FrameChoice choice = frame_choice(k->log_n, k->nf, desc_.fft_form, count, ring.slots);
+            const auto choose = [&](int have) {
+                return frame_choice(k->log_n, k->nf, desc_.fft_form, false, 0, count, std::min(count, 3), have);
+            };
+            const Ring ring = ring_for(k, static_cast<size_t>(choose(INT_MAX).ring));
+            const FrameChoice choice = choose(ring.slots);
             q.slots = choice.slots;
             a.inter = ring.inter;
             const int grid = frame_grid(k->log_n, k->nf, desc_.fft_form, false, choice.plan, count,

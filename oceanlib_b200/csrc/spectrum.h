@@ -118,14 +118,15 @@ int kernel_plan(int log_n, int nf, int form, bool fuse_foam, int plan, int count
 // Ocean slots of `inter` that launches of up to `count` oceans with
 // q.slots <= slots use, whatever the plan, alone or as a group of a mixed one.
 int frame_ring_slots(int log_n, int nf, int form, int slots, int count);
-// How to launch `count` oceans (plan 0, no foam) where `inter` holds `have` of them, at
-// least min(count, 3): the kernel plan, QueueArgs::slots, and the oceans of
-// `inter` it uses. A ring too short for all its rows ahead runs half of them
-// if that fits, else the kernel of three slots.
+// How to launch `count` oceans under task plan `plan` with up to `slots` slots
+// (2 or 3; 1 for one ocean) where `inter` holds `have` oceans, at least
+// min(count, 3): the kernel plan, QueueArgs::slots, and the oceans of `inter` it
+// uses. A ring too short for all its rows ahead runs half of them if that fits,
+// else the kernel of three slots.
 struct FrameChoice {
     int plan, slots, ring;
 };
-FrameChoice frame_choice(int log_n, int nf, int form, int count, int have);
+FrameChoice frame_choice(int log_n, int nf, int form, bool fuse_foam, int plan, int count, int slots, int have);
 // CTAs to launch a frame of `count` oceans with, of the `wave` that are resident
 // on `sms` SMs: no more per SM than it takes to hand every SM its even share of
 // the row tasks. (All CTAs of a wave draw their tickets at once, so with more of
