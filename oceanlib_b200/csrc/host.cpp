@@ -1422,7 +1422,7 @@ public:
         concurrent_ = true;
         describe_ = "concurrent, SM shares by work estimate";
         if (tune) autotune();
-        use_graph_ = true;  // after the autotuner, which times per-call launches
+        use_graph_ = true;
     }
 
     ~Ensemble()
@@ -1627,14 +1627,37 @@ private:
         return best;
     }
 
+    // The frame as use will run it: the graph of the settings at hand, replayed.
+    // (Concurrent launches interleave otherwise than when each is issued by
+    // itself: 6 x 128^2 and 3 x 256^2 in 33 us issued, 39.7 replayed.)
+    double time_replays(int frames)
+    {
+        drop_graph();
+        use_graph_ = true;
+        const double ms = time_frames(frames, [&](double t) { update(t, stream_); });
+        use_graph_ = false;
+        drop_graph();
+        return ms;
+    }
+
     // Candidates: (1) sizes one after another, each with the whole GPU;
     // (2) concurrent, SM shares by the work estimate; (3) concurrent, shares
     // by each size's measured stand-alone time; (4) every size in one mixed
-    // launch, when the sizes allow it. The fastest is kept, the one launch
-    // unless another is more than 3 % faster.
+    // launch, when the sizes allow it; (5) as (2) with the sizes' default plans:
+    // what is fastest for a size alone need not be beside others (precise form,
+    // 8 x 64^2, 8 x 256^2 and 4 x 512^2: 103 us, 121 with the sizes' own
+    // choices). The fastest is kept, the one launch unless another is more than
+    // 3 % faster.
     void autotune()
     {
         const int frames = 5;
+        struct Setting {
+            int plan, slots;
+            bool defer;
+        };
+        std::vector<Setting> defaults;
+        for (auto& b : batches_) defaults.push_back({b->plan(), b->ring_slots(), b->deferred_publish()});
+        const double t_plain = time_replays(frames);  // as constructed
         // Per size: the persistent kernel's task plans, timed alone on the
         // whole GPU (the construction left each size its work-share grid).
         full_grids();
@@ -1657,12 +1680,12 @@ private:
         for (size_t g = 0; g < batches_.size(); ++g)
             alone[g] = time_frames(frames, [&](double t) { batches_[g]->update(&t, false, 0.0f, stream_); });
         concurrent_ = false;
-        const double t_seq = time_frames(frames, [&](double t) { update(t, stream_); });
+        const double t_seq = time_replays(frames);
         concurrent_ = true;
         apply_shares(work_);
-        const double t_work = time_frames(frames, [&](double t) { update(t, stream_); });
+        const double t_work = time_replays(frames);
         apply_shares(alone);
-        const double t_meas = time_frames(frames, [&](double t) { update(t, stream_); });
+        const double t_meas = time_replays(frames);
         double t_mixed = -1.0;
         if (mixed_ok_) {
             mixed_ = true;
@@ -1697,28 +1720,38 @@ private:
         // launch stayed within 1 %. So the one launch is kept unless another
         // schedule is more than 3 % faster (on those oceans now it is: 0.48 ms
         // against 0.56).
-        const double other = std::min(t_seq, std::min(t_work, t_meas));
+        const double other = std::min({t_seq, t_work, t_meas, t_plain});
         const bool mixed_wins = t_mixed >= 0.0 && t_mixed <= 1.03 * other;
         if (mixed_wins) {
             mixed_ = true;
             concurrent_ = false;
             full_grids();
             std::snprintf(buf, sizeof(buf), "mixed: every size in one persistent launch%s, %s publish (%.3f ms; "
-                          "sequential %.3f, work-share %.3f, measured-share %.3f)",
+                          "sequential %.3f, work-share %.3f, measured-share %.3f, default plans %.3f)",
                           mixed_shallow_ ? " at 2 ring slots" : "", mix_defer_ ? "deferred" : "immediate", t_mixed,
-                          t_seq, t_work, t_meas);
+                          t_seq, t_work, t_meas, t_plain);
+        } else if (t_plain < t_seq && t_plain < t_work && t_plain < t_meas) {
+            for (size_t g = 0; g < batches_.size(); ++g) {
+                batches_[g]->set_plan(defaults[g].plan);
+                batches_[g]->set_ring_slots(defaults[g].slots);
+                batches_[g]->set_deferred_publish(defaults[g].defer);
+            }
+            apply_shares(work_);
+            plans.clear();
+            std::snprintf(buf, sizeof(buf), "concurrent, shares by work estimate, default plans (%.3f ms; sequential "
+                          "%.3f, work-share %.3f, measured-share %.3f)", t_plain, t_seq, t_work, t_meas);
         } else if (t_seq <= t_work && t_seq <= t_meas) {
             concurrent_ = false;
             full_grids();
-            std::snprintf(buf, sizeof(buf), "sequential (%.3f ms; concurrent %.3f / %.3f ms)", t_seq, t_work,
-                          t_meas);
+            std::snprintf(buf, sizeof(buf), "sequential (%.3f ms; concurrent %.3f / %.3f ms, default plans %.3f)",
+                          t_seq, t_work, t_meas, t_plain);
         } else if (t_work <= t_meas) {
             apply_shares(work_);
             std::snprintf(buf, sizeof(buf), "concurrent, shares by work estimate (%.3f ms; sequential %.3f, "
-                          "measured-share %.3f)", t_work, t_seq, t_meas);
+                          "measured-share %.3f, default plans %.3f)", t_work, t_seq, t_meas, t_plain);
         } else {
             std::snprintf(buf, sizeof(buf), "concurrent, shares by measured time (%.3f ms; sequential %.3f, "
-                          "work-share %.3f)", t_meas, t_seq, t_work);
+                          "work-share %.3f, default plans %.3f)", t_meas, t_seq, t_work, t_plain);
         }
         describe_ = buf;
         if (!plans.empty()) describe_ += "; task plans: " + plans;
