@@ -727,6 +727,7 @@ public:
     int ring_slots() const { return slots_; }
     int ring() const { return ring_; }
     int min_ring_slots() const { return std::min(max_slots_, 2); }
+    int max_ring_slots() const { return max_slots_; }
     void set_ring_slots(int slots)
     {
         if (slots < min_ring_slots() || slots > max_slots_) throw std::invalid_argument("ring slots");
@@ -1567,7 +1568,7 @@ private:
         for (size_t k = 0; k < mix_order_.size(); ++k) {
             Batch& b = *batches_[mix_order_[k]];
             m.g[k] = b.mixed_group(t_over_2pi, st);
-            if (mixed_shallow_) m.g[k].slots = b.min_ring_slots();
+            m.g[k].slots = mixed_shallow_ ? b.min_ring_slots() : b.max_ring_slots();
         }
         const FrameQueue::Set ticket = mix_ticket_.take(st);
         m.ticket = ticket.ticket;
@@ -1690,11 +1691,12 @@ private:
         if (mixed_ok_) {
             mixed_ = true;
             t_mixed = time_frames(frames, [&](double t) { update(t, stream_); });
-            // The one launch again with every group at its shallowest ring:
-            // all sizes' intermediates share L2 in this schedule. (Register-
-            // resident tasks have the one depth of the launch.)
+            // The one launch (at every group's deepest ring, whatever its size
+            // chose alone) again with every group at its shallowest ring: all
+            // sizes' intermediates share L2 in this schedule. (Register-resident
+            // tasks have the one depth of the launch.)
             bool shallower = false;
-            for (auto& b : batches_) shallower = shallower || b->ring_slots() > b->min_ring_slots();
+            for (auto& b : batches_) shallower = shallower || b->max_ring_slots() > b->min_ring_slots();
             if (shallower && !mix_pairs_) {
                 mixed_shallow_ = true;
                 const double t2 = time_frames(frames, [&](double t) { update(t, stream_); });
