@@ -462,8 +462,9 @@ public:
         const uint32_t steps = foam_on_ ? foam_accumulate(foam_dt) : 0u;
         if (steps > 0) set_foam_args(a);
         // Foam beyond the fused substep (all of it above N = 1024) comes after
-        // every ocean's frame, so copies start per chunk only without it.
-        const bool pipelined = steps == 0 || (steps == 1 && !large());
+        // every ocean's frame, and its plane is copied then; it changes no other
+        // output.
+        const bool foam_last = steps > 1 || (steps == 1 && large());
         const size_t bytes4 = cells_ * sizeof(float4);
         uint32_t c = 0;
         for (uint32_t base = 0; base < count_; base += chunk_, ++c) {
@@ -476,11 +477,9 @@ public:
                 run_row(a, stream_);
                 run_col(a, stream_, steps > 0);
             }
-            if (pipelined) {
-                check(cudaEventRecord(chunk_events_[c], stream_), "event");
-                check(cudaStreamWaitEvent(copy_stream_, chunk_events_[c], 0), "wait");
-                copy_out(base, k, bytes4, h_disp, h_normal, h_vel, h_foam, steps > 0);
-            }
+            check(cudaEventRecord(chunk_events_[c], stream_), "event");
+            check(cudaStreamWaitEvent(copy_stream_, chunk_events_[c], 0), "wait");
+            copy_out(base, k, bytes4, h_disp, h_normal, h_vel, foam_last ? nullptr : h_foam, steps > 0);
         }
         if (steps > 0) {
             if (large()) foam_substep(stream_);
@@ -490,14 +489,11 @@ public:
                 foam_cur_ ^= 1;
             }
         }
-        if (!pipelined) {
+        if (foam_last && h_foam) {
             check(cudaEventRecord(chunk_events_[0], stream_), "event");
             check(cudaStreamWaitEvent(copy_stream_, chunk_events_[0], 0), "wait");
-            copy_out(0, count_, bytes4, h_disp, h_normal, h_vel, h_foam, false);
-            if (h_foam) {
-                check(cudaMemcpyAsync(h_foam, foam_ptr(0), cells_ * count_ * sizeof(float),
-                                      cudaMemcpyDeviceToHost, copy_stream_), "copy foam");
-            }
+            check(cudaMemcpyAsync(h_foam, foam_ptr(0), cells_ * count_ * sizeof(float), cudaMemcpyDeviceToHost,
+                                  copy_stream_), "copy foam");
         }
         check(cudaStreamSynchronize(copy_stream_), "copy back");
         check(cudaStreamSynchronize(stream_), "frame");
